@@ -1143,92 +1143,218 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
 // LU with the reference's 4-row-panel pivoting (LUsolver.C:106-246 panel,
 // 503-660 two- and three-row tails, 3058-3143 driver): partial pivoting
 // restricted to the current panel, exact-zero pivots replaced by 2.22e-16,
-// whole-row interchanges recorded LAPACK style.
+// whole-row interchanges.
 
+// t < v for v >= 0 or NaN, on the integer pipe for doubles (an FP64 compare
+// costs as much as a multiply-add): the order of non-negative doubles is the
+// order of their bits, a negative t sorts below them, NaN compares false.
+__device__ __forceinline__ bool less_abs(double t, double v) {
+    const long long a = __double_as_longlong(t), b = __double_as_longlong(v);
+    return a < b && b <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool less_abs(float t, float v) { return t < v; }
+
+// The panel's diagonal block, size x size, one element per lane: lane 4r + c
+// of a warp holds a = A[r][c] (lanes 16..31 mirror 0..15).  The pivot search
+// never leaves these rows, so the block is factored on its own; on return a
+// holds its L and U, invD[k] the reciprocal pivots, and the result is the
+// row of the panel that moved to row r.
+// The loop over its columns stays rolled: unrolled per size it was no faster
+// (the reciprocals' latency sets its time) and four times the code.
 template<class MT>
-__device__ __forceinline__ int choose_pivot(const MT* A, int ld, int k, int pos, int size) {
-    const int cand = size - pos;
-    if (cand <= 1) return k;
-    if (pos == 0 && size >= 3) {
-        int best = 0;
-        double t = 0;
-        for (int c = 0; c < size; c++) {
-            const double v = fabs(double(A[(size_t)(k + c) * ld + k]));
-            if (t < v) { best = c; t = v; }
+__device__ __forceinline__ int lu_diagonal_block(MT& a, int size, double* invD, int lane) {
+    const unsigned FULL = 0xffffffffu;
+    const int r = (lane >> 2) & 3, c = lane & 3;
+    int from = r;
+    if (size == 1) {
+        if (lane == 0) invD[0] = 1.0 / double(a);
+        return from;
+    }
+    #pragma unroll 1
+    for (int k = 0; k < size; k++) {
+        // every lane inverts its own element while the pivot search runs; the
+        // chosen row's reciprocal is then one shuffle away
+        double own = double(a);
+        if ((__double_as_longlong(own) << 1) == 0) own = kPivEps;
+        own = double(MT(1.0 / own));
+        // choose_pivot of the reference: the first column of a panel of 3 or
+        // 4 rows compares all its rows, the others their own and the next
+        // (the second of four also the last, LUsolver.C:169-185, where the
+        // running maximum keeps the signed value of the middle row)
+        int p = k;
+        if (size - k > 1) {
+            const MT v0 = fabs(__shfl_sync(FULL, a, 5 * k)), v1 = __shfl_sync(FULL, a, 4 * (k + 1) + k);
+            const MT v2 = fabs(__shfl_sync(FULL, a, 4 * ((k + 2) & 3) + k));
+            const MT v3 = fabs(__shfl_sync(FULL, a, 4 * ((k + 3) & 3) + k));
+            if (k == 0 && size >= 3) {
+                MT t = MT(0);
+                if (less_abs(t, v0)) t = v0;
+                if (less_abs(t, MT(fabs(v1)))) { p = 1; t = fabs(v1); }
+                if (less_abs(t, v2)) { p = 2; t = v2; }
+                if (size == 4 && less_abs(t, v3)) p = 3;
+            } else if (size == 4 && k == 1) {
+                MT t = v0;
+                if (less_abs(t, MT(fabs(v1)))) { p = 2; t = v1; }
+                if (less_abs(t, v2)) p = 3;
+            } else if (less_abs(v0, MT(fabs(v1)))) {
+                p = k + 1;
+            }
         }
-        return k + best;
+        const int src = r == k ? p : (r == p ? k : r);
+        a = __shfl_sync(FULL, a, 4 * src + c);
+        from = __shfl_sync(FULL, from, 4 * src + c);
+        const double inv = __shfl_sync(FULL, own, 4 * p + k);
+        if (lane == 0) invD[k] = inv;
+        if (k + 1 < size) {
+            const MT l = a * MT(inv);
+            if (c == k && r > k) a = l;
+            const MT lr = __shfl_sync(FULL, a, 4 * r + k), uc = __shfl_sync(FULL, a, 4 * k + c);
+            const MT u = fma(-lr, uc, a);
+            if (r > k && c > k) a = u;
+        }
     }
-    if (size == 4 && pos == 1) {
-        // LUsolver.C:169-185: the running maximum keeps the signed value of row 2
-        double t = fabs(double(A[(size_t)k * ld + k]));
-        int best = 0;
-        const double v1 = double(A[(size_t)(k + 1) * ld + k]);
-        if (t < fabs(v1)) { best = 1; t = v1; }
-        if (t < fabs(double(A[(size_t)(k + 2) * ld + k]))) best = 2;
-        return k + best;
-    }
-    return (fabs(double(A[(size_t)k * ld + k])) < fabs(double(A[(size_t)(k + 1) * ld + k]))) ? k + 1 : k;
+    return from;
 }
 
-// work: n ints of slot scratch that is free during the factorisation (the
-// permutation is built there and copied over piv).
+// One element of the trailing block: the panel's four updates.
+template<class MT>
+__device__ __forceinline__ MT lu_rank4(const MT* l, const MT* u, int ld, MT x) {
+    return fma(-l[3], u[3 * ld], fma(-l[2], u[2 * ld], fma(-l[1], u[ld], fma(-l[0], u[0], x))));
+}
+
+// Right-looking by panels of four columns, every element's multiply-adds in
+// the order of the column-by-column elimination.  Per panel, with two
+// barriers: (1) threads own whole rows below the panel (their four L
+// entries) and whole columns beside it (interchange, then the U entries);
+// (2) the trailing block takes the panel's four updates at once, its elements
+// spread over the threads row by row (m^2 / G of them each, where a fixed
+// thread grid would round both dimensions up), while warp 0 updates and
+// factors the next panel's diagonal block ahead of the others: that block is
+// a chain of four divisions (about kAhead element updates long) which would
+// otherwise keep the whole group waiting.  An FP64 instruction holds its
+// scheduler for 64 cycles, so what counts is how many are issued and how
+// long the group waits, not the shared-memory traffic.  Measured against the
+// column-by-column form (four barriers a column, the pivot and its division
+// on one thread), whole steps: 150 cells of 200 species at 256 threads
+// 441 -> 288 ms, 400 of 111 species at 64 threads 82 -> 70 ms, 2,000 of 53
+// species 69.3 -> 66.4 ms; 10 to 16 species unchanged (the chain of
+// reciprocals sets the time there in either form).
+// work: 4 ints of slot scratch that is free during the factorisation.  piv
+// receives the gather permutation of the solves, (P b)[i] = b[piv[i]].
 template<int G, class MT>
 __device__ __noinline__ void lu_factor(const Grp<G>& g, MT* A, int n, int ld, int* piv, double* invD, int* work) {
-    const int rem = n & 3;
-    constexpr int TC = 8, TR = G / TC;
-    const int tr = g.rank / TC, tc = g.rank % TC;
-    for (int k = 0; k < n; k++) {
-        const bool tail = k >= n - rem;
-        const int size = tail ? rem : 4;
-        const int pos = tail ? k - (n - rem) : (k & 3);
-        if (size == 1) {
-            if (g.rank == 0) { invD[k] = 1.0 / double(A[(size_t)k * ld + k]); piv[k] = k; }
-            g.sync();
-            break;
+    constexpr int W = G / 32, kAhead = 12;
+    const int lane = g.rank & 31, warp = g.rank >> 5;
+    const int br = (lane >> 2) & 3, bc = lane & 3;
+    for (int i = g.rank; i < n; i += G) piv[i] = i;
+    if (warp == 0) {
+        const int size = n < 4 ? n : 4;
+        const bool in = br < size && bc < size;
+        MT a = in ? A[br * ld + bc] : MT(0);
+        const int from = lu_diagonal_block<MT>(a, size, invD, lane);
+        if (in && lane < 16) A[br * ld + bc] = a;
+        if (lane < 16 && bc == 0) work[br] = from;
+    }
+    g.sync();
+    for (int k0 = 0; k0 < n; k0 += 4) {
+        const int size = n - k0 < 4 ? n - k0 : 4;
+        const int k1 = k0 + size, m = n - k1;
+        MT* P = A + k0 * ld + k0;  // the diagonal block
+        const int f0 = work[0], f1 = work[1], f2 = work[2], f3 = work[3];
+        const bool moved = f0 != 0 || f1 != 1 || (size > 2 && f2 != 2);
+        if (m > 0) {
+            const MT r0 = MT(invD[k0]), r1 = MT(invD[k0 + 1]), r2 = MT(invD[k0 + 2]), r3 = MT(invD[k0 + 3]);
+            const MT u01 = P[1], u02 = P[2], u03 = P[3], u12 = P[ld + 2], u13 = P[ld + 3], u23 = P[2 * ld + 3];
+            for (int i = k1 + g.rank; i < n; i += G) {
+                MT* x = A + i * ld + k0;
+                const MT l0 = x[0] * r0;
+                MT l1 = fma(-l0, u01, x[1]), l2 = fma(-l0, u02, x[2]), l3 = fma(-l0, u03, x[3]);
+                l1 *= r1;
+                l2 = fma(-l1, u12, l2);
+                l3 = fma(-l1, u13, l3);
+                l2 *= r2;
+                l3 = fma(-l2, u23, l3);
+                x[0] = l0; x[1] = l1; x[2] = l2; x[3] = l3 * r3;
+            }
         }
-        // One thread picks the pivot row and the reciprocal of the pivot
-        // (read from that row before the interchange) and publishes both
-        // through piv[k] / invD[k]: the FP64 division and compares are issued
-        // once per column, not by every warp of the group.
-        if (g.rank == 0) {
-            const int pr = choose_pivot(A, ld, k, pos, size);
-            double akk = double(A[(size_t)pr * ld + k]);
-            if (akk == 0) akk = kPivEps;
-            invD[k] = double(MT(1.0 / akk));
-            piv[k] = pr;
+        if (m > 0 || moved) {
+            // columns right of the panel, and with an interchange those left of it
+            MT l10 = 0, l20 = 0, l21 = 0, l30 = 0, l31 = 0, l32 = 0;
+            if (m > 0) {
+                l10 = P[ld];
+                l20 = P[2 * ld]; l21 = P[2 * ld + 1];
+                l30 = P[3 * ld]; l31 = P[3 * ld + 1]; l32 = P[3 * ld + 2];
+            }
+            // the rows above took the first m threads: start with the next warp
+            const int first = G == 32 ? g.rank : (g.rank + G - ((m + 31) & ~31) % G) % G;
+            const int cols = moved ? m + k0 : m;
+            for (int t = first; t < cols; t += G) {
+                MT* x = A + k0 * ld + (t < m ? k1 + t : t - m);
+                MT x0 = x[f0 * ld], x1 = x[f1 * ld], x2 = size > 2 ? x[f2 * ld] : MT(0), x3 = size > 3 ? x[f3 * ld] : MT(0);
+                if (t < m) {
+                    x1 = fma(-l10, x0, x1);
+                    x2 = fma(-l21, x1, fma(-l20, x0, x2));
+                    x3 = fma(-l32, x2, fma(-l31, x1, fma(-l30, x0, x3)));
+                }
+                x[0] = x0;
+                x[ld] = x1;
+                if (size > 2) x[2 * ld] = x2;
+                if (size > 3) x[3 * ld] = x3;
+            }
+            if (moved && g.rank == G - 1) {
+                const int q0 = piv[k0 + f0], q1 = piv[k0 + f1], q2 = size > 2 ? piv[k0 + f2] : 0,
+                          q3 = size > 3 ? piv[k0 + f3] : 0;
+                piv[k0] = q0;
+                piv[k0 + 1] = q1;
+                if (size > 2) piv[k0 + 2] = q2;
+                if (size > 3) piv[k0 + 3] = q3;
+            }
         }
         g.sync();
-        const int p = piv[k];
-        const MT rinv = MT(invD[k]);
-        if (p != k) {
-            MT* rk = A + (size_t)k * ld;
-            MT* rp = A + (size_t)p * ld;
-            for (int j = g.rank; j < n; j += G) { const MT t = rk[j]; rk[j] = rp[j]; rp[j] = t; }
-            g.sync();
+        if (m == 0) break;
+        const int next = m < 4 ? m : 4;
+        const int iters = (m * m + 31) >> 5;
+        int share = iters;  // warp 0's
+        if constexpr (W > 1) {
+            share = (iters - kAhead * (W - 1)) / W;
+            share = share > 0 ? share : 0;
         }
-        for (int i = k + 1 + g.rank; i < n; i += G) A[(size_t)i * ld + k] *= rinv;
-        g.sync();
-        const MT* rk = A + (size_t)k * ld;
-        for (int i = k + 1 + tr; i < n; i += TR) {
-            MT* ri = A + (size_t)i * ld;
-            const MT l = ri[k];
-            for (int j = k + 1 + tc; j < n; j += TC) ri[j] = fma(-l, rk[j], ri[j]);
+        if (warp == 0) {
+            const bool in = br < next && bc < next;
+            MT a = MT(0);
+            MT* x = A + (k1 + br) * ld + k1 + bc;
+            if (in) a = lu_rank4(A + (k1 + br) * ld + k0, A + k0 * ld + k1 + bc, ld, *x);
+            const int from = lu_diagonal_block<MT>(a, next, invD + k1, lane);
+            if (in && lane < 16) *x = a;
+            if (lane < 16 && bc == 0) work[br] = from;
+        }
+        {
+            // two elements per step: the loads of the second overlap the
+            // first's chain of multiply-adds
+            const int it1 = warp == 0 ? share : iters, by = warp == 0 ? 1 : W - 1;
+            int it = warp == 0 ? 0 : share + warp - 1;
+            int i = (it * 32 + lane) / m, j = it * 32 + lane - i * m;
+            const int di = (32 * by) / m, dj = 32 * by - di * m;
+            #pragma unroll 1
+            for (; it < it1; it += 2 * by) {
+                int i2 = i + di, j2 = j + dj;
+                if (j2 >= m) { j2 -= m; i2++; }
+                const bool one = i < m && !(i < next && j < next);
+                const bool two = it + by < it1 && i2 < m && !(i2 < next && j2 < next);
+                MT* x = A + (k1 + i) * ld + k1 + j;
+                MT* x2 = A + (k1 + i2) * ld + k1 + j2;
+                MT v = 0, v2 = 0;
+                if (one) v = lu_rank4(A + (k1 + i) * ld + k0, A + k0 * ld + k1 + j, ld, *x);
+                if (two) v2 = lu_rank4(A + (k1 + i2) * ld + k0, A + k0 * ld + k1 + j2, ld, *x2);
+                if (one) *x = v;
+                if (two) *x2 = v2;
+                i = i2 + di;
+                j = j2 + dj;
+                if (j >= m) { j -= m; i++; }
+            }
         }
         g.sync();
     }
-    // The interchange sequence as one gather permutation (P b)[i] = b[perm[i]]
-    // for the solves, built in the slot scratch and written over piv.
-    for (int i = g.rank; i < n; i += G) work[i] = i;
-    g.sync();
-    if (g.rank == 0) {
-        for (int j = 0; j < n; j++) {
-            const int pj = piv[j];
-            if (pj != j) { const int t = work[j]; work[j] = work[pj]; work[pj] = t; }
-        }
-    }
-    g.sync();
-    for (int i = g.rank; i < n; i += G) piv[i] = work[i];
-    g.sync();
 }
 
 // Forward/back substitution with the factors of lu_factor after the row

@@ -21,6 +21,7 @@
 #include "fcs_internal.h"
 #include "fcs_lane_layout.h"
 #include "fcs_launch.h"
+#include "fcs_lists.h"
 #include "fcs_ctx.h"
 
 using namespace fcs;
@@ -132,6 +133,7 @@ extern "C" fcs_status fcs_destroy(fcs_ctx* ctx) {
                             &ctx->bSub, &ctx->bRR, &ctx->bDt, &ctx->bOut, &ctx->bJ, &ctx->bQ})
         b->release();
     ctx->dRx.release();
+    ctx->dLists.release();
     ctx->dPlogOff.release(); ctx->dIncOff.release(); ctx->dInc.release(); ctx->dTbInc.release();
     ctx->bStatus.release(); ctx->bOrder.release(); ctx->bHead.release();
     ctx->bStats.release(); ctx->bMin.release(); ctx->gws.release(); ctx->bBin.release(); ctx->bAtt.release();
@@ -329,6 +331,24 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
         incv.insert(incv.end(), inc[i].begin(), inc[i].end());
     }
     if (incv.empty()) incv.push_back(0);
+    for (const auto& v : inc)  // a sum's length has 16 bits in the lists, a Jacobian element's terms two per entry
+        if (v.size() > 32767) return set_err(ctx, FCS_ERR_UNSUPPORTED, "a species takes part in too many reactions");
+    int spBegin = 0, nSp = 0;
+    for (int k = 0; k < nr; k++)
+        if (rx[k].fo >= 0 || rx[k].nq >= 0) {
+            if (nSp == 0) spBegin = k;
+            nSp = k + 1 - spBegin;
+        }
+    const HostLists lists = build_lists(ns, rx, nr, inc, spBegin, nSp);
+    std::vector<double> wiw((size_t)ns * ns);
+    for (int i = 0; i < ns; i++)
+        for (int j = 0; j < ns; j++) wiw[(size_t)i * ns + j] = W[i] * invW[j];
+    ListBlock at;
+    at.ev = at.put(lists.ev);
+    at.wiw = at.put(wiw);
+    at.prod = at.put(lists.prod);
+    for (int v = 0; v < kJacVariants; v++)
+        at.jac[v] = ListBlock::Jac{at.put(lists.jac[v].ev), at.put(lists.jac[v].chunk), at.put(lists.jac[v].sums)};
     const int nTbInc = (int)tbInc.size();
     if (tbInc.empty()) tbInc.push_back(0);
     if (nTB >= 32768) return set_err(ctx, FCS_ERR_UNSUPPORTED, "too many third-body reactions");
@@ -345,6 +365,7 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
     CK(up(ctx->dRx, rx)); CK(up(ctx->dEff, eff)); CK(up(ctx->dPlogOff, plogOff));
     CK(up(ctx->dPlogRow, plogRow)); CK(up(ctx->dPlogTa, plogTa)); CK(up(ctx->dIncOff, incOff));
     CK(up(ctx->dInc, incv)); CK(up(ctx->dHf, hf)); CK(up(ctx->dTbInc, tbInc)); CK(up(ctx->dFo, fo));
+    CK(up(ctx->dLists, at.bytes));
     DevMech& M = ctx->M;
     M.ns = ns; M.n = ns + 1; M.nr = nr; M.nTB = nTB; M.nPlog = nPlog;
     M.TlowMin = TlowMin; M.ThighMax = ThighMax; M.TcommonMin = TcMin; M.TcommonMax = TcMax;
@@ -355,13 +376,21 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
     M.fo = ctx->dFo.p;
     // the special block: first to last non-equilibrium or fall-off reaction
     // (third-body reactions between them included)
-    M.spBegin = 0;
-    M.nSp = 0;
-    for (int k = 0; k < nr; k++)
-        if (rx[k].fo >= 0 || rx[k].nq >= 0) {
-            if (M.nSp == 0) M.spBegin = k;
-            M.nSp = k + 1 - M.spBegin;
-        }
+    M.spBegin = spBegin;
+    M.nSp = nSp;
+    M.ev = reinterpret_cast<const RxnEv*>(ctx->dLists.p + at.ev);
+    M.evThird = lists.evThird;
+    M.evSpecial = lists.evSpecial;
+    M.wiw = reinterpret_cast<const double*>(ctx->dLists.p + at.wiw);
+    M.prod = at.sums(ctx->dLists.p, at.prod, lists.prod);
+    for (int v = 0; v < kJacVariants; v++) {
+        const HostChunks& j = lists.jac[v];
+        M.jac[v].size = j.size;
+        M.jac[v].values = j.values;
+        M.jac[v].ev = reinterpret_cast<const RxnEv*>(ctx->dLists.p + at.jac[v].ev);
+        M.jac[v].chunk = reinterpret_cast<const JacChunk*>(ctx->dLists.p + at.jac[v].chunk);
+        M.jac[v].sums = at.sums(ctx->dLists.p, at.jac[v].sums, j.sums);
+    }
     ctx->loaded = true;
     ctx->tuned.clear();
     if (ctx->gexec) {  // a captured step holds the old mechanism's scalars
@@ -446,22 +475,21 @@ bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, Shape& sh) {
         r.cells = r.gpb * r.perSM;
         return r;
     };
-    // One chunk of reactions unless smaller chunks let more cells reside;
-    // then the largest chunk (a multiple of the group size) that does.
-    const int nr = std::max(1, ctx->M.nr);
-    auto layout = [&](int rc) { return make_layout(ctx->M.ns, ctx->M.nr, ctx->M.nTB, mixed, seulex, rc); };
-    sh.L = layout(nr);
-    Res res = residency(sh.L);
-    if (!res.global && nr > group) {
-        const Res best = residency(layout(group));
-        if (!best.global && best.cells > res.cells) {
-            for (int rc = ((nr - 1) / group) * group; rc >= group; rc -= group) {
-                const SlotLayout L = layout(rc);
-                const Res r = residency(L);
-                if (r.cells == best.cells) { sh.L = L; res = r; break; }
-            }
-        }
+    // The largest Jacobian chunk that does not cost a resident cell: larger
+    // chunks fill more threads and need fewer barriers.  53 species at 64
+    // threads: chunks of 64 reactions (3 KB of values) keep six cells per SM,
+    // chunks of 256 (12 KB) would keep four.
+    Res res{};
+    for (int v = kJacVariants - 1; v >= 0; v--) {
+        const SlotLayout L = make_layout(ctx->M.ns, ctx->M.nr, ctx->M.nTB, mixed, seulex, 1,
+                                         std::max(ctx->M.nr, ctx->M.jac[v].values));
+        const Res r = residency(L);
+        if (v < kJacVariants - 1 && (r.global || (!res.global && r.cells <= res.cells))) continue;
+        sh.L = L;
+        sh.L.jv = v;
+        res = r;
     }
+    sh.L.rw = group;
     sh.global = res.global;
     sh.lc.block = group * res.gpb;
     if (sh.lc.block > maxThreads) return false;

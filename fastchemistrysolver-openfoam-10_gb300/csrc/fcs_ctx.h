@@ -80,6 +80,7 @@ struct fcs_ctx {
     fcs::DBuf<double> dW, dInvW, dTc, dCoef, dEff, dPlogRow, dPlogTa, dHf, dFo;
     fcs::DBuf<fcs::RxnInfo> dRx;
     fcs::DBuf<int> dPlogOff, dIncOff, dInc, dTbInc;
+    fcs::DBuf<char> dLists;                               // the cell groups' lists (fcs_lists.h), one block
     // options
     fcs_options opt{};
     // per-call buffers

@@ -87,29 +87,6 @@ __device__ __forceinline__ double gmax(const Grp<G>& g, double v, double* red) {
     }
 }
 
-// log(Tc) and 1/Tc for the whole group.  With several warps, thread 0
-// computes them and publishes them through red[44..45]; the caller's next
-// group reduction (which synchronises) makes them visible -- call
-// thermo_scalars_read after it.  A single warp computes them in every lane.
-template<int G>
-__device__ __forceinline__ void thermo_scalars_publish(const Grp<G>& g, double Tc, double* red) {
-    if constexpr (G > 32) {
-        if (g.rank == 0) { red[44] = log(Tc); red[45] = 1.0 / Tc; }
-    }
-}
-
-template<int G>
-__device__ __forceinline__ void thermo_scalars_read(const Grp<G>& g, double Tc, const double* red, double& logT,
-                                                    double& invT) {
-    if constexpr (G > 32) {
-        logT = red[44];
-        invT = red[45];
-    } else {
-        logT = log(Tc);
-        invT = 1.0 / Tc;
-    }
-}
-
 // Two maxima at once of non-negative values (or NaN, which wins), compared
 // as integers on their bit patterns: the order of non-negative doubles is the
 // order of their bits, and NaN patterns sit above +inf.  No FP64 compares.
@@ -142,6 +119,32 @@ __device__ __forceinline__ void gmax2_nonneg(const Grp<G>& g, double& a, double&
 }
 
 // ------------------------------------------------------------------------
+// Comparisons on the integer pipe.  An FP64 compare, minimum or maximum holds
+// a scheduler as long as a multiply-add does (64 cycles); the order of
+// doubles of one sign is the order of their bits, and NaN patterns sit above
+// infinity.
+
+__device__ __forceinline__ bool ordered(long long magnitude) { return magnitude <= 0x7ff0000000000000LL; }
+
+// x > 0
+__device__ __forceinline__ bool positive(double x) {
+    const long long b = __double_as_longlong(x);
+    return b > 0 && ordered(b);
+}
+
+// a < b for b >= 0 or NaN
+__device__ __forceinline__ bool less_than(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return x < y && ordered(y) && ordered(x & 0x7fffffffffffffffLL);
+}
+
+// a <= b for b > 0 or NaN
+__device__ __forceinline__ bool at_most(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return x <= y && ordered(y) && ordered(x & 0x7fffffffffffffffLL);
+}
+
+// ------------------------------------------------------------------------
 // slot layout (byte offsets inside one cell's workspace)
 
 struct SlotLayout {
@@ -154,12 +157,14 @@ struct SlotLayout {
     int offInvD;       // [n] double
     int offScale;      // row / column equilibration factors [2n] double (mixed precision)
     int offPiv;        // [n] int
-    int offRx;         // Kf, Kr, q, dqdT [rc] each: one chunk of reactions
-    int rc;            // reactions per chunk (at most nr)
-    int offCur;        // [ns] int: per-species incidence cursor across chunks
+    int offRx;         // max(4 rc, values) doubles: the net rates, or one Jacobian chunk (fcs_lists.h)
+    int rc;
+    int offCur;        // [ns] int scratch
+    int jv;            // Jacobian chunking (kJacChunk) the region at offRx holds
+    int rw;            // threads that carry the partial sums of the group's reductions
     int offTb;         // M (third-body concentration), third-body column weight [nTB] each
     int offTable;      // Seulex extrapolation table [12][n] doubles
-    int offRed;        // 48 doubles of reduction / broadcast scratch
+    int offRed;        // 48 doubles of reduction / broadcast scratch (32..36 thermo scalars, 37 log p, 38 LU)
     int bytes;         // total, multiple of 16
 };
 
@@ -173,9 +178,10 @@ __host__ __device__ inline int align16(int x) { return (x + 15) & ~15; }
 //   mixed Rosenbrock: FP32 Jacobian + FP32 LU; the FP64 view (Jacobian assembly in
 //                     FP64, and the FP64 fallback attempt) overlays both
 //   mixed Seulex    : as FP64 Seulex, with the two FP32 matrices inside the FP64 Jacobian
-// rc: reactions per chunk (clamped to [1, nr]); the host picks it so that the
-// chunks are no smaller than needed for the most cells per SM.
-__host__ __device__ inline SlotLayout make_layout(int ns, int nr, int nTB, bool mixed, bool seulex, int rc) {
+// values: doubles wanted at offRx; rc: a quarter of the least there (clamped
+// to [1, nr]).
+__host__ __device__ inline SlotLayout make_layout(int ns, int nr, int nTB, bool mixed, bool seulex, int rc,
+                                                  int values = 0) {
     SlotLayout L;
     const int n = ns + 1;
     L.ld = n | 1;
@@ -194,13 +200,16 @@ __host__ __device__ inline SlotLayout make_layout(int ns, int nr, int nTB, bool 
     L.offScale = o; if (mixed) o = align16(o + 2 * n * 8);
     L.offPiv = o;   o = align16(o + n * 4);
     L.rc = rc < 1 ? 1 : (nr > 0 && rc > nr ? nr : rc);
-    L.offRx = o;    o = align16(o + (4 * L.rc * 8 > n * 4 ? 4 * L.rc * 8 : n * 4));  // also the LU's permutation scratch
+    const int rx = 4 * L.rc > values ? 4 * L.rc : values;
+    L.offRx = o;    o = align16(o + (rx * 8 > n * 4 ? rx * 8 : n * 4));  
     L.offCur = o;   o = align16(o + ns * 4);
     L.offTb = o;    o = align16(o + 2 * (nTB > 0 ? nTB : 1) * 8);
     L.offTable = o;
     if (seulex) o = align16(o + 12 * n * 8);
     L.offRed = o;   o = align16(o + 48 * 8);
     L.bytes = o;
+    L.jv = 0;
+    L.rw = 0;
     return L;
 }
 
@@ -216,9 +225,9 @@ struct Slot {
     double* invD;
     double *dr, *dc;
     int* piv;
-    double *Kf, *Kr, *q, *dqdT;   // one chunk of reactions: index r - c0
-    int rc;                        // reactions per chunk
-    int* cur;                      // per-species incidence cursor
+    double* q;                     // net rates by packed reaction, or a Jacobian chunk's values
+    int* cur;                      // ns ints of scratch
+    int jv, rw;
     double *Mtb, *tbF;
     double* table;
     double* red;
@@ -247,9 +256,9 @@ __device__ __forceinline__ Slot<MT> make_slot(char* base, const SlotLayout& L, c
     s.dr = reinterpret_cast<double*>(base + L.offScale);
     s.dc = s.dr + M.n;
     s.piv = reinterpret_cast<int*>(base + L.offPiv);
-    double* rx = reinterpret_cast<double*>(base + L.offRx);
-    s.rc = L.rc;
-    s.Kf = rx; s.Kr = rx + L.rc; s.q = rx + 2 * L.rc; s.dqdT = rx + 3 * L.rc;
+    s.q = reinterpret_cast<double*>(base + L.offRx);
+    s.jv = L.jv;
+    s.rw = L.rw;
     s.cur = reinterpret_cast<int*>(base + L.offCur);
     double* tb = reinterpret_cast<double*>(base + L.offTb);
     const int nt = M.nTB > 0 ? M.nTB : 1;
@@ -265,9 +274,9 @@ __device__ __forceinline__ Slot<MT> make_slot(char* base, const SlotLayout& L, c
 __device__ __forceinline__ const double* species_coeffs(const DevMech& M, int i, double Tb) {
     // setPtrCoeffs (ThermoFunctionI.H:1-31)
     const double* base = M.coef + 16 * i;
-    if (Tb < M.TcommonMin) return base;
-    if (Tb > M.TcommonMax) return base + 8;
-    return (Tb < __ldg(&M.Tcommon[i])) ? base : base + 8;
+    if (less_than(Tb, M.TcommonMin)) return base;
+    if (less_than(M.TcommonMax, Tb)) return base + 8;
+    return less_than(Tb, __ldg(&M.Tcommon[i])) ? base : base + 8;
 }
 
 struct Nasa { double a0, a1, a2, a3, a4, a5, a6; };
@@ -307,8 +316,8 @@ __device__ __forceinline__ double ha_of(const Nasa& a, double T, double RuInvW) 
 }
 
 __device__ __forceinline__ double clampT(const DevMech& M, double T) {
-    T = T < M.TlowMin ? M.TlowMin : T;
-    T = T > M.ThighMax ? M.ThighMax : T;
+    T = less_than(T, M.TlowMin) ? M.TlowMin : T;
+    T = less_than(M.ThighMax, T) ? M.ThighMax : T;
     return T;
 }
 
@@ -342,7 +351,8 @@ __device__ const double kExp2Table[64] = {
     1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951};
 
 __device__ __forceinline__ double fast_exp(double x) {
-    if (!(fabs(x) <= 707.0)) return exp(x);
+    // |x| <= 707 (0x4086180000000000), false for NaN
+    if ((__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x4086180000000000LL) return exp(x);
     const double kInvL = 92.33248261689366;          // 64/ln2
     const double kL1 = 0.010830424696223417;         // head of ln2/64 (36 bits)
     const double kL2 = 2.572804622327669e-14;        // tail
@@ -399,7 +409,8 @@ __device__ __forceinline__ double pressure_factor(const PFactor& pf, int dnu) {
 }
 
 // The clamp of 1/Kc: RFG/JFG (more than 3 species on a side) use the other constant
-__device__ __forceinline__ double inv_kc_clamp(const RxnInfo& x) {
+template<class Rxn>
+__device__ __forceinline__ double inv_kc_clamp(const Rxn& x) {
     return (x.nl > 3 || x.nr > 3) ? kInvKcClampG : kInvKcClamp;
 }
 
@@ -418,7 +429,7 @@ __device__ __forceinline__ double inv_equilibrium_kc(const RxnInfo& x, const dou
     for (int q = 0; q < x.nr; q++) v *= Einv[x.sr[q]];
     if (x.dnu != 0) v *= pressure_factor(pf, x.dnu);
     const double cl = inv_kc_clamp(x);
-    return v > cl ? cl : v;
+    return less_than(cl, v) ? cl : v;
 }
 
 // ------------------------------------------------------------------------
@@ -432,11 +443,11 @@ __device__ __forceinline__ double plog_rate(const DevMech& M, int ip, double p, 
     const int len = __ldg(&M.plogOff[ip + 1]) - o;
     const double* R = M.plogRow;
     double lk, dk;
-    if (p <= __ldg(&R[4 * o])) {
+    if (at_most(p, __ldg(&R[4 * o]))) {
         const double la = __ldg(&R[4 * o + 2]), b = __ldg(&R[4 * o + 3]), ta = __ldg(&M.plogTa[o]);
         lk = la + b * logT - ta * invT;
         dk = (b + ta * invT) * invT;
-    } else if (p >= __ldg(&R[4 * (o + len - 1)])) {
+    } else if (at_most(__ldg(&R[4 * (o + len - 1)]), p)) {
         const int e = o + len - 1;
         const double la = __ldg(&R[4 * e + 2]), b = __ldg(&R[4 * e + 3]), ta = __ldg(&M.plogTa[e]);
         lk = la + b * logT - ta * invT;
@@ -444,7 +455,7 @@ __device__ __forceinline__ double plog_rate(const DevMech& M, int ip, double p, 
     } else {
         int idx = 0;
         for (int j = 0; j < len - 1; j++) {
-            if (__ldg(&R[4 * (o + j)]) <= p && p <= __ldg(&R[4 * (o + j + 1)])) { idx = j; break; }
+            if (at_most(__ldg(&R[4 * (o + j)]), p) && at_most(p, __ldg(&R[4 * (o + j + 1)]))) { idx = j; break; }
         }
         const int a = o + idx, b = a + 1;
         const double lpa = __ldg(&R[4 * a + 1]), lpb = __ldg(&R[4 * b + 1]);
@@ -619,92 +630,207 @@ static __device__ __forceinline__ SpecialK special_rates(const DevMech& M, const
 }
 
 // ------------------------------------------------------------------------
-// Reactions are evaluated in chunks of s.rc so that the per-reaction arrays
-// of a cell slot hold one chunk, not the whole mechanism, where that lets
-// more cells reside per SM (otherwise one chunk holds every reaction).  Every sum keeps its order: a species' terms
-// are added in reaction order across the chunks, its incidence cursor
-// (s.cur) carrying over from one chunk to the next.
+// Thermo scalars of one evaluation: log Tc, 1/Tc, num/p, Pstd/(Ru Tc) and its
+// inverse.  A logarithm is 31 FP64 instructions and a division 8, and an
+// instruction costs the same for one lane as for 32, so one warp takes the
+// logarithm and another the divisions, side by side in its lanes, and a
+// barrier (cheaper than one of those instructions) publishes them.
 
-// Net rates q of the reactions [c0, c1) into s.q[r - c0] (ReactionRate.C:521-575
-// and the RF* functions).  The special block [spBegin, spBegin + nSp) of the
-// packed order (first non-equilibrium to last fall-off reaction) runs in a
-// loop of its own, so that the main loop carries neither the fall-off call
-// nor a second Arrhenius.
-template<int G, class MT>
-__device__ __forceinline__ void net_rates_chunk(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double p,
-                                                double logP, double Tc, double logT, double invT,
-                                                const PFactor& pf, int c0, int c1) {
-    const int sp0 = M.spBegin, sp1 = M.spBegin + M.nSp;
-    auto finish = [&](const int r, const RxnInfo& x, const double Kf, const double Kr) {
-        double CF = s.C[x.sl[0]];
-        #pragma unroll 1
-        for (int q = 1; q < x.nl; q++) CF *= s.C[x.sl[q]];
-        double CR = s.C[x.sr[0]];
-        #pragma unroll 1
-        for (int q = 1; q < x.nr; q++) CR *= s.C[x.sr[q]];
-        s.q[r - c0] = Kf * CF - Kr * CR;
-    };
-    for (int r = c0 + g.rank; r < c1; r += G) {
-        if (r >= sp0 && r < sp1) continue;
-        const RxnInfo x = load_rx(M.rx + r);
-        double Kf;
-        if (x.kind == FCS_RXN_PLOG) {
-            double dk;
-            Kf = plog_rate(M, x.plog, p, logP, logT, invT, &dk);
-        } else if (x.tind) {
-            Kf = x.A;
+struct ThermoScalars { double logT, invT, numByP; PFactor pf; };
+
+template<int G>
+__device__ __forceinline__ ThermoScalars thermo_scalars(const Grp<G>& g, double* red, double Tc, double num, double p) {
+    const int lane = g.rank & 31, warp = g.rank >> 5;
+    ThermoScalars t;
+    if (G == 32 || warp == 1) {
+        const double q = (lane == 0 ? 1.0 : lane == 1 ? num : kRu * Tc) / (lane == 0 ? Tc : lane == 1 ? p : kPstd);
+        const double inv = 1.0 / q;
+        if constexpr (G == 32) {
+            t.invT = __shfl_sync(0xffffffffu, q, 0);
+            t.numByP = __shfl_sync(0xffffffffu, q, 1);
+            t.pf.invP = __shfl_sync(0xffffffffu, q, 2);
+            t.pf.P = __shfl_sync(0xffffffffu, inv, 2);
         } else {
-            Kf = x.A * fast_exp(fma(x.beta, logT, -(x.Ta * invT)));
+            if (lane < 3) red[33 + lane] = q;
+            if (lane == 2) red[36] = inv;
         }
-        if (x.tb >= 0) Kf *= s.Mtb[x.tb];
-        double Kr = 0;
-        if (x.rev) Kr = Kf * inv_equilibrium_kc(x, s.B, s.Binv, pf);
-        finish(r, x, Kf, Kr);
     }
-    for (int r = max(c0, sp0) + g.rank; r < min(c1, sp1); r += G) {
-        const RxnInfo x = load_rx(M.rx + r);
-        const SpecialK k = special_rates(M, x, s.Mtb, Tc, logT, invT, false);
-        double Kr = k.Kr;  // non-equilibrium: its own reverse rate
-        if (x.rev == 1) Kr = k.Kf * inv_equilibrium_kc(x, s.B, s.Binv, pf);
-        finish(r, x, k.Kf, Kr);
+    if (G == 32 || warp == 0) {
+        const double l = log(Tc);
+        if constexpr (G == 32) t.logT = l;
+        else if (lane == 0) red[32] = l;
     }
-}
-
-// acc[i] += the net rates of the chunk [c0, c1) for species i (+q as a
-// product, -q as a reactant), in reaction order.
-template<int G, class MT>
-__device__ __forceinline__ void gather_chunk(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, int c0, int c1,
-                                             double* acc) {
-    for (int i = g.rank; i < M.ns; i += G) {
-        double w = acc[i];
-        int e = s.cur[i];
-        const int e1 = __ldg(&M.incOff[i + 1]);
-        for (; e < e1; e++) {
-            const int v = __ldg(&M.inc[e]);
-            if ((v >> 1) >= c1) break;
-            const double qq = s.q[(v >> 1) - c0];
-            w = (v & 1) ? w + qq : w - qq;
-        }
-        s.cur[i] = e;
-        acc[i] = w;
-    }
-}
-
-// Sum over the chunks: acc[i] = w_i for every species.
-template<int G, class MT>
-__device__ __forceinline__ void net_production(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double p,
-                                               double logP, double Tc, double logT, double invT,
-                                               const PFactor& pf, double* acc) {
-    for (int i = g.rank; i < M.ns; i += G) {
-        s.cur[i] = __ldg(&M.incOff[i]);
-        acc[i] = 0.0;
-    }
-    for (int c0 = 0; c0 < M.nr; c0 += s.rc) {
-        const int c1 = min(M.nr, c0 + s.rc);
-        net_rates_chunk<G, MT>(g, M, s, p, logP, Tc, logT, invT, pf, c0, c1);
+    if constexpr (G > 32) {
         g.sync();
-        gather_chunk<G, MT>(g, M, s, c0, c1, acc);
-        if (c1 < M.nr) g.sync();  // the next chunk overwrites q
+        t.logT = red[32];
+        t.invT = red[33];
+        t.numByP = red[34];
+        t.pf.invP = red[35];
+        t.pf.P = red[36];
+    }
+    return t;
+}
+
+// M_t = sum_j eff[t][j] C_j (ThirdBodyFactor1D)
+template<int G, class MT>
+__device__ __forceinline__ void third_bodies(const Grp<G>& g, const DevMech& M, const Slot<MT>& s) {
+    const int ns = M.ns;
+    for (int t = g.rank; t < M.nTB; t += G) {
+        const double* e = M.eff + (size_t)t * ns;
+        double m = 0;
+        #pragma unroll 8
+        for (int j = 0; j < ns; j++) m = fma(__ldg(&e[j]), s.C[j], m);
+        s.Mtb[t] = m;
+    }
+}
+
+// ------------------------------------------------------------------------
+// reactions, one per thread, from the sorted records of fcs_lists.h
+
+__device__ __forceinline__ RxnEv load_ev(const RxnEv* p) {
+    RxnEv x;
+    const double2* s = reinterpret_cast<const double2*>(p);
+    double2* d = reinterpret_cast<double2*>(&x);
+    d[0] = __ldg(s);
+    d[1] = __ldg(s + 1);
+    d[2] = __ldg(s + 2);
+    d[3] = __ldg(s + 3);
+    return x;
+}
+
+// The values of X at the first three slots of a side; unused slots hold
+// species 0, so that the three loads go out together.
+struct Three { double a, b, c; };
+__device__ __forceinline__ Three load3(const double* X, const uint8_t* s) { return Three{X[s[0]], X[s[1]], X[s[2]]}; }
+__device__ __forceinline__ double product3(const Three& t, int k) {
+    double v = t.a;
+    if (k > 1) v *= t.b;
+    if (k > 2) v *= t.c;
+    return v;
+}
+__device__ __forceinline__ bool three_at_most(const RxnEv& x) { return x.nl <= 3 && x.nr <= 3; }
+
+__device__ __forceinline__ double product_over(const double* X, const uint8_t* s, int k) {
+    double v = X[s[0]];
+    #pragma unroll 1
+    for (int q = 1; q < k; q++) v *= X[s[q]];
+    return v;
+}
+
+// 1/Kc = prod_reactants E prod_products 1/E (Pstd/(Ru T))^-dnu, clamped as
+// inv_equilibrium_kc clamps it (ReactionFunctionI.H:17)
+__device__ __forceinline__ double inverse_kc(const RxnEv& x, const double* E, const double* Einv, const PFactor& pf) {
+    double v;
+    if (three_at_most(x)) {
+        const Three e = load3(E, x.sl), i = load3(Einv, x.sr);
+        v = product3(e, x.nl);
+        v *= i.a;
+        if (x.nr > 1) v *= i.b;
+        if (x.nr > 2) v *= i.c;
+    } else {
+        v = product_over(E, x.sl, x.nl);
+        #pragma unroll 1
+        for (int q = 0; q < x.nr; q++) v *= Einv[x.sr[q]];
+    }
+    if (x.nr != x.nl) v *= pressure_factor(pf, x.nr - x.nl);
+    const double cl = inv_kc_clamp(x);
+    return less_than(cl, v) ? cl : v;
+}
+
+// Forward rate constant without third bodies; dkdT its temperature derivative
+__device__ __forceinline__ double forward_k(const DevMech& M, const RxnEv& x, double p, double logP, double logT,
+                                            double invT, double* dkdT) {
+    if (x.plog >= 0) return plog_rate(M, x.plog, p, logP, logT, invT, dkdT);
+    double Kf = x.A;
+    *dkdT = 0;
+    if (!x.tind) {
+        Kf = x.A * fast_exp(fma(x.beta, logT, -(x.Ta * invT)));
+        *dkdT = Kf * (fma(x.Ta, invT, x.beta) * invT);
+    }
+    return Kf;
+}
+
+template<class MT>
+__device__ __forceinline__ double net_rate(const Slot<MT>& s, const RxnEv& x, double Kf, double Kr) {
+    double CF, CR;
+    if (three_at_most(x)) {
+        const Three a = load3(s.C, x.sl), b = load3(s.C, x.sr);
+        CF = product3(a, x.nl);
+        CR = product3(b, x.nr);
+    } else {
+        CF = product_over(s.C, x.sl, x.nl);
+        CR = product_over(s.C, x.sr, x.nr);
+    }
+    return Kf * CF - Kr * CR;
+}
+
+// Net rates of all reactions into s.q (ReactionRate.C:521-575 and the RF*
+// functions), with the third-body concentrations: the plain reactions do not
+// wait for them.  The special block (first non-equilibrium to last fall-off
+// reaction) runs in a loop of its own, so that the others carry neither the
+// fall-off call nor a second Arrhenius.
+template<int G, class MT>
+__device__ __forceinline__ void net_rates(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double p, double logP,
+                                          double Tc, const ThermoScalars& t) {
+    third_bodies<G, MT>(g, M, s);
+    #pragma unroll 1
+    for (int part = 0; part < 2; part++) {
+        const int end = part ? M.evSpecial : M.evThird;
+        #pragma unroll 1
+        for (int k = (part ? M.evThird : 0) + g.rank; k < end; k += G) {
+            const RxnEv x = load_ev(M.ev + k);
+            double dk;
+            double Kf = forward_k(M, x, p, logP, t.logT, t.invT, &dk);
+            if (x.tb >= 0) Kf *= s.Mtb[x.tb];
+            double Kr = 0;
+            if (x.rev) Kr = Kf * inverse_kc(x, s.B, s.Binv, t.pf);
+            s.q[x.r] = net_rate(s, x, Kf, Kr);
+        }
+        if (part == 0) g.sync();
+    }
+    #pragma unroll 1
+    for (int k = M.evSpecial + g.rank; k < M.nr; k += G) {
+        const RxnEv x = load_ev(M.ev + k);
+        const RxnInfo xi = load_rx(M.rx + x.r);
+        const SpecialK c = special_rates(M, xi, s.Mtb, Tc, t.logT, t.invT, false);
+        double Kr = c.Kr;  // non-equilibrium: its own reverse rate
+        if (x.rev == 1) Kr = c.Kf * inverse_kc(x, s.B, s.Binv, t.pf);
+        s.q[x.r] = net_rate(s, x, c.Kf, Kr);
+    }
+}
+
+// v plus the terms of one lane's sum (n of them, of the group's most), in
+// order; four terms' loads are issued together, lanes that are done add 0.
+__device__ __forceinline__ double sum_terms(const uint32_t* __restrict__ con, int n, int most, const double* q,
+                                            double v) {
+    auto term = [&](uint32_t c, int k) {
+        const long long b = __double_as_longlong(q[c >> 1]) ^ ((long long)(~c & 1u) << 63);
+        return k < n ? __longlong_as_double(b) : 0.0;
+    };
+    int k = 0;
+    #pragma unroll 1
+    for (; k + 4 <= most; k += 4, con += 128) {
+        const uint32_t c0 = __ldg(con), c1 = __ldg(con + 32), c2 = __ldg(con + 64), c3 = __ldg(con + 96);
+        const double a = term(c0, k), b = term(c1, k + 1), c = term(c2, k + 2), d = term(c3, k + 3);
+        v += a;
+        v += b;
+        v += c;
+        v += d;
+    }
+    #pragma unroll 1
+    for (; k < most; k++, con += 32) v += term(__ldg(con), k);
+    return v;
+}
+
+// out[i] = net molar production of species i over s.q, in reaction order
+template<int G, class MT>
+__device__ __forceinline__ void net_production(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double* out) {
+    const int lane = g.rank & 31;
+    for (int k = g.rank >> 5; k < M.prod.groups; k += G / 32) {
+        const uint32_t e = __ldg(M.prod.elem + 32 * k + lane);
+        const int n = e & 0xffff, most = __shfl_sync(0xffffffffu, n, 0), i = e >> 16;
+        const double v = sum_terms(M.prod.con + __ldg(M.prod.off + k) + lane, n, most, s.q, 0.0);
+        if (i != 0xffff) out[i] = v;
     }
 }
 
@@ -712,32 +838,36 @@ __device__ __forceinline__ void net_production(const Grp<G>& g, const DevMech& M
 // right-hand side: FastChemistryModel::derivatives (FastChemistryModel.C:194-273
 // for mode 1, 340-417 for mode 2) over OptReaction::dNdtByV
 // (ReactionRate.C:732-1503).  YT is clamped (Y >= 0) in place.
+//
+// Bound by the count of FP64 warp instructions (19 cycles each per SM) when
+// the SM is full of cells and by their latency when it holds one.  Reactions
+// sorted by path, sums by length, scalars side by side, compares on integers:
+// 877 -> 735 instructions on 53 species with 64 threads, fcs_rhs on
+// 2,001 cells 0.19 -> 0.15 ms.
 
 template<int G, class MT>
 __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double p,
                          double* YT, double* out, int mode) {
     const int ns = M.ns;
+    const int r0 = g.rank < s.rw ? g.rank : ns;  // the threads that carry the partial sums
     const double T = YT[ns];
     const double Tc = clampT(M, T);
-    thermo_scalars_publish(g, Tc, s.red);
-    const double RuTByP = kRu * T / p;
+    const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * T, p);
     double part = 0;
-    for (int i = g.rank; i < ns; i += G) {
+    for (int i = r0; i < ns; i += s.rw) {
         const double y0 = YT[i];
-        const double y = y0 > 0 ? y0 : 0.0;
-        YT[i] = y;
-        part = fma(y * __ldg(&M.invW[i]), RuTByP, part);
+        part = fma((positive(y0) ? y0 : 0.0) * __ldg(&M.invW[i]), t.numByP, part);
     }
     const double invrhoM = gsum(g, part, s.red);
-    double logT, invT;
-    thermo_scalars_read(g, Tc, s.red, logT, invT);
     const double rhoM = 1.0 / invrhoM;
     const double Tp = mode == 2 ? T : Tc;
     for (int i = g.rank; i < ns; i += G) {
         const double invW = __ldg(&M.invW[i]);
-        s.C[i] = rhoM * invW * YT[i];
+        const double y0 = YT[i], y = positive(y0) ? y0 : 0.0;
+        YT[i] = y;
+        s.C[i] = rhoM * invW * y;
         const Nasa a = load_nasa(species_coeffs(M, i, Tc));
-        const double Ei = fast_exp(gibbs_exponent(a, Tc, invT, logT));
+        const double Ei = fast_exp(gibbs_exponent(a, Tc, t.invT, t.logT));
         s.B[i] = Ei;
         s.Binv[i] = 1.0 / Ei;
         const double RuInvW = invW * kRu;
@@ -745,22 +875,16 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
         s.Ha[i] = ha_of(a, Tp, RuInvW);
     }
     g.sync();
-    for (int t = g.rank; t < M.nTB; t += G) {
-        const double* e = M.eff + (size_t)t * ns;
-        double m = 0;
-        for (int j = 0; j < ns; j++) m = fma(__ldg(&e[j]), s.C[j], m);
-        s.Mtb[t] = m;
-    }
+    net_rates<G, MT>(g, M, s, p, s.red[37], Tc, t);
     g.sync();
-    const PFactor pf = pressure_factors(Tc);
-    const double logP = M.nPlog ? log(p) : 0.0;
-    net_production<G, MT>(g, M, s, p, logP, Tc, logT, invT, pf, out);
+    net_production<G, MT>(g, M, s, out);
+    g.sync();
+    for (int i = g.rank; i < ns; i += G) out[i] = (__ldg(&M.W[i]) * invrhoM) * out[i];
+    if (s.rw < G) g.sync();
     double cpm = 0, dtd = 0;
-    for (int i = g.rank; i < ns; i += G) {
-        const double dY = (__ldg(&M.W[i]) * invrhoM) * out[i];
-        out[i] = dY;
+    for (int i = r0; i < ns; i += s.rw) {
         cpm = fma(YT[i], s.Cp[i], cpm);
-        dtd = fma(s.Ha[i], dY, dtd);
+        dtd = fma(s.Ha[i], out[i], dtd);
     }
     gsum2(g, cpm, dtd, s.red);
     if (g.rank == 0) out[ns] = -dtd / cpm;
@@ -863,31 +987,23 @@ __device__ __noinline__ double rates_eval(const Grp<G>& g, const DevMech& M, con
                                           double p, double T, double rho, const double* Y, double* RR) {
     const int ns = M.ns;
     const double Tc = clampT(M, T);
-    const double logT = log(Tc), invT = 1.0 / Tc;
+    const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * Tc, p);
     for (int i = g.rank; i < ns; i += G) {
         s.C[i] = rho * Y[i] / __ldg(&M.W[i]);
         const Nasa a = load_nasa(species_coeffs(M, i, Tc));
-        const double Ei = fast_exp(gibbs_exponent(a, Tc, invT, logT));
+        const double Ei = fast_exp(gibbs_exponent(a, Tc, t.invT, t.logT));
         s.B[i] = Ei;
         s.Binv[i] = 1.0 / Ei;
     }
     g.sync();
-    for (int t = g.rank; t < M.nTB; t += G) {
-        const double* e = M.eff + (size_t)t * ns;
-        double m = 0;
-        for (int j = 0; j < ns; j++) m = fma(__ldg(&e[j]), s.C[j], m);
-        s.Mtb[t] = m;
-    }
+    net_rates<G, MT>(g, M, s, p, s.red[37], Tc, t);
     g.sync();
-    const PFactor pf = pressure_factors(Tc);
-    const double logP = M.nPlog ? log(p) : 0.0;
-    net_production<G, MT>(g, M, s, p, logP, Tc, logT, invT, pf, RR);
+    net_production<G, MT>(g, M, s, RR);
+    g.sync();
+    for (int i = g.rank; i < ns; i += G) RR[i] = RR[i] * __ldg(&M.W[i]);
+    if (s.rw < G) g.sync();
     double qd = 0;
-    for (int i = g.rank; i < ns; i += G) {
-        const double rr = RR[i] * __ldg(&M.W[i]);
-        RR[i] = rr;
-        qd -= __ldg(&M.hf[i]) * rr;
-    }
+    for (int i = g.rank < s.rw ? g.rank : ns; i < ns; i += s.rw) qd -= __ldg(&M.hf[i]) * RR[i];
     qd = gsum(g, qd, s.red);
     g.sync();
     return qd;
@@ -899,35 +1015,79 @@ __device__ __noinline__ double rates_eval(const Grp<G>& g, const DevMech& M, con
 // conversion (Jacobian.C:2814-2858 exact written as diagonal scaling plus a
 // rank-1 correction, 4541-4568 fast, 3709-3741 T column, 3743-3793 T row).
 // Writes J (row-major, leading dimension s.ld) and f = dy/dt; YT clamped in
-// place.  Accumulation happens in MT (double, or float in mixed precision);
-// rate constants, equilibrium constants and f stay double.
+// place.  With iterate, J receives the iteration matrix shift I - J instead.
+//
+// One thread evaluates a reaction with all its d q / d C; then every element
+// of the matrix that any reaction touches is one sum, as are the species'
+// net production (collected in the temperature row) and dq/dT (in the
+// temperature column).  The former column owners walked incidence lists of
+// unequal length in which reactants and products took different branches:
+// 3,011 FP64 warp instructions on 53 species with 64 threads, now 2,143, and
+// 2,000 such matrices 0.65 -> 0.50 ms.
+
+// d q / d C of every occurrence of x's species, into v (reactants, then
+// products when there is a reverse rate): the rate constant times the side's
+// other concentrations (the first slot of the same species left out)
+__device__ __forceinline__ void rate_gradients(const RxnEv& x, const double* C, double Kf, double Kr, double* v) {
+    if (three_at_most(x)) {
+        auto side = [&](const Three& c, int k, unsigned f1, unsigned f2, double K, double* o) {
+            double d = K;
+            if (k > 1) d *= c.b;
+            if (k > 2) d *= c.c;
+            o[0] = d;
+            if (k > 1) {
+                d = K * (f1 ? c.a : c.b);
+                if (k > 2) d *= c.c;
+                o[1] = d;
+            }
+            if (k > 2) o[2] = K * (f2 == 0 ? c.b : c.a) * (f2 == 2 ? c.b : c.c);
+        };
+        side(load3(C, x.sl), x.nl, x.first >> 2 & 3, x.first >> 4 & 3, Kf, v);
+        if (x.rev) side(load3(C, x.sr), x.nr, x.first >> 11 & 7, x.first >> 14 & 7, -Kr, v + x.nl);
+        return;
+    }
+    #pragma unroll 1
+    for (int a = 0; a < x.nl; a++) {
+        const int skip = x.first >> (2 * a) & 3;
+        double d = Kf;
+        #pragma unroll 1
+        for (int q = 0; q < x.nl; q++)
+            if (q != skip) d *= C[x.sl[q]];
+        v[a] = d;
+    }
+    if (!x.rev) return;
+    #pragma unroll 1
+    for (int a = 0; a < x.nr; a++) {
+        const int skip = x.first >> (8 + 3 * a) & 7;
+        double d = -Kr;
+        #pragma unroll 1
+        for (int q = 0; q < x.nr; q++)
+            if (q != skip) d *= C[x.sr[q]];
+        v[x.nl + a] = d;
+    }
+}
 
 template<int G, class MT>
 __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double p,
-                         double* YT, double* f, MT* J, int fast) {
+                         double* YT, double* f, MT* J, int fast, bool iterate, double shift) {
     const int ns = M.ns, n = M.n, ld = s.ld;
-    for (int i = g.rank; i < ns; i += G) {
-        const double y0 = YT[i];
-        YT[i] = y0 > 0 ? y0 : 0.0;
-    }
+    const int r0 = g.rank < s.rw ? g.rank : ns;
     const double T = YT[ns];
     const double Tc = clampT(M, T);
-    thermo_scalars_publish(g, Tc, s.red);
     // JacobianThermo (ThermoFunctionI.H:33-371) at the clamped temperature
-    const double RuTByP = (kRu * Tc) / p;
+    const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * Tc, p);
+    const double logT = t.logT, invT = t.invT;
     double rs = 0, mws = 0;
-    for (int i = g.rank; i < ns; i += G) {
-        const double y = YT[i], invW = __ldg(&M.invW[i]);
-        rs = fma(RuTByP, y * invW, rs);
+    for (int i = r0; i < ns; i += s.rw) {
+        const double y0 = YT[i], y = positive(y0) ? y0 : 0.0, invW = __ldg(&M.invW[i]);
+        rs = fma(t.numByP, y * invW, rs);
         mws = fma(y, invW, mws);
     }
     gsum2(g, rs, mws, s.red);
-    double logT, invT;
-    thermo_scalars_read(g, Tc, s.red, logT, invT);
     const double rhoM = 1.0 / rs, invRhoM = rs, MW = 1.0 / mws;
-    double cpm = 0, dcpm = 0;
     for (int i = g.rank; i < ns; i += G) {
-        const double y = YT[i], invW = __ldg(&M.invW[i]);
+        const double y0 = YT[i], y = positive(y0) ? y0 : 0.0, invW = __ldg(&M.invW[i]);
+        YT[i] = y;
         const Nasa a = load_nasa(species_coeffs(M, i, Tc));
         s.C[i] = rhoM * y * invW;
         const double Ei = fast_exp(gibbs_exponent(a, Tc, invT, logT));
@@ -936,84 +1096,76 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
         s.dBdT[i] = fma(fma(a.a5, invT, a.a0), invT,
                         fma(fma(fma(a.a4 * 0.2, Tc, a.a3 * 0.25), Tc, a.a2 * (1.0 / 3.0)), Tc, a.a1 * 0.5));
         const double RuInvW = invW * kRu;
-        const double cp = cp_of(a, Tc, RuInvW);
-        const double dcp = RuInvW * fma(Tc, fma(Tc, fma(Tc, 4 * a.a4, 3 * a.a3), 2 * a.a2), a.a1);
-        s.Cp[i] = cp;
-        s.dCpdT[i] = dcp;
+        s.Cp[i] = cp_of(a, Tc, RuInvW);
+        s.dCpdT[i] = RuInvW * fma(Tc, fma(Tc, fma(Tc, 4 * a.a4, 3 * a.a3), 2 * a.a2), a.a1);
         s.Ha[i] = ha_of(a, Tc, RuInvW);
-        cpm = fma(y, cp, cpm);
-        dcpm = fma(y, dcp, dcpm);
     }
-    gsum2(g, cpm, dcpm, s.red);
+    for (int idx = g.rank; idx < n * ld; idx += G) J[idx] = MT(0);
+    g.sync();
+    third_bodies<G, MT>(g, M, s);
+    if constexpr (G == 32) g.sync();
+    double cpm = 0, dcpm = 0;
+    for (int i = r0; i < ns; i += s.rw) {
+        cpm = fma(YT[i], s.Cp[i], cpm);
+        dcpm = fma(YT[i], s.dCpdT[i], dcpm);
+    }
+    gsum2(g, cpm, dcpm, s.red);  // its barriers publish the third bodies
     const double CpM = cpm, dCpMdT = dcpm;
-    g.sync();
-    for (int t = g.rank; t < M.nTB; t += G) {
-        const double* e = M.eff + (size_t)t * ns;
-        double m = 0;
-        for (int j = 0; j < ns; j++) m = fma(__ldg(&e[j]), s.C[j], m);
-        s.Mtb[t] = m;
-    }
-    g.sync();
-    // per-reaction rate constants, their temperature derivatives and q, one
-    // chunk of reactions at a time (see net_rates_chunk)
-    const PFactor pf = pressure_factors(Tc);
-    const double logP = M.nPlog ? log(p) : 0.0;
+    const double logP = s.red[37];
+    const JacLists& L = M.jac[s.jv];
+    const int size = L.size;
     // Kr, dKr/dT and dKr/dM through Kc (JF* reversible branch)
-    auto through_kc = [&](const RxnInfo& x, const double Kf, const double dKfdT, const double dKfdC,
+    auto through_kc = [&](const RxnEv& x, const double Kf, const double dKfdT, const double dKfdC,
                           double& Kr, double& dKrdT, double& dKrdC) {
-        const double invKc = inv_equilibrium_kc(x, s.B, s.Binv, pf);
-        double sv = s.dBdT[x.sr[0]];
-        #pragma unroll 1
-        for (int q = 1; q < x.nr; q++) sv += s.dBdT[x.sr[q]];
-        double sl = s.dBdT[x.sl[0]];
-        #pragma unroll 1
-        for (int q = 1; q < x.nl; q++) sl += s.dBdT[x.sl[q]];
-        const double dKcdTByKc = (sv - sl) - x.dnu * invT;
+        const double invKc = inverse_kc(x, s.B, s.Binv, t.pf);
+        double sv, sl;
+        if (three_at_most(x)) {
+            const Three v = load3(s.dBdT, x.sr), l = load3(s.dBdT, x.sl);
+            sv = v.a;
+            if (x.nr > 1) sv += v.b;
+            if (x.nr > 2) sv += v.c;
+            sl = l.a;
+            if (x.nl > 1) sl += l.b;
+            if (x.nl > 2) sl += l.c;
+        } else {
+            sv = s.dBdT[x.sr[0]];
+            #pragma unroll 1
+            for (int q = 1; q < x.nr; q++) sv += s.dBdT[x.sr[q]];
+            sl = s.dBdT[x.sl[0]];
+            #pragma unroll 1
+            for (int q = 1; q < x.nl; q++) sl += s.dBdT[x.sl[q]];
+        }
+        const double dKcdTByKc = (sv - sl) - (x.nr - x.nl) * invT;
         Kr = Kf * invKc;
         // the Kc term of dKr/dT is dropped when Kc sits on its clamp (JacobianFunctionI.H:246-249)
-        dKrdT = dKfdT * invKc - (invKc < inv_kc_clamp(x) ? Kr * dKcdTByKc : 0.0);
+        dKrdT = dKfdT * invKc - (less_than(invKc, inv_kc_clamp(x)) ? Kr * dKcdTByKc : 0.0);
         dKrdC = dKfdC * invKc;
     };
-    // The running sums of the rows: f[i] collects w_i (the net production),
-    // s.dCpdT[i] (free once CpM and dCpM/dT are formed) collects the
-    // temperature-column sum of dq/dT.
-    double* tcAcc = s.dCpdT;
-    for (int i = g.rank; i < ns; i += G) {
-        s.cur[i] = __ldg(&M.incOff[i]);
-        f[i] = 0.0;
-        tcAcc[i] = 0.0;
-    }
-    for (int idx = g.rank; idx < ns * ld; idx += G) J[idx] = MT(0);
-    const int sp0 = M.spBegin, sp1 = M.spBegin + M.nSp;
-    for (int c0 = 0; c0 < M.nr; c0 += s.rc) {
-        const int c1 = min(M.nr, c0 + s.rc);
-        auto finish = [&](const int r, const RxnInfo& x, const double Kf, const double dKfdT, const double dKfdC,
-                          const double Kr, const double dKrdT, const double dKrdC) {
-            double CF = s.C[x.sl[0]];
-            #pragma unroll 1
-            for (int q = 1; q < x.nl; q++) CF *= s.C[x.sl[q]];
-            double CR = s.C[x.sr[0]];
-            #pragma unroll 1
-            for (int q = 1; q < x.nr; q++) CR *= s.C[x.sr[q]];
-            s.Kf[r - c0] = Kf;
-            s.Kr[r - c0] = Kr;
-            s.q[r - c0] = Kf * CF - Kr * CR;
-            s.dqdT[r - c0] = dKfdT * CF - dKrdT * CR;
-            // third-body weight w = dKf/dM CF - dKr/dM CR
-            if (x.tb >= 0) s.tbF[x.tb] = dKfdC * CF - dKrdC * CR;
-        };
-        for (int r = c0 + g.rank; r < c1; r += G) {
-            if (r >= sp0 && r < sp1) continue;
-            const RxnInfo x = load_rx(M.rx + r);
-            double Kf, dKfdT;
-            if (x.kind == FCS_RXN_PLOG) {
-                Kf = plog_rate(M, x.plog, p, logP, logT, invT, &dKfdT);
-            } else if (x.tind) {
-                Kf = x.A; dKfdT = 0;
-            } else {
-                Kf = x.A * fast_exp(fma(x.beta, logT, -(x.Ta * invT)));
-                dKfdT = Kf * (fma(x.Ta, invT, x.beta) * invT);
-            }
+    auto finish = [&](const RxnEv& x, int l, const double Kf, const double dKfdT, const double dKfdC,
+                      const double Kr, const double dKrdT, const double dKrdC) {
+        double CF, CR;
+        if (three_at_most(x)) {
+            CF = product3(load3(s.C, x.sl), x.nl);
+            CR = product3(load3(s.C, x.sr), x.nr);
+        } else {
+            CF = product_over(s.C, x.sl, x.nl);
+            CR = product_over(s.C, x.sr, x.nr);
+        }
+        s.q[l] = Kf * CF - Kr * CR;
+        s.q[size + l] = dKfdT * CF - dKrdT * CR;
+        // third-body weight w = dKf/dM CF - dKr/dM CR
+        if (x.tb >= 0) s.tbF[x.tb] = dKfdC * CF - dKrdC * CR;
+        rate_gradients(x, s.C, Kf, Kr, s.q + x.ent);
+    };
+    #pragma unroll 1
+    for (int c = 0, c0 = 0; c0 < M.nr; c++, c0 += size) {
+        const int c1 = min(M.nr, c0 + size);
+        const int special = __ldg(&L.chunk[c].special);
+        #pragma unroll 1
+        for (int k = c0 + g.rank; k < special; k += G) {
+            const RxnEv x = load_ev(L.ev + k);
+            double dKfdT;
+            double Kf = forward_k(M, x, p, logP, logT, invT, &dKfdT);
             double dKfdC = 0;
             if (x.tb >= 0) {
                 const double Mt = s.Mtb[x.tb];
@@ -1023,102 +1175,86 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
             }
             double Kr = 0, dKrdT = 0, dKrdC = 0;
             if (x.rev) through_kc(x, Kf, dKfdT, dKfdC, Kr, dKrdT, dKrdC);
-            finish(r, x, Kf, dKfdT, dKfdC, Kr, dKrdT, dKrdC);
+            finish(x, x.r - c0, Kf, dKfdT, dKfdC, Kr, dKrdT, dKrdC);
         }
-        for (int r = max(c0, sp0) + g.rank; r < min(c1, sp1); r += G) {
-            const RxnInfo x = load_rx(M.rx + r);
-            SpecialK k = special_rates(M, x, s.Mtb, Tc, logT, invT, true);
+        #pragma unroll 1
+        for (int k = special + g.rank; k < c1; k += G) {
+            const RxnEv x = load_ev(L.ev + k);
+            const RxnInfo xi = load_rx(M.rx + x.r);
+            SpecialK v = special_rates(M, xi, s.Mtb, Tc, logT, invT, true);
             // non-equilibrium: the reverse Arrhenius (JacobianFunctionI.H:129-130, Jacobian.C:412-422)
-            if (x.rev == 1) through_kc(x, k.Kf, k.dKfdT, k.dKfdC, k.Kr, k.dKrdT, k.dKrdC);
-            finish(r, x, k.Kf, k.dKfdT, k.dKfdC, k.Kr, k.dKrdT, k.dKrdC);
+            if (x.rev == 1) through_kc(x, v.Kf, v.dKfdT, v.dKfdC, v.Kr, v.dKrdT, v.dKrdC);
+            finish(x, x.r - c0, v.Kf, v.dKfdT, v.dKfdC, v.Kr, v.dKrdT, v.dKrdC);
         }
         g.sync();
-        // Per species j and reaction r of the chunk (reaction order): the row
-        // sums of j (w_j, dq/dT), and as the owner of column j, d q_r / d C_j
-        // scattered down column j to the rows of reaction r (JF11..JF33
-        // reverse and forward concentration terms).
-        for (int j = g.rank; j < ns; j += G) {
-            double w = f[j], tc = tcAcc[j];
-            int e = s.cur[j];
-            const int e1 = __ldg(&M.incOff[j + 1]);
-            for (; e < e1; e++) {
-                const int v = __ldg(&M.inc[e]);
-                const int r = v >> 1;
-                if (r >= c1) break;
-                const bool prod = v & 1;
-                const double qq = s.q[r - c0], dq = s.dqdT[r - c0];
-                if (prod) { w += qq; tc += dq; } else { w -= qq; tc -= dq; }
-                const RxnInfo x = load_rx(M.rx + r);
-                double d;
-                if (!prod) {
-                    // forward: Kf * product of the other reactant concentrations
-                    bool skipped = false;
-                    d = s.Kf[r - c0];
-                    #pragma unroll 1
-                    for (int q = 0; q < x.nl; q++) {
-                        if (!skipped && x.sl[q] == j) { skipped = true; continue; }
-                        d *= s.C[x.sl[q]];
-                    }
-                } else {
-                    if (!x.rev) continue;
-                    bool skipped = false;
-                    d = -s.Kr[r - c0];
-                    #pragma unroll 1
-                    for (int q = 0; q < x.nr; q++) {
-                        if (!skipped && x.sr[q] == j) { skipped = true; continue; }
-                        d *= s.C[x.sr[q]];
-                    }
-                }
-                const MT md = MT(d);
-                #pragma unroll 1
-                for (int q = 0; q < x.nl; q++) { MT& c = J[(size_t)x.sl[q] * ld + j]; c = c - md; }
-                #pragma unroll 1
-                for (int q = 0; q < x.nr; q++) { MT& c = J[(size_t)x.sr[q] * ld + j]; c = c + md; }
-            }
-            s.cur[j] = e;
-            f[j] = w;
-            tcAcc[j] = tc;
+        const int lane = g.rank & 31, g1 = __ldg(&L.chunk[c].groupEnd);
+        #pragma unroll 1
+        for (int k = __ldg(&L.chunk[c].group0) + (g.rank >> 5); k < g1; k += G / 32) {
+            const uint32_t e = __ldg(L.sums.elem + 32 * k + lane);
+            const int m = e & 0xffff, most = __shfl_sync(0xffffffffu, m, 0), tgt = e >> 16;
+            MT* o = J + (tgt >> 8) * ld + (tgt & 0xff);
+            const bool valid = tgt != 0xffff;
+            const double v = sum_terms(L.sums.con + __ldg(L.sums.off + k) + lane, m, most, s.q, valid ? double(*o) : 0.0);
+            if (valid) *o = MT(v);
         }
-        g.sync();  // the next chunk overwrites Kf, Kr, q, dq/dT; the passes below read J
+        g.sync();  // the next chunk overwrites the values; the passes below read J
     }
-    // (2) third-body columns, J_ij += nu_i w_t E_tj (JF* third-body block)
+    // third-body columns, J_ij += nu_i w_t E_tj (JF* third-body block): the
+    // entries come in reaction order, a reaction's products E w computed once
     for (int j = g.rank; j < ns; j += G) {
+        int last = -1;
+        double wd = 0;
         for (int e = 0; e < M.nTbInc; e++) {
             const int v = __ldg(&M.tbInc[e]);
-            const int i = v >> 16, t = (v >> 1) & 0x7fff;
-            const double wd = __ldg(&M.eff[(size_t)t * ns + j]) * s.tbF[t];
-            MT& c = J[(size_t)i * ld + j];
+            const int i = v >> 16, tb = (v >> 1) & 0x7fff;
+            if (tb != last) {
+                wd = __ldg(&M.eff[(size_t)tb * ns + j]) * s.tbF[tb];
+                last = tb;
+            }
+            MT& c = J[i * ld + j];
             c = (v & 1) ? c + MT(wd) : c - MT(wd);
         }
     }
+    // dB/dT is free now: the column factors of the conversion
+    double* mj = s.dBdT;
+    for (int j = g.rank; j < ns; j += G) mj[j] = MW * __ldg(&M.invW[j]);
     g.sync();
-    // (3) row owners: production rate, temperature column and the dC/dY
-    // conversion of the row (diagonal scaling + rank-1 correction)
-    double dtd = 0, dd = 0;
+    // rows: production rate and temperature column; K_i for the conversion
+    double* rowK = s.dCpdT;
     for (int i = g.rank; i < ns; i += G) {
-        MT* row = J + (size_t)i * ld;
-        const double w = f[i], tc = tcAcc[i];
+        MT* row = J + i * ld;
+        const double w = double(J[ns * ld + i]), tc = double(row[ns]);
         const double WiByrhoM = invRhoM * __ldg(&M.W[i]);
         const double dY = w * WiByrhoM;
         double S = 0;
+        #pragma unroll 8
         for (int k = 0; k < ns; k++) S = fma(double(row[k]), s.C[k], S);
         const double tcol = WiByrhoM * (tc - S * invT) + invT * dY;
-        if (fast) {
-            for (int j = 0; j < ns; j++) {
-                const double invWj = __ldg(&M.invW[j]);
-                row[j] = MT(WiByrhoM * (double(row[j]) * (rhoM * invWj)) + (MW * invWj) * dY);
-            }
-        } else {
-            // Wi/rho (Jc_ij rho/Wj - m_j S) + m_j dY = Jc_ij (Wi/Wj) + m_j (dY - Wi/rho S)
-            const double K = dY - WiByrhoM * S;
-            const double Wi = __ldg(&M.W[i]);
-            for (int j = 0; j < ns; j++) {
-                const double invWj = __ldg(&M.invW[j]);
-                row[j] = MT(fma(double(row[j]), Wi * invWj, (MW * invWj) * K));
-            }
-        }
+        // exact: Wi/rho (Jc_ij rho/Wj - m_j S) + m_j dY = Jc_ij (Wi/Wj) + m_j (dY - Wi/rho S)
+        rowK[i] = fast ? WiByrhoM : dY - WiByrhoM * S;
         row[ns] = MT(tcol);
         f[i] = dY;
+    }
+    g.sync();
+    // the dC/dY conversion, element by element: rows do not matter here, and
+    // ns^2 elements fill the threads better than ns rows
+    {
+        int i = g.rank / ns, j = g.rank - i * ns;
+        const int di = G / ns, dj = G - di * ns;
+        for (int idx = g.rank; idx < ns * ns; idx += G) {
+            MT* e = J + i * ld + j;
+            double v;
+            if (fast) v = fma(mj[j], f[i], rowK[i] * (double(*e) * (rhoM * __ldg(&M.invW[j]))));
+            else v = fma(double(*e), __ldg(&M.wiw[idx]), mj[j] * rowK[i]);
+            *e = MT(iterate ? -v : v);
+            i += di;
+            j += dj;
+            if (j >= ns) { j -= ns; i++; }
+        }
+    }
+    double dtd = 0, dd = 0;
+    for (int i = r0; i < ns; i += s.rw) {
+        const double dY = f[i], tcol = double(J[i * ld + ns]);
         dtd = fma(s.Ha[i], dY, dtd);
         dd += dY * s.Cp[i] + tcol * s.Ha[i];
     }
@@ -1128,13 +1264,25 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     // temperature row (ddTdtdYT): column owners
     for (int j = g.rank; j < ns; j += G) {
         double v = 0;
-        for (int i = 0; i < ns; i++) v -= double(J[(size_t)i * ld + j]) * s.Ha[i];
+        #pragma unroll 8
+        for (int i = 0; i < ns; i++) {
+            const double a = double(J[i * ld + j]);
+            v -= (iterate ? -a : a) * s.Ha[i];
+        }
         v -= s.Cp[j] * dTdt;
-        J[(size_t)ns * ld + j] = MT(v / CpM);
+        const double r = v / CpM;
+        J[ns * ld + j] = MT(iterate ? -r : r);
     }
-    if (g.rank == 0) {
-        J[(size_t)ns * ld + ns] = MT((-dd - dTdt * dCpMdT) / CpM);
-        f[ns] = dTdt;
+    if (g.rank == 0) f[ns] = dTdt;
+    if (iterate) {
+        g.sync();
+        for (int i = g.rank; i < n; i += G) {
+            const double a = i == ns ? -((-dd - dTdt * dCpMdT) / CpM) : double(J[i * ld + i]);
+            J[i * ld + i] = MT(a + shift);
+            if (i < ns) J[i * ld + ns] = -J[i * ld + ns];
+        }
+    } else if (g.rank == 0) {
+        J[ns * ld + ns] = MT((-dd - dTdt * dCpMdT) / CpM);
     }
     g.sync();
 }

@@ -43,6 +43,44 @@ struct RxnInfo {            // 64 bytes
 };
 static_assert(sizeof(RxnInfo) == 64, "RxnInfo must stay 64 bytes");
 
+// A reaction as the cell groups evaluate it (fcs_lists.h).
+struct RxnEv {              // 64 bytes
+    double A, beta, Ta;
+    uint8_t sl[kMaxL];
+    uint8_t sr[kMaxR];
+    int8_t nl, nr, rev, kind;
+    int32_t tb, plog;       // third-body row, PLOG index or -1
+    int32_t r;              // packed reaction
+    int32_t ent;            // first value of its d q / d C in a Jacobian chunk
+    uint32_t first;         // per slot the first slot of its side with the same species (2 bits each for
+                            // reactants, 3 for products)
+    int32_t tind;           // temperature independent
+};
+static_assert(sizeof(RxnEv) == 64, "RxnEv must stay 64 bytes");
+
+struct JacChunk { int special, group0, groupEnd, pad; };  // first special reaction, groups of sums
+
+// Reactions per Jacobian chunk: a chunk's values stay in the slot until they
+// are summed, so small chunks let more cells reside and large ones keep more
+// threads busy (make_shape chooses).
+constexpr int kJacVariants = 3;
+constexpr int kJacChunk[kJacVariants] = {16, 64, 256};
+constexpr uint32_t kNoSum = 0xffff0000u;
+
+struct SumLists {
+    int groups;
+    const uint32_t* elem;
+    const int* off;
+    const uint32_t* con;
+};
+
+struct JacLists {
+    int size, values;       // reactions per chunk, doubles a chunk needs
+    const RxnEv* ev;
+    const JacChunk* chunk;
+    SumLists sums;
+};
+
 struct DevMech {
     int ns, n, nr;
     int nTB, nPlog;
@@ -63,6 +101,11 @@ struct DevMech {
     int nTbInc;             // third-body incidences (species row, third-body row, side)
     const int* tbInc;       // (row << 16) | (tb << 1) | (1 if product else 0), reaction order
     const double* hf;       // [ns] formation enthalpy at 298.15 K, J/kg (for Qdot)
+    const RxnEv* ev;        // [nr] plain, third-body, special block (fcs_lists.h)
+    int evThird, evSpecial;
+    SumLists prod;          // net production per species
+    JacLists jac[kJacVariants];
+    const double* wiw;      // [ns][ns] W_i / W_j as W_i invW_j
     const double* fo;       // [n fall-off + n non-equilibrium][8]: kInf A, beta, Ta; Troe alpha, T*, T**,
                             // T*** / SRI a, b, c, d, e -- or the reverse A, beta, Ta of a non-equilibrium reaction
 };

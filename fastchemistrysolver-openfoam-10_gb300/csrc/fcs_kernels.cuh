@@ -134,15 +134,29 @@ __device__ __noinline__ bool linear_solve_mixed(const Grp<G>& g, const DevMech& 
 template<int G, class MT>
 __device__ __forceinline__ void jacobian_into(const Grp<G>& g, const DevMech& M, const Slot<MT>& s,
                                               const Slot<double>& sd, double p, double* y, double* f, int fast) {
-    jac_eval<G, double>(g, M, sd, p, y, f, sd.J, fast);
+    jac_eval<G, double>(g, M, sd, p, y, f, sd.J, fast, false, 0.0);
 }
 
 template<int G, class MT>
 __device__ __forceinline__ void factor_iteration(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double c) {
     if constexpr (sizeof(MT) == 8) form_iteration_matrix<G>(g, s, M.n, c);
     else form_iteration_matrix_scaled<G>(g, s, M.n, c);
-    // the reaction-chunk arrays are free between a Jacobian and the next RHS
-    lu_factor<G, MT>(g, s.LU, M.n, s.ld, s.piv, s.invD, reinterpret_cast<int*>(s.Kf));
+    lu_factor<G, MT>(g, s.LU, M.n, s.ld, s.piv, s.invD, reinterpret_cast<int*>(s.red + 38));
+}
+
+// The Jacobian at y and the factors of c I - J.  The FP64 Rosenbrock methods
+// keep no Jacobian: it is assembled as c I - J and factored in place.
+template<int G, class MT>
+__device__ __forceinline__ void jacobian_and_lu(const Grp<G>& g, const DevMech& M, const Slot<MT>& s,
+                                                const Slot<double>& sd, double p, double* y, double* f, int fast,
+                                                double c) {
+    if constexpr (sizeof(MT) == 8) {
+        jac_eval<G, double>(g, M, sd, p, y, f, sd.J, fast, true, c);
+        lu_factor<G, MT>(g, s.LU, M.n, s.ld, s.piv, s.invD, reinterpret_cast<int*>(s.red + 38));
+    } else {
+        jacobian_into<G, MT>(g, M, s, sd, p, y, f, fast);
+        factor_iteration<G, MT>(g, M, s, c);
+    }
 }
 
 template<int G, class MT>
@@ -181,9 +195,8 @@ __device__ __noinline__ double rodas34_attempt(const Grp<G>& g, const DevMech& M
                  c64 = 0.1631930543123136e2, c65 = -0.6058818238834054e1;
     const double invgamma = 1.0 / 0.25;
 
-    jacobian_into<G, MT>(g, M, s, sd, p, y0, dfdx, o.jacobian);
     const double cdiag = 1.0 * invdx * invgamma;
-    factor_iteration<G, MT>(g, M, s, cdiag);
+    jacobian_and_lu<G, MT>(g, M, s, sd, p, y0, dfdx, o.jacobian, cdiag);
     cc.jac++; cc.lu++; cc.rhs += 5; cc.solves += 6;
 
     const double dxd1 = dx * d1 + 1;
@@ -273,9 +286,8 @@ __device__ __noinline__ double ros34_attempt(const Grp<G>& g, const DevMech& M, 
     const double d1 = 1.0 / 2.0, d2 = -3.0 / 2.0, d3 = 605.0 / 250.0, d4 = 29.0 / 250.0;
     const double invgamma = 1.0 / (1.0 / 2.0);
 
-    jacobian_into<G, MT>(g, M, s, sd, p, y0, dfdx, o.jacobian);
     const double cdiag = invdx * invgamma;
-    factor_iteration<G, MT>(g, M, s, cdiag);
+    jacobian_and_lu<G, MT>(g, M, s, sd, p, y0, dfdx, o.jacobian, cdiag);
     cc.jac++; cc.lu++; cc.rhs += 2; cc.solves += 4;
 
     const double dxd1 = dx * d1 + 1;
@@ -333,9 +345,8 @@ __device__ __noinline__ double rodas23_attempt(const Grp<G>& g, const DevMech& M
     const double c41 = 1, c42 = -1, c43 = -8.0 / 3.0;
     const double invgamma = 1.0 / (1.0 / 2.0);
 
-    jacobian_into<G, MT>(g, M, s, sd, p, y0, dfdx, o.jacobian);
     const double cdiag = invdx * invgamma;
-    factor_iteration<G, MT>(g, M, s, cdiag);
+    jacobian_and_lu<G, MT>(g, M, s, sd, p, y0, dfdx, o.jacobian, cdiag);
     cc.jac++; cc.lu++; cc.rhs += 2; cc.solves += 4;
 
     const double dxd1 = dx * d1, dxd2 = dx * d2;
@@ -392,9 +403,8 @@ __device__ __noinline__ double ros23_attempt(const Grp<G>& g, const DevMech& M, 
     const double d1 = 0.43586652150845899941601945119356, d2 = 0.24291996454816804366592249683314;
     const double d3 = 2.1851380027664058511513169485832;
 
-    jacobian_into<G, MT>(g, M, s, sd, p, y0, dfdx, o.jacobian);
     const double cdiag = invdx * invgamma;
-    factor_iteration<G, MT>(g, M, s, cdiag);
+    jacobian_and_lu<G, MT>(g, M, s, sd, p, y0, dfdx, o.jacobian, cdiag);
     cc.jac++; cc.lu++; cc.rhs += 1; cc.solves += 3;
 
     const double dxd1 = dx * d1, dxd2 = dx * d2, dxd3 = dx * d3;
@@ -836,9 +846,12 @@ integrate_kernel(const DevMech M, const KOpts o, const SlotLayout L, CellIO io, 
         double* y = s.v(0);
         for (int i = g.rank; i < ns; i += G) {
             const double Yi = io.Y[(size_t)i * nc + c];
-            y[i] = Yi > 0 ? Yi : 0.0;
+            y[i] = positive(Yi) ? Yi : 0.0;
         }
-        if (g.rank == 0) y[ns] = T0;
+        if (g.rank == 0) {
+            y[ns] = T0;
+            s.red[37] = M.nPlog ? log(p) : 0.0;
+        }
         g.sync();
         const double subDt0 = io.subDt[c];
         double subDt = subDt0;
@@ -923,13 +936,16 @@ eval_kernel(const DevMech M, const KOpts o, const SlotLayout L, long long nc, co
     double* y = s.v(0);
     double* f = s.v(1);
     for (int i = g.rank; i < ns; i += G) y[i] = Y[(size_t)i * nc + c];
-    if (g.rank == 0) y[ns] = T[c];
+    if (g.rank == 0) {
+        y[ns] = T[c];
+        s.red[37] = M.nPlog ? log(p[c]) : 0.0;
+    }
     g.sync();
     if (mode == 0) {
         rhs_eval<G, MT>(g, M, s, p[c], y, f, 1);
     } else if (mode == 1) {
         const Slot<double> sd = make_slot<double>(base, L, M);
-        jac_eval<G, double>(g, M, sd, p[c], y, f, sd.J, o.jacobian);
+        jac_eval<G, double>(g, M, sd, p[c], y, f, sd.J, o.jacobian, false, 0.0);
         for (int idx = g.rank; idx < n * n; idx += G) {
             const int i = idx / n, j = idx - i * n;
             Jout[(size_t)c * n * n + idx] = sd.J[(size_t)i * s.ld + j];

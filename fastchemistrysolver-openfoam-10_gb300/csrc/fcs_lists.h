@@ -1,0 +1,222 @@
+// fcs_lists.h -- reaction lists of the cell-group kernels, built once per
+// mechanism on the host (fcs_capi.cu) and read by fcs_device.cuh.
+//
+// A cell group evaluates reactions one per thread and then sums their terms
+// per species (rates) and per Jacobian element.  Both are lists here:
+//   * RxnEv records sorted so that the reactions of one warp take the same
+//     branches (a divergent branch costs a whole warp's FP64 instruction on
+//     either side);
+//   * per sum, its terms in the order the packed reactions are added (the
+//     order is part of the result), the sums sorted by length and laid out 32
+//     side by side, so that a warp reads its terms as one line and its lanes
+//     end together.
+#pragma once
+#include <algorithm>
+#include <cstdint>
+#include <cstring>
+#include <numeric>
+#include <tuple>
+#include <utility>
+#include <vector>
+
+#include "fcs_internal.h"
+
+namespace fcs {
+
+// Sums, 32 to a group: elem[32 g + lane] = target << 16 | terms, the group's
+// terms from con[off[g]] on, term k of a lane at off[g] + 32 k + lane, each
+// value index << 1 | (1: added, 0: subtracted).
+struct HostSums {
+    std::vector<uint32_t> elem;
+    std::vector<int> off;
+    std::vector<uint32_t> con;
+    int groups() const { return (int)off.size(); }
+
+    // targets[t], lists[t]: appended, longest first
+    void append(const std::vector<uint32_t>& targets, const std::vector<std::vector<uint32_t>>& lists) {
+        std::vector<int> order(targets.size());
+        std::iota(order.begin(), order.end(), 0);
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return lists[a].size() > lists[b].size(); });
+        for (size_t g = 0; g < order.size(); g += 32) {
+            const size_t len = lists[order[g]].size();
+            off.push_back((int)con.size());
+            const size_t base = con.size();
+            con.resize(base + 32 * len, 0);
+            for (size_t l = 0; l < 32; l++) {
+                if (g + l >= order.size()) { elem.push_back(kNoSum); continue; }
+                const auto& v = lists[order[g + l]];
+                elem.push_back(targets[order[g + l]] << 16 | (uint32_t)v.size());
+                for (size_t k = 0; k < v.size(); k++) con[base + 32 * k + l] = v[k];
+            }
+        }
+    }
+};
+
+// One chunking of the Jacobian's reactions: chunk c holds the packed
+// reactions [c size, (c + 1) size).  Values of a chunk: its net rates q
+// (size), dq/dT (size), then d q / d C of every reactant occurrence and, for
+// reactions with a reverse rate, product occurrence.  Targets: row << 8 |
+// column of the N x N matrix; the species' net production is summed in the
+// temperature row, dq/dT in the temperature column.
+struct HostChunks {
+    int size = 0, values = 0;  // values: most doubles any chunk needs
+    std::vector<RxnEv> ev;     // sorted within each chunk, special reactions last
+    std::vector<JacChunk> chunk;
+    HostSums sums;
+};
+
+struct HostLists {
+    std::vector<RxnEv> ev;     // all reactions: plain ones, third-body ones, the special block
+    int evThird = 0, evSpecial = 0;  // first third-body / special position
+    HostSums prod;             // net production per species over q[r]
+    HostChunks jac[kJacVariants];
+};
+
+// The lists as one block of device memory, each part on a 16-byte boundary.
+struct ListBlock {
+    struct Sums { size_t elem, off, con; };
+    struct Jac { size_t ev, chunk; Sums sums; };
+    std::vector<char> bytes;
+    size_t ev = 0, wiw = 0;
+    Sums prod{};
+    Jac jac[kJacVariants]{};
+    template<class T>
+    size_t put(const std::vector<T>& v) {
+        const size_t o = (bytes.size() + 15) & ~size_t(15);
+        bytes.resize(o + std::max<size_t>(1, v.size()) * sizeof(T));
+        if (!v.empty()) std::memcpy(bytes.data() + o, v.data(), v.size() * sizeof(T));
+        return o;
+    }
+    Sums put(const HostSums& s) {
+        Sums o;
+        o.elem = put(s.elem);
+        o.off = put(s.off);
+        o.con = put(s.con);
+        return o;
+    }
+    static SumLists sums(const char* base, const Sums& o, const HostSums& s) {
+        return SumLists{s.groups(), reinterpret_cast<const uint32_t*>(base + o.elem),
+                        reinterpret_cast<const int*>(base + o.off), reinterpret_cast<const uint32_t*>(base + o.con)};
+    }
+};
+
+inline RxnEv make_ev(const RxnInfo& x, int r) {
+    RxnEv e{};
+    e.A = x.A; e.beta = x.beta; e.Ta = x.Ta;
+    for (int q = 0; q < kMaxL; q++) e.sl[q] = x.sl[q];
+    for (int q = 0; q < kMaxR; q++) e.sr[q] = x.sr[q];
+    e.nl = x.nl; e.nr = x.nr; e.rev = x.rev; e.kind = x.kind;
+    e.tb = x.tb; e.plog = x.plog; e.r = r; e.tind = x.tind;
+    for (int q = 0; q < x.nl; q++) {
+        int f = 0;
+        while (x.sl[f] != x.sl[q]) f++;
+        e.first |= uint32_t(f) << (2 * q);
+    }
+    for (int q = 0; q < x.nr; q++) {
+        int f = 0;
+        while (x.sr[f] != x.sr[q]) f++;
+        e.first |= uint32_t(f) << (8 + 3 * q);
+    }
+    return e;
+}
+
+// Reactions that take the same path next to each other, the dearest kind first.
+inline void sort_ev(std::vector<RxnEv>::iterator a, std::vector<RxnEv>::iterator b) {
+    auto key = [](const RxnEv& e) {
+        return std::make_tuple(e.plog < 0, e.tind, e.tb >= 0, e.rev, e.nl, e.nr, e.r);
+    };
+    std::sort(a, b, [&](const RxnEv& x, const RxnEv& y) { return key(x) < key(y); });
+}
+
+// rx: the packed reactions; inc[i]: (reaction << 1 | product) of species i in
+// reaction order; [spBegin, spBegin + nSp): the special block.
+inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, const std::vector<std::vector<int>>& inc,
+                             int spBegin, int nSp) {
+    HostLists H;
+    auto special = [&](int r) { return r >= spBegin && r < spBegin + nSp; };
+    std::vector<RxnEv> part[3];
+    for (int r = 0; r < nr; r++) part[special(r) ? 2 : rx[r].tb >= 0 ? 1 : 0].push_back(make_ev(rx[r], r));
+    for (auto& p : part) {
+        sort_ev(p.begin(), p.end());
+        H.ev.insert(H.ev.end(), p.begin(), p.end());
+    }
+    H.evThird = (int)part[0].size();
+    H.evSpecial = H.evThird + (int)part[1].size();
+    {
+        std::vector<uint32_t> tgt;
+        std::vector<std::vector<uint32_t>> terms;
+        for (int i = 0; i < ns; i++) {
+            tgt.push_back(i);
+            terms.emplace_back(inc[i].begin(), inc[i].end());
+        }
+        H.prod.append(tgt, terms);
+    }
+    for (int v = 0; v < kJacVariants; v++) {
+        HostChunks& J = H.jac[v];
+        J.size = kJacChunk[v];
+        std::vector<size_t> at(ns, 0);  // position in inc[i]
+        for (int c0 = 0; c0 < nr; c0 += J.size) {
+            const int c1 = std::min(nr, c0 + J.size);
+            std::vector<RxnEv> main, sp;
+            for (int r = c0; r < c1; r++) (special(r) ? sp : main).push_back(make_ev(rx[r], r));
+            sort_ev(main.begin(), main.end());
+            sort_ev(sp.begin(), sp.end());
+            main.insert(main.end(), sp.begin(), sp.end());
+            // value index of every occurrence of the chunk's reactions
+            std::vector<int> ent(c1 - c0);
+            int n = 2 * J.size;
+            for (int r = c0; r < c1; r++) {
+                ent[r - c0] = n;
+                n += rx[r].nl + (rx[r].rev ? rx[r].nr : 0);
+            }
+            J.values = std::max(J.values, n);
+            for (RxnEv& e : main) e.ent = ent[e.r - c0];
+            JacChunk ch{(int)J.ev.size() + (int)(main.size() - sp.size()), J.sums.groups(), 0, 0};
+            J.ev.insert(J.ev.end(), main.begin(), main.end());
+            std::vector<uint32_t> tgt;
+            std::vector<std::vector<uint32_t>> terms;
+            for (int j = 0; j < ns; j++) {
+                std::vector<uint32_t> w, tc;
+                std::vector<std::pair<int, uint32_t>> col;  // (row, term) of column j
+                int seen[2] = {-1, -1}, occ[2] = {0, 0};  // occurrence of j on the side so far
+                for (; at[j] < inc[j].size() && (inc[j][at[j]] >> 1) < c1; at[j]++) {
+                    const int r = inc[j][at[j]] >> 1, side = inc[j][at[j]] & 1, l = r - c0;
+                    const RxnInfo& x = rx[r];
+                    w.push_back(uint32_t(l) << 1 | side);
+                    tc.push_back(uint32_t(J.size + l) << 1 | side);
+                    if (seen[side] != r) { seen[side] = r; occ[side] = 0; }
+                    // the occ-th slot of this side that holds j
+                    int slot = 0, k = occ[side]++;
+                    const uint8_t* s = side ? x.sr : x.sl;
+                    for (;; slot++)
+                        if (s[slot] == j && k-- == 0) break;
+                    if (side && !x.rev) continue;
+                    const uint32_t val = uint32_t(ent[l] + (side ? x.nl : 0) + slot);
+                    for (int q = 0; q < x.nl; q++) col.emplace_back(x.sl[q], val << 1);
+                    for (int q = 0; q < x.nr; q++) col.emplace_back(x.sr[q], val << 1 | 1);
+                }
+                if (!w.empty()) {
+                    tgt.push_back(uint32_t(ns) << 8 | uint32_t(j));
+                    terms.push_back(w);
+                    tgt.push_back(uint32_t(j) << 8 | uint32_t(ns));
+                    terms.push_back(tc);
+                }
+                std::stable_sort(col.begin(), col.end(),
+                                 [](const auto& a, const auto& b) { return a.first < b.first; });
+                for (size_t a = 0; a < col.size(); a++) {
+                    if (a == 0 || col[a].first != col[a - 1].first) {
+                        tgt.push_back(uint32_t(col[a].first) << 8 | uint32_t(j));
+                        terms.emplace_back();
+                    }
+                    terms.back().push_back(col[a].second);
+                }
+            }
+            J.sums.append(tgt, terms);
+            ch.groupEnd = J.sums.groups();
+            J.chunk.push_back(ch);
+        }
+    }
+    return H;
+}
+
+}  // namespace fcs

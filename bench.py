@@ -485,7 +485,7 @@ def main():
         torch.cuda.synchronize()
         return max_over_ranks(statistics.mean(times), dev), out
 
-    # the first call autotunes the cell-to-thread mapping (outside the graph)
+    # the first call outside the graph
     step_plain(graph=False)
     for _ in range(args.warmup):
         step_plain(graph=not args.no_graph)

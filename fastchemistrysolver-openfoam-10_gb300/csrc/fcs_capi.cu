@@ -1,6 +1,6 @@
 // fcs_capi.cu -- the C ABI of libfcs_cuda.so (include/fcs.h): context and
 // device-memory management, mechanism packing, launch-shape selection
-// (autotuner) and the batched integrate / rhs / jacobian / rates entry points.
+// and the batched integrate / rhs / jacobian / rates entry points.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -346,6 +346,8 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
     ListBlock at;
     at.ev = at.put(lists.ev);
     at.wiw = at.put(wiw);
+    at.tbRow = at.put(lists.tbRow);
+    at.tbTerm = at.put(lists.tbTerm);
     at.prod = at.put(lists.prod);
     for (int v = 0; v < kJacVariants; v++)
         at.jac[v] = ListBlock::Jac{at.put(lists.jac[v].ev), at.put(lists.jac[v].chunk), at.put(lists.jac[v].sums)};
@@ -381,6 +383,15 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
     M.ev = reinterpret_cast<const RxnEv*>(ctx->dLists.p + at.ev);
     M.evThird = lists.evThird;
     M.evSpecial = lists.evSpecial;
+    M.evTroe = lists.evTroe;
+    M.evSri = lists.evSri;
+    M.nTbRow = (int)lists.tbRow.size() / 2 - 1;
+    M.tbRow = reinterpret_cast<const int*>(ctx->dLists.p + at.tbRow);
+    M.tbTerm = reinterpret_cast<const int*>(ctx->dLists.p + at.tbTerm);
+    M.plogSorted = 1;
+    for (size_t q = 0; q + 1 < plogOff.size(); q++)
+        for (int k = plogOff[q]; k + 1 < plogOff[q + 1]; k++)
+            if (!(plogRow[4 * (size_t)k] <= plogRow[4 * (size_t)k + 4])) M.plogSorted = 0;
     M.wiw = reinterpret_cast<const double*>(ctx->dLists.p + at.wiw);
     M.prod = at.sums(ctx->dLists.p, at.prod, lists.prod);
     for (int v = 0; v < kJacVariants; v++) {
@@ -392,7 +403,6 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
         M.jac[v].sums = at.sums(ctx->dLists.p, at.jac[v].sums, j.sums);
     }
     ctx->loaded = true;
-    ctx->tuned.clear();
     if (ctx->gexec) {  // a captured step holds the old mechanism's scalars
         cudaGraphExecDestroy(ctx->gexec);
         ctx->gexec = nullptr;
@@ -442,14 +452,21 @@ static bool make_lane_shape(fcs_ctx* ctx, bool integrate, Shape& sh) {
     sh.global = true;
     sh.lc.group = 1;
     sh.lc.block = kBlock;
+    sh.lc.perSM = perSM;
     sh.lc.grid = ctx->numSMs * perSM;
     sh.L = SlotLayout{};
     sh.L.bytes = make_lane_layout(ctx->M.ns, ctx->M.nr, ctx->M.nTB, mixed).words * (int)sizeof(double);
     return true;
 }
 
+// Threads that carry the partial sums of a group's reductions: fixed by the
+// mechanism, so that the results do not depend on the group AUTO chooses.
+static int sum_threads(const fcs_ctx* ctx, int group) {
+    return ctx->opt.mapping ? group : std::min(group, ctx->M.n <= 128 ? 64 : 128);
+}
+
 // Build the launch shape for a group size; returns false when impossible.
-bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, Shape& sh) {
+bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, Shape& sh) {
     if (group == FCS_MAPPING_LANE) return make_lane_shape(ctx, integrate, sh);
     const fcs_options& o = ctx->opt;
     const bool mixed = o.precision == FCS_PRECISION_MIXED;
@@ -489,12 +506,20 @@ bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, Shape& sh) {
         sh.L.jv = v;
         res = r;
     }
-    sh.L.rw = group;
+    sh.L.rw = sum_threads(ctx, group);
     sh.global = res.global;
     sh.lc.block = group * res.gpb;
     if (sh.lc.block > maxThreads) return false;
-    const int perSM = res.perSM;
-    sh.lc.grid = ctx->numSMs * perSM;
+    // Blocks per SM: what fits, but for few cells no more than spread them
+    // evenly over the SMs (a grid of every block that fits lets some SMs take
+    // several cells while others have none), and then somewhat fewer than one
+    // per cell: co-resident cells slow the dearest one, which the others end
+    // before.  600 cells of 53 species (four per SM): four blocks 33.1 ms,
+    // three 32.8, two 30.1; 1,024 of 10 species gain nothing from fewer.
+    const double per = (double)cells / std::max(1, ctx->numSMs) / res.gpb;
+    const int want = per <= 2 ? (int)std::ceil(per) : std::max(2, (int)std::ceil(0.6 * per));
+    sh.lc.perSM = std::max(1, std::min(res.perSM, want));
+    sh.lc.grid = ctx->numSMs * sh.lc.perSM;
     return true;
 }
 
@@ -506,10 +531,26 @@ fcs_status fcs::ensure_gws(fcs_ctx* ctx, const Shape& sh) {
     return FCS_OK;
 }
 
-int fcs::default_group(fcs_ctx* ctx) {
+// AUTO's threads per cell, from the mechanism and the cells per SM (Rodas34,
+// FP64, GB300).  Few cells: enough threads to shorten one cell's chain of
+// dependent work; many: as few as fill their lanes, so that more cells reside
+// and fewer FP64 instructions are issued twice.
+//   up to 31 species      1 cell per SM: 10 species 64 threads 12.6 ms (32: 16.4, 128: 12.6); 16 species
+//                         with fall-off 128 threads 41.3 ms (64: 51.5, 256: 44.8)
+//                         7 per SM: 10 species 32 threads 18.2 ms (64: 20.8); 20: 37.4 (64: 46.7)
+//                         13 per SM: 16 species with fall-off 64 threads 182 ms (32: 185, 128: 227)
+//   up to 63 (53 species) 1 per SM: 128 threads 25.9 ms (64: 30.4, 256: 26.8); 6: 34.1 (64: 36.0);
+//                         12: 64 threads 50.6 ms (128: 56.0); 24: 88.6 (128: 111)
+//   up to 127 (111)       one cell resides: 256 threads 99.8 ms (128: 112, 512: 108)
+//   above (200)           one cell per SM: 512 threads 132 ms (256: 140)
+int fcs::auto_group(fcs_ctx* ctx, long long cells) {
+    if (ctx->opt.mapping) return ctx->opt.mapping;
     const int n = ctx->M.n;
-    if (n <= 128) return 64;
-    return 128;
+    const double perSM = (double)cells / std::max(1, ctx->numSMs);
+    if (n <= 32) return ctx->M.nSp > 0 ? (perSM > 4 ? 64 : 128) : (perSM > 4 ? 32 : 64);
+    if (n <= 64) return perSM > 9 ? 64 : 128;
+    if (n <= 128) return 256;
+    return 512;
 }
 
 // AUTO chooses the lane mapping for a Rosenbrock-family FP64 step with cells
@@ -518,69 +559,8 @@ int fcs::default_group(fcs_ctx* ctx) {
 bool fcs::lane_auto(fcs_ctx* ctx, long long cells) {
     if (ctx->opt.mapping != FCS_MAPPING_AUTO) return false;
     Shape sh;
-    if (!make_shape(ctx, FCS_MAPPING_LANE, true, sh)) return false;
+    if (!make_shape(ctx, FCS_MAPPING_LANE, true, cells, sh)) return false;
     return cells * 4 >= 3LL * sh.lc.grid * sh.lc.block;
-}
-
-int fcs::cached_group(fcs_ctx* ctx) {
-    if (ctx->opt.mapping) return ctx->opt.mapping;
-    const auto it = ctx->tuned.find(
-        std::make_tuple(ctx->M.n, (int)ctx->opt.precision, (int)ctx->opt.solver, (int)ctx->opt.jacobian));
-    return it != ctx->tuned.end() ? it->second : default_group(ctx);
-}
-
-// Autotuner for FCS_MAPPING_AUTO: times every candidate cell-to-thread
-// mapping on the first `sample` queued cells, integrated from copies of their
-// state (the caller's arrays are not touched), and keeps the fastest for this
-// (mechanism size, precision, solver, Jacobian) key.
-static int tuned_group(fcs_ctx* ctx, const CellIO& io, int nActive) {
-    const auto key = std::make_tuple(ctx->M.n, (int)ctx->opt.precision, (int)ctx->opt.solver, (int)ctx->opt.jacobian);
-    auto it = ctx->tuned.find(key);
-    if (it != ctx->tuned.end()) return it->second;
-    const int fallback = default_group(ctx);
-    if (nActive < 2048) return fallback;  // too few cells to time reliably; not cached
-    const int ns = ctx->M.ns;
-    const long long nc = io.nCells;
-    cudaStream_t st = ctx->stream;
-    DBuf<double> T, Y, S;
-    DBuf<int> stat, head;
-    if (T.ensure(nc) || Y.ensure((size_t)ns * nc) || S.ensure(nc) || stat.ensure(nc) || head.ensure(1)) {
-        T.release(); Y.release(); S.release(); stat.release(); head.release();
-        return fallback;
-    }
-    const KOpts ko = kopts(ctx->opt);
-    int best = fallback;
-    float bestMs = 1e30f;
-    for (int g : {32, 64, 128, 256}) {
-        Shape sh;
-        if (!make_shape(ctx, g, true, sh)) continue;
-        if (ensure_gws(ctx, sh) != FCS_OK) continue;
-        const int groups = sh.lc.grid * (sh.lc.block / g);
-        const int sample = std::min(nActive, 2 * groups);
-        CellIO sio = io;
-        sio.T = T.p; sio.Y = Y.p; sio.subDt = S.p; sio.RR = nullptr; sio.status = stat.p;
-        cudaMemcpyAsync(T.p, io.T, nc * 8, cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(Y.p, io.Y, (size_t)ns * nc * 8, cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(S.p, io.subDt, nc * 8, cudaMemcpyDeviceToDevice, st);
-        cudaMemsetAsync(head.p, 0, sizeof(int), st);
-        WorkQueue q{head.p, ctx->bOrder.p, sample};
-        cudaEventRecord(ctx->ev0, st);
-        const cudaError_t e = launch_integrate(sh.lc, sh.mixed, ctx->M, ko, sh.L, sio, q,
-                                               sh.global ? ctx->gws.p : nullptr, st);
-        cudaEventRecord(ctx->ev1, st);
-        if (e != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) continue;
-        float ms = 0;
-        cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-        const float perCell = ms / sample;
-        if (perCell < bestMs) { bestMs = perCell; best = g; }
-    }
-    T.release(); Y.release(); S.release(); stat.release(); head.release();
-    // the statistics of the sample runs are not the caller's
-    cudaMemsetAsync(ctx->bStats.p, 0, ST_COUNT * sizeof(long long), st);
-    cudaMemsetAsync(ctx->bMin.p, 0x7f, sizeof(unsigned long long), st);
-    cudaStreamSynchronize(st);
-    ctx->tuned[key] = best;
-    return best;
 }
 
 // ------------------------------------------------------------------------
@@ -672,13 +652,9 @@ static fcs_status integrate_impl(fcs_ctx* ctx, int64_t nc, double dt, const doub
         if (!ctx->hStats) CK(cudaMallocHost(&ctx->hStats, (ST_COUNT + 1) * sizeof(long long)));
         hs = ctx->hStats;
         hmin = reinterpret_cast<unsigned long long*>(ctx->hStats + ST_COUNT);
-        group = ctx->opt.mapping ? ctx->opt.mapping : lane_auto(ctx, nc) ? (int)FCS_MAPPING_LANE : [&] {
-            const auto it = ctx->tuned.find(std::make_tuple(ctx->M.n, (int)ctx->opt.precision, (int)ctx->opt.solver,
-                                                            (int)ctx->opt.jacobian));
-            return it != ctx->tuned.end() ? it->second : default_group(ctx);
-        }();
+        group = lane_auto(ctx, nc) ? (int)FCS_MAPPING_LANE : auto_group(ctx, nc);
         Shape sh;
-        if (!make_shape(ctx, group, true, sh))
+        if (!make_shape(ctx, group, true, nc, sh))
             return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
         fcs_status s = ensure_gws(ctx, sh);
         if (s != FCS_OK) return s;
@@ -723,10 +699,9 @@ static fcs_status integrate_impl(fcs_ctx* ctx, int64_t nc, double dt, const doub
         int nActive = 0;
         CK(cudaMemcpyAsync(&nActive, ctx->bHead.p + QC_LEN, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        group = ctx->opt.mapping ? ctx->opt.mapping
-                                 : lane_auto(ctx, nActive) ? (int)FCS_MAPPING_LANE : tuned_group(ctx, io, nActive);
+        group = lane_auto(ctx, nActive) ? (int)FCS_MAPPING_LANE : auto_group(ctx, nActive);
         Shape sh;
-        if (!make_shape(ctx, group, true, sh))
+        if (!make_shape(ctx, group, true, nActive, sh))
             return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
         fcs_status s = ensure_gws(ctx, sh);
         if (s != FCS_OK) return s;
@@ -827,9 +802,10 @@ static fcs_status eval_impl(fcs_ctx* ctx, int64_t nc, const double* p, const dou
         if (Qdot) { CK(ctx->bQ.ensure(nc)); dQ = ctx->bQ.p; }
     }
     // the per-cell evaluations run on cell groups (the lane mapping is the integrator's)
-    const int group = ctx->opt.mapping > FCS_MAPPING_LANE ? ctx->opt.mapping : default_group(ctx);
+    const int group = ctx->opt.mapping > FCS_MAPPING_LANE ? ctx->opt.mapping
+                                                          : ctx->M.n <= 64 ? 64 : ctx->M.n <= 128 ? 256 : 512;
     Shape sh;
-    if (!make_shape(ctx, group, false, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape");
+    if (!make_shape(ctx, group, false, nc, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape");
     const int gpb = sh.lc.block / sh.lc.group;
     sh.lc.grid = (int)((nc + gpb - 1) / gpb);
     char* gws = nullptr;

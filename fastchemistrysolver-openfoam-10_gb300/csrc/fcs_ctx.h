@@ -5,9 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <map>
 #include <string>
-#include <tuple>
 
 #include "../../include/fcs.h"
 #include "fcs_device.cuh"
@@ -89,7 +87,6 @@ struct fcs_ctx {
     fcs::DBuf<long long> bStats;
     fcs::DBuf<unsigned long long> bMin;
     fcs::DBuf<char> gws;
-    std::map<std::tuple<int, int, int, int>, int> tuned;  // (n, precision, solver, jac) -> group
     fcs::GateState* gate = nullptr;                       // attached surrogate, if any
     // per-cell attempts of the last integration, for the cost-ordered queue
     fcs::DBuf<int> bAtt;
@@ -120,11 +117,10 @@ fcs_status refuse_if_async_pending(fcs_ctx* ctx);
 // handed to a kernel would fault.
 fcs_status check_device_array(fcs_ctx* ctx, const void* ptr, const char* name, size_t align);
 KOpts kopts(const fcs_options& o);
-// Launch shape for a group size; false when impossible.
-bool make_shape(fcs_ctx* ctx, int group, bool integrate, Shape& sh);
-int default_group(fcs_ctx* ctx);
-// The option's mapping, else one the autotuner cached for this key, else the default.
-int cached_group(fcs_ctx* ctx);
+// Launch shape of a group size for this many cells; false when impossible.
+bool make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, Shape& sh);
+// The option's mapping, else AUTO's threads per cell for this many cells.
+int auto_group(fcs_ctx* ctx, long long cells);
 // AUTO mapping: the lane mapping for this many reacting cells?
 bool lane_auto(fcs_ctx* ctx, long long cells);
 // Global-memory workspace for shapes whose slot exceeds shared memory.

@@ -454,7 +454,12 @@ __device__ __forceinline__ double plog_rate(const DevMech& M, int ip, double p, 
         dk = (b + ta * invT) * invT;
     } else {
         int idx = 0;
-        for (int j = 0; j < len - 1; j++) {
+        if (M.plogSorted) {
+            // the first bracket that holds p: one below the number of rows
+            // under p, counted without waiting for one load before the next
+            #pragma unroll 4
+            for (int j = 1; j < len - 1; j++) idx += less_than(__ldg(&R[4 * (o + j)]), p);
+        } else for (int j = 0; j < len - 1; j++) {
             if (at_most(__ldg(&R[4 * (o + j)]), p) && at_most(p, __ldg(&R[4 * (o + j + 1)]))) { idx = j; break; }
         }
         const int a = o + idx, b = a + 1;
@@ -764,20 +769,46 @@ __device__ __forceinline__ double net_rate(const Slot<MT>& s, const RxnEv& x, do
     return Kf * CF - Kr * CR;
 }
 
+// The thread's rank when ranks are counted from warp w on
+template<int G>
+__device__ __forceinline__ int rank_from(const Grp<G>& g, int w) {
+    return (g.rank + G - 32 * (w % (G / 32))) % G;
+}
+
 // Net rates of all reactions into s.q (ReactionRate.C:521-575 and the RF*
-// functions), with the third-body concentrations: the plain reactions do not
-// wait for them.  The special block (first non-equilibrium to last fall-off
-// reaction) runs in a loop of its own, so that the others carry neither the
-// fall-off call nor a second Arrhenius.
+// functions), with the third-body concentrations.  The special block (first
+// non-equilibrium to last fall-off reaction) runs in a loop of its own, so
+// that the others carry neither the fall-off call nor a second Arrhenius: its
+// Troe and SRI rates (some 300 FP64 instructions each) begin on a warp each,
+// the other reactions on the warp after those.  Without a special block the
+// plain reactions do not wait for the third bodies.
 template<int G, class MT>
 __device__ __forceinline__ void net_rates(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double p, double logP,
                                           double Tc, const ThermoScalars& t) {
     third_bodies<G, MT>(g, M, s);
+    const bool special = M.evSpecial < M.nr;
+    if (special) {
+        g.sync();
+        #pragma unroll 1
+        for (int part = 0; part < 3; part++) {
+            const int k0 = part == 0 ? M.evTroe : part == 1 ? M.evSri : M.evSpecial;
+            const int k1 = part == 0 ? M.evSri : part == 1 ? M.nr : M.evTroe;
+            #pragma unroll 1
+            for (int k = k0 + rank_from<G>(g, part); k < k1; k += G) {
+                const RxnEv x = load_ev(M.ev + k);
+                const RxnInfo xi = load_rx(M.rx + x.r);
+                const SpecialK c = special_rates(M, xi, s.Mtb, Tc, t.logT, t.invT, false);
+                double Kr = c.Kr;  // non-equilibrium: its own reverse rate
+                if (x.rev == 1) Kr = c.Kf * inverse_kc(x, s.B, s.Binv, t.pf);
+                s.q[x.r] = net_rate(s, x, c.Kf, Kr);
+            }
+        }
+    }
     #pragma unroll 1
     for (int part = 0; part < 2; part++) {
         const int end = part ? M.evSpecial : M.evThird;
         #pragma unroll 1
-        for (int k = (part ? M.evThird : 0) + g.rank; k < end; k += G) {
+        for (int k = (part ? M.evThird : 0) + rank_from<G>(g, special ? 2 : 0); k < end; k += G) {
             const RxnEv x = load_ev(M.ev + k);
             double dk;
             double Kf = forward_k(M, x, p, logP, t.logT, t.invT, &dk);
@@ -786,16 +817,7 @@ __device__ __forceinline__ void net_rates(const Grp<G>& g, const DevMech& M, con
             if (x.rev) Kr = Kf * inverse_kc(x, s.B, s.Binv, t.pf);
             s.q[x.r] = net_rate(s, x, Kf, Kr);
         }
-        if (part == 0) g.sync();
-    }
-    #pragma unroll 1
-    for (int k = M.evSpecial + g.rank; k < M.nr; k += G) {
-        const RxnEv x = load_ev(M.ev + k);
-        const RxnInfo xi = load_rx(M.rx + x.r);
-        const SpecialK c = special_rates(M, xi, s.Mtb, Tc, t.logT, t.invT, false);
-        double Kr = c.Kr;  // non-equilibrium: its own reverse rate
-        if (x.rev == 1) Kr = c.Kf * inverse_kc(x, s.B, s.Binv, t.pf);
-        s.q[x.r] = net_rate(s, x, c.Kf, Kr);
+        if (part == 0 && !special) g.sync();
     }
 }
 
@@ -1162,7 +1184,7 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
         const int c1 = min(M.nr, c0 + size);
         const int special = __ldg(&L.chunk[c].special);
         #pragma unroll 1
-        for (int k = c0 + g.rank; k < special; k += G) {
+        for (int k = c0 + rank_from<G>(g, special < c1 ? 2 : 0); k < special; k += G) {
             const RxnEv x = load_ev(L.ev + k);
             double dKfdT;
             double Kf = forward_k(M, x, p, logP, logT, invT, &dKfdT);
@@ -1177,14 +1199,21 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
             if (x.rev) through_kc(x, Kf, dKfdT, dKfdC, Kr, dKrdT, dKrdC);
             finish(x, x.r - c0, Kf, dKfdT, dKfdC, Kr, dKrdT, dKrdC);
         }
+        const int troe = __ldg(&L.chunk[c].troe), sri = __ldg(&L.chunk[c].sri);
         #pragma unroll 1
-        for (int k = special + g.rank; k < c1; k += G) {
+        for (int part = 0; part < 3; part++) {
+            // Troe rates start at warp 0, SRI rates at warp 1, the others at warp 2
+            const int k0 = part == 0 ? troe : part == 1 ? sri : special;
+            const int k1 = part == 0 ? sri : part == 1 ? c1 : troe;
+            #pragma unroll 1
+            for (int k = k0 + rank_from<G>(g, part); k < k1; k += G) {
             const RxnEv x = load_ev(L.ev + k);
             const RxnInfo xi = load_rx(M.rx + x.r);
             SpecialK v = special_rates(M, xi, s.Mtb, Tc, logT, invT, true);
             // non-equilibrium: the reverse Arrhenius (JacobianFunctionI.H:129-130, Jacobian.C:412-422)
             if (x.rev == 1) through_kc(x, v.Kf, v.dKfdT, v.dKfdC, v.Kr, v.dKrdT, v.dKrdC);
             finish(x, x.r - c0, v.Kf, v.dKfdT, v.dKfdC, v.Kr, v.dKrdT, v.dKrdC);
+            }
         }
         g.sync();
         const int lane = g.rank & 31, g1 = __ldg(&L.chunk[c].groupEnd);
@@ -1199,20 +1228,44 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
         }
         g.sync();  // the next chunk overwrites the values; the passes below read J
     }
-    // third-body columns, J_ij += nu_i w_t E_tj (JF* third-body block): the
-    // entries come in reaction order, a reaction's products E w computed once
-    for (int j = g.rank; j < ns; j += G) {
-        int last = -1;
-        double wd = 0;
-        for (int e = 0; e < M.nTbInc; e++) {
-            const int v = __ldg(&M.tbInc[e]);
-            const int i = v >> 16, tb = (v >> 1) & 0x7fff;
-            if (tb != last) {
-                wd = __ldg(&M.eff[(size_t)tb * ns + j]) * s.tbF[tb];
-                last = tb;
+    // third-body columns, J_ij += nu_i w_t E_tj (JF* third-body block).  Up to
+    // 64 threads own columns: the entries come in reaction order and a
+    // reaction's products E w are formed once.  More threads than columns
+    // share out the elements of the rows that have terms (one more product a
+    // term, 53 species: 24,000 cycles by columns at any group size, 15,000
+    // with 128 threads, 9,000 with 256).
+    if constexpr (G <= 64) {
+        for (int j = g.rank; j < ns; j += G) {
+            int last = -1;
+            double wd = 0;
+            for (int e = 0; e < M.nTbInc; e++) {
+                const int v = __ldg(&M.tbInc[e]);
+                const int i = v >> 16, tb = (v >> 1) & 0x7fff;
+                if (tb != last) {
+                    wd = __ldg(&M.eff[(size_t)tb * ns + j]) * s.tbF[tb];
+                    last = tb;
+                }
+                MT& c = J[i * ld + j];
+                c = (v & 1) ? c + MT(wd) : c - MT(wd);
             }
-            MT& c = J[i * ld + j];
-            c = (v & 1) ? c + MT(wd) : c - MT(wd);
+        }
+    } else {
+        int r = g.rank / ns, j = g.rank - r * ns;
+        const int dr = G / ns, dj = G - dr * ns;
+        while (r < M.nTbRow) {
+            const int i = __ldg(M.tbRow + 2 * r), e0 = __ldg(M.tbRow + 2 * r + 1), e1 = __ldg(M.tbRow + 2 * r + 3);
+            MT& o = J[i * ld + j];
+            double v = double(o);
+            #pragma unroll 2
+            for (int e = e0; e < e1; e++) {
+                const int c = __ldg(M.tbTerm + e), tb = c >> 1;
+                const double wd = __dmul_rn(__ldg(&M.eff[(size_t)tb * ns + j]), s.tbF[tb]);
+                v += (c & 1) ? wd : -wd;
+            }
+            o = MT(v);
+            r += dr;
+            j += dj;
+            if (j >= ns) { j -= ns; r++; }
         }
     }
     // dB/dT is free now: the column factors of the conversion
@@ -1240,16 +1293,25 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     // ns^2 elements fill the threads better than ns rows
     {
         int i = g.rank / ns, j = g.rank - i * ns;
-        const int di = G / ns, dj = G - di * ns;
-        for (int idx = g.rank; idx < ns * ns; idx += G) {
-            MT* e = J + i * ld + j;
-            double v;
-            if (fast) v = fma(mj[j], f[i], rowK[i] * (double(*e) * (rhoM * __ldg(&M.invW[j]))));
-            else v = fma(double(*e), __ldg(&M.wiw[idx]), mj[j] * rowK[i]);
-            *e = MT(iterate ? -v : v);
-            i += di;
-            j += dj;
-            if (j >= ns) { j -= ns; i++; }
+        const int di = G / ns, dj = G - di * ns, m = ns * ns;
+        #pragma unroll 1
+        for (int idx = g.rank; idx < m; idx += 4 * G) {
+            double w[4];
+            #pragma unroll
+            for (int u = 0; u < 4; u++) w[u] = !fast && idx + u * G < m ? __ldg(&M.wiw[idx + u * G]) : 0.0;
+            #pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (idx + u * G < m) {
+                    MT* e = J + i * ld + j;
+                    double v;
+                    if (fast) v = fma(mj[j], f[i], rowK[i] * (double(*e) * (rhoM * __ldg(&M.invW[j]))));
+                    else v = fma(double(*e), w[u], mj[j] * rowK[i]);
+                    *e = MT(iterate ? -v : v);
+                }
+                i += di;
+                j += dj;
+                if (j >= ns) { j -= ns; i++; }
+            }
         }
     }
     double dtd = 0, dd = 0;

@@ -96,6 +96,7 @@ cudaError_t launch_integrate(const LaunchCfg& lc, bool mixed, const DevMech& M, 
         case 64: return launch_integrate_g<64>(lc, mixed, M, o, L, io, q, gws, st);
         case 128: return launch_integrate_g<128>(lc, mixed, M, o, L, io, q, gws, st);
         case 256: return launch_integrate_g<256>(lc, mixed, M, o, L, io, q, gws, st);
+        case 512: return launch_integrate_g<512>(lc, mixed, M, o, L, io, q, gws, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -109,6 +110,7 @@ cudaError_t launch_eval(const LaunchCfg& lc, bool mixed, const DevMech& M, const
         case 64: return launch_eval_g<64>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
         case 128: return launch_eval_g<128>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
         case 256: return launch_eval_g<256>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
+        case 512: return launch_eval_g<512>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -120,6 +122,7 @@ cudaError_t integrate_attributes(int group, bool mixed, int* maxThreads, int* re
         case 64: return integrate_attributes_g<64>(mixed, maxThreads, regs);
         case 128: return integrate_attributes_g<128>(mixed, maxThreads, regs);
         case 256: return integrate_attributes_g<256>(mixed, maxThreads, regs);
+        case 512: return integrate_attributes_g<512>(mixed, maxThreads, regs);
         default: return cudaErrorInvalidValue;
     }
 }

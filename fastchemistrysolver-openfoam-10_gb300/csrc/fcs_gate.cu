@@ -364,13 +364,9 @@ extern "C" fcs_status fcs_integrate_gated(fcs_ctx* ctx, int64_t nc, double dt, c
     CK(cudaMemsetAsync(g->counters.p, 0, QC_COUNT * sizeof(int), st));
     CK(cudaMemsetAsync(g->gstats.p, 0, GS_COUNT * sizeof(unsigned long long), st));
     // the fallback cells run with the plain method's mapping for this batch
-    const int group = ctx->opt.mapping ? ctx->opt.mapping : lane_auto(ctx, nc) ? (int)FCS_MAPPING_LANE : [&] {
-        const auto key = std::make_tuple(ctx->M.n, (int)ctx->opt.precision, (int)ctx->opt.solver, (int)ctx->opt.jacobian);
-        const auto it = ctx->tuned.find(key);
-        return it != ctx->tuned.end() ? it->second : default_group(ctx);
-    }();
+    const int group = lane_auto(ctx, nc) ? (int)FCS_MAPPING_LANE : auto_group(ctx, nc);
     Shape sh;
-    if (!make_shape(ctx, group, true, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
+    if (!make_shape(ctx, group, true, nc, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
     if (sh.global) {
         const size_t groups = (size_t)sh.lc.grid * (sh.lc.block / sh.lc.group);
         if (ctx->gws.ensure(groups * (size_t)sh.L.bytes) != cudaSuccess)

@@ -58,7 +58,8 @@ struct RxnEv {              // 64 bytes
 };
 static_assert(sizeof(RxnEv) == 64, "RxnEv must stay 64 bytes");
 
-struct JacChunk { int special, group0, groupEnd, pad; };  // first special reaction, groups of sums
+// Positions of a chunk's first special, Troe and SRI reaction; its groups of sums.
+struct JacChunk { int special, troe, sri, group0, groupEnd, pad[3]; };
 
 // Reactions per Jacobian chunk: a chunk's values stay in the slot until they
 // are summed, so small chunks let more cells reside and large ones keep more
@@ -98,11 +99,15 @@ struct DevMech {
     const double* plogTa;   // [rows]
     const int* incOff;      // [ns+1]
     const int* inc;         // (reaction << 1) | (1 if product else 0)
+    int plogSorted;         // every PLOG table's pressures ascend
     int nTbInc;             // third-body incidences (species row, third-body row, side)
     const int* tbInc;       // (row << 16) | (tb << 1) | (1 if product else 0), reaction order
     const double* hf;       // [ns] formation enthalpy at 298.15 K, J/kg (for Qdot)
     const RxnEv* ev;        // [nr] plain, third-body, special block (fcs_lists.h)
-    int evThird, evSpecial;
+    int evThird, evSpecial, evTroe, evSri;  // first of each part
+    int nTbRow;             // matrix rows with third-body terms
+    const int* tbRow;       // [nTbRow + 1][2] row, first term
+    const int* tbTerm;      // (third-body row << 1) | (1 if product else 0), in reaction order
     SumLists prod;          // net production per species
     JacLists jac[kJacVariants];
     const double* wiw;      // [ns][ns] W_i / W_j as W_i invW_j

@@ -50,9 +50,10 @@ __device__ __forceinline__ int attempt_bin(int attempts) {
 #endif
 
 struct LaunchCfg {
-    int group;                 // threads per cell: 32, 64, 128, 256, or 1 (lane per cell)
+    int group;                 // threads per cell: 32, 64, 128, 256, 512, or 1 (lane per cell)
     int block;                 // threads per block
     int grid;                  // blocks
+    int perSM;                 // blocks meant to reside per SM
 };
 
 cudaError_t launch_integrate(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,

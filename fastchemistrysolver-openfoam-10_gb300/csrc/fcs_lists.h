@@ -19,9 +19,12 @@
 #include <utility>
 #include <vector>
 
+#include "../../include/fcs.h"
 #include "fcs_internal.h"
 
 namespace fcs {
+
+constexpr int kTroe = FCS_RXN_TROE_FALLOFF, kSri = FCS_RXN_SRI_FALLOFF;
 
 // Sums, 32 to a group: elem[32 g + lane] = target << 16 | terms, the group's
 // terms from con[off[g]] on, term k of a lane at off[g] + 32 k + lane, each
@@ -67,7 +70,8 @@ struct HostChunks {
 
 struct HostLists {
     std::vector<RxnEv> ev;     // all reactions: plain ones, third-body ones, the special block
-    int evThird = 0, evSpecial = 0;  // first third-body / special position
+    int evThird = 0, evSpecial = 0, evTroe = 0, evSri = 0;  // first position of each part
+    std::vector<int> tbRow, tbTerm;  // third-body columns by matrix row (DevMech)
     HostSums prod;             // net production per species over q[r]
     HostChunks jac[kJacVariants];
 };
@@ -77,7 +81,7 @@ struct ListBlock {
     struct Sums { size_t elem, off, con; };
     struct Jac { size_t ev, chunk; Sums sums; };
     std::vector<char> bytes;
-    size_t ev = 0, wiw = 0;
+    size_t ev = 0, wiw = 0, tbRow = 0, tbTerm = 0;
     Sums prod{};
     Jac jac[kJacVariants]{};
     template<class T>
@@ -120,12 +124,23 @@ inline RxnEv make_ev(const RxnInfo& x, int r) {
     return e;
 }
 
+// Fall-off kinds last, each to itself: a Troe and an SRI rate are some 300
+// FP64 instructions each, so the kernels give each kind its own warp.
+inline int falloff_class(const RxnEv& e) { return e.kind == kTroe ? 1 : e.kind == kSri ? 2 : 0; }
+
 // Reactions that take the same path next to each other, the dearest kind first.
-inline void sort_ev(std::vector<RxnEv>::iterator a, std::vector<RxnEv>::iterator b) {
+inline void sort_ev(std::vector<RxnEv>& v) {
     auto key = [](const RxnEv& e) {
-        return std::make_tuple(e.plog < 0, e.tind, e.tb >= 0, e.rev, e.nl, e.nr, e.r);
+        return std::make_tuple(falloff_class(e), e.plog < 0, e.tind, e.tb >= 0, e.rev, e.nl, e.nr, e.r);
     };
-    std::sort(a, b, [&](const RxnEv& x, const RxnEv& y) { return key(x) < key(y); });
+    std::sort(v.begin(), v.end(), [&](const RxnEv& x, const RxnEv& y) { return key(x) < key(y); });
+}
+
+// First position of fall-off class c or above in v
+inline int first_of(const std::vector<RxnEv>& v, int c) {
+    int k = 0;
+    while (k < (int)v.size() && falloff_class(v[k]) < c) k++;
+    return k;
 }
 
 // rx: the packed reactions; inc[i]: (reaction << 1 | product) of species i in
@@ -137,11 +152,29 @@ inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, con
     std::vector<RxnEv> part[3];
     for (int r = 0; r < nr; r++) part[special(r) ? 2 : rx[r].tb >= 0 ? 1 : 0].push_back(make_ev(rx[r], r));
     for (auto& p : part) {
-        sort_ev(p.begin(), p.end());
+        sort_ev(p);
         H.ev.insert(H.ev.end(), p.begin(), p.end());
     }
     H.evThird = (int)part[0].size();
     H.evSpecial = H.evThird + (int)part[1].size();
+    H.evTroe = H.evSpecial + first_of(part[2], 1);
+    H.evSri = H.evSpecial + first_of(part[2], 2);
+    {
+        std::vector<std::vector<int>> rows(ns);
+        for (int r = 0; r < nr; r++) {
+            if (rx[r].tb < 0) continue;
+            for (int q = 0; q < rx[r].nl; q++) rows[rx[r].sl[q]].push_back(rx[r].tb << 1);
+            for (int q = 0; q < rx[r].nr; q++) rows[rx[r].sr[q]].push_back(rx[r].tb << 1 | 1);
+        }
+        for (int i = 0; i < ns; i++) {
+            if (rows[i].empty()) continue;
+            H.tbRow.push_back(i);
+            H.tbRow.push_back((int)H.tbTerm.size());
+            H.tbTerm.insert(H.tbTerm.end(), rows[i].begin(), rows[i].end());
+        }
+        H.tbRow.push_back(0);
+        H.tbRow.push_back((int)H.tbTerm.size());
+    }
     {
         std::vector<uint32_t> tgt;
         std::vector<std::vector<uint32_t>> terms;
@@ -159,8 +192,10 @@ inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, con
             const int c1 = std::min(nr, c0 + J.size);
             std::vector<RxnEv> main, sp;
             for (int r = c0; r < c1; r++) (special(r) ? sp : main).push_back(make_ev(rx[r], r));
-            sort_ev(main.begin(), main.end());
-            sort_ev(sp.begin(), sp.end());
+            sort_ev(main);
+            sort_ev(sp);
+            const int at0 = (int)(J.ev.size() + main.size());
+            JacChunk ch{at0, at0 + first_of(sp, 1), at0 + first_of(sp, 2), J.sums.groups(), 0, {}};
             main.insert(main.end(), sp.begin(), sp.end());
             // value index of every occurrence of the chunk's reactions
             std::vector<int> ent(c1 - c0);
@@ -171,7 +206,6 @@ inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, con
             }
             J.values = std::max(J.values, n);
             for (RxnEv& e : main) e.ent = ent[e.r - c0];
-            JacChunk ch{(int)J.ev.size() + (int)(main.size() - sp.size()), J.sums.groups(), 0, 0};
             J.ev.insert(J.ev.end(), main.begin(), main.end());
             std::vector<uint32_t> tgt;
             std::vector<std::vector<uint32_t>> terms;

@@ -112,17 +112,11 @@ extern "C" fcs_status fcs_integrate_noalloc(fcs_ctx* ctx, int64_t nc, double dt,
     CK(cudaMemcpyAsync(&nActive, dHead + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
 
-    // The autotuner allocates its trial copies, so it is not run here: an
-    // explicit mapping, else one the autotuner cached for this key, else the
-    // default for the mechanism size.
-    int group = ctx->opt.mapping;
-    if (!group) {
-        const auto key = std::make_tuple(ctx->M.n, (int)ctx->opt.precision, (int)ctx->opt.solver, (int)ctx->opt.jacobian);
-        const auto it = ctx->tuned.find(key);
-        group = it != ctx->tuned.end() ? it->second : default_group(ctx);
-    }
+    // AUTO as for many cells, whatever the call's count: another kernel variant
+    // could make the driver enlarge its local-memory reservation.
+    const int group = auto_group(ctx, FCS_NOALLOC_MAX_CELLS);
     Shape sh;
-    if (!make_shape(ctx, group, true, sh))
+    if (!make_shape(ctx, group, true, nActive, sh))
         return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
     if (sh.global)
         return set_err(ctx, FCS_ERR_UNSUPPORTED,

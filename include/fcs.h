@@ -92,7 +92,7 @@ enum { FCS_JACOBIAN_EXACT = 0, FCS_JACOBIAN_FAST = 1 };
  * small is redone in FP64.  Rates, thermo, equilibrium constants, the
  * Jacobian assembly, state and the step controller stay FP64. */
 enum { FCS_PRECISION_FP64 = 0, FCS_PRECISION_MIXED = 1 };
-/* Cell-to-thread mapping: AUTO lets the autotuner choose.  LANE: one thread
+/* Cell-to-thread mapping: AUTO chooses by mechanism size and cells.  LANE: one thread
  * per cell, the cells' working sets in a global-memory workspace interleaved
  * across the lanes of a warp (Rosenbrock-family solvers, FP64 or mixed); the others:
  * a group of 32..256 threads per cell with its working set in shared memory
@@ -110,9 +110,8 @@ enum {
                                   graph (counters, classify, queue, integrator,
                                   statistics), captured on the first call and
                                   replayed while the arrays, n_cells, delta_t and
-                                  options stay the same; the mapping is the
-                                  option's, else one the autotuner already chose,
-                                  else the default */
+                                  options stay the same; AUTO chooses the
+                                  mapping by n_cells */
 };
 
 /*
@@ -188,7 +187,7 @@ typedef struct fcs_step_stats {
     double  kernel_ms;           /* device time of the integration kernel */
     double  call_ms;             /* device time of the whole call on the library's
                                     stream, host<->device copies included */
-    int32_t mapping;             /* threads per cell used (autotuned for AUTO) */
+    int32_t mapping;             /* threads per cell used (AUTO: the one chosen) */
     int32_t reserved;
 } fcs_step_stats;
 
@@ -263,9 +262,8 @@ fcs_status fcs_integrate(fcs_ctx* ctx, int64_t n_cells, double delta_t,
  * reaches them; fcs_sync waits for the step and returns its statistics and
  * delta_t_min (same meaning as fcs_integrate's).  One step in flight per
  * context: a second fcs_integrate_async before fcs_sync returns
- * FCS_ERR_STATE.  The mapping is the option's, else one the autotuner already
- * chose for this context, else the default (the autotuner needs a host round
- * trip and is not run here).  flags: FCS_NO_QUEUE_SORT.
+ * FCS_ERR_STATE.  AUTO chooses the mapping by n_cells.  flags:
+ * FCS_NO_QUEUE_SORT.
  */
 fcs_status fcs_integrate_async(fcs_ctx* ctx, int64_t n_cells, double delta_t,
                                const double* p, const double* rho0,
@@ -321,9 +319,8 @@ fcs_status fcs_integrate_lts(fcs_ctx* ctx, int64_t n_cells, const double* delta_
  *     contexts) race on that array and must be serialised by the caller;
  *     consecutive calls from one thread are safe (each call returns after its
  *     work has finished);
- *   - the mapping autotuner is not run (it allocates trial copies): the
- *     mapping is fcs_options.mapping, else one the autotuner already cached in
- *     this context, else the default for the mechanism size;
+ *   - the mapping is fcs_options.mapping, else one chosen by the mechanism
+ *     size alone, so that a run launches one kernel variant;
  *   - the first call on a device looks up the array's address (which may load
  *     this library's device code); make it before any stream capture begins.
  */

@@ -45,3 +45,36 @@ def test_step_matches_oracle_at_panel_and_warp_edges(built, ns, mapping):
     assert (out["status"] == 0).all()
     np.testing.assert_allclose(out["T"], ref["T"], rtol=1e-7, atol=0)
     np.testing.assert_allclose(out["Y"], ref["Y"], rtol=0, atol=1e-8)
+
+
+@pytest.mark.parametrize("ns,solver", [(12, "OptRodas34"), (34, "OptSeulex"), (70, "OptRodas34"), (130, "OptRosenbrock34"),
+                                       (70, "OptSeulex")])
+def test_auto_results_do_not_depend_on_the_number_of_cells(built, ns, solver):
+    """AUTO takes other group sizes for few cells than for many; a cell's result is
+    the same to the last bit."""
+    from fcs import _lib
+    flat, cells = small_case(ns, n=8)
+    many = 12 * 152 if ns < 64 else 40
+    outs = []
+    for idx in (np.arange(8), np.arange(many) % 8):
+        ctx = _lib.Context(0)
+        ctx.load_mechanism(flat)
+        ctx.set_options(solver=solver)
+        outs.append(ctx.integrate(cells.subset(idx), 1e-7))
+    a, b = outs
+    for k in ("T", "Y", "subDt", "RR", "status"):
+        assert np.array_equal(a[k], b[k][..., :8]), k
+
+
+@pytest.mark.parametrize("ns", [34, 70])
+def test_auto_equals_its_partial_sum_width(built, ns):
+    """Up to 127 species AUTO sums as a group of 64 threads does, on any group."""
+    from fcs import _lib
+    flat, cells = small_case(ns, n=8)
+    outs = []
+    for mapping in (0, 64):
+        ctx = _lib.Context(0)
+        ctx.load_mechanism(flat)
+        ctx.set_options(mapping=mapping)
+        outs.append(ctx.integrate(cells, 1e-7))
+    assert np.array_equal(outs[0]["T"], outs[1]["T"]) and np.array_equal(outs[0]["Y"], outs[1]["Y"])

@@ -3,11 +3,12 @@
 // TMEM -> fused epilogue) and the forward, backward and Adam passes built on
 // it.  No counterpart in the reference.
 //
-// One GEMM kernel serves every product of training and inference:
+// One GEMM kernel serves every product of training (inference runs the whole
+// network in one kernel of its own, below):
 //   D[M][N] = A[M][K] . B[N][K]^T      (A, B BF16 K-major, D FP32 in TMEM)
 // with the epilogue selecting what happens to D:
 //   EPI_HIDDEN  z = D + b;  h = GELU(z)  -> h (row-major), z, h^T  (BF16)
-//   EPI_OUT     y = D + b (optionally de-normalised)   -> FP32 rows
+//   EPI_OUT     y = D + b                              -> FP32 rows
 //   EPI_DGRAD   dz = D * GELU'(z)        -> dz (row-major), dz^T  (BF16)
 //   EPI_WGRAD   dW += D                  (FP32 atomics; split-K over the batch)
 // Layers: forward  h_l = GELU(h_{l-1} W_l^T + b_l)      A = h_{l-1}, B = W_l
@@ -48,8 +49,6 @@ struct GemmArgs {
     int mode;
     int nValid;         // columns of D that are stored
     const float* bias;  // [N] (HIDDEN, OUT)
-    const float* outScale;  // OUT: y = (D + b) * scale + shift (null: no de-normalisation)
-    const float* outShift;
     bf16* h; int ldh;   // HIDDEN: GELU output; DGRAD: dz (row-major)
     bf16* z; int ldz;   // HIDDEN: pre-activation out (may be null); DGRAD: pre-activation in
     bf16* t; int ldt;   // HIDDEN: GELU output transposed; DGRAD: dz transposed (may be null)
@@ -185,9 +184,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
                 for (int i = 0; i < 16; i++) {
                     const int n = nb + i;
                     if (n < a.nValid) {
-                        float y = v[i] + a.bias[n];
-                        if (a.outScale) y = fmaf(y, a.outScale[n], a.outShift[n]);
-                        a.f[(size_t)m * a.ldf + n] = y;
+                        a.f[(size_t)m * a.ldf + n] = v[i] + a.bias[n];
                     }
                 }
             } else if (a.mode == EPI_DGRAD) {
@@ -212,6 +209,223 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
     if (warp == 1) {
         tc::tc_fence_after();
         tc::tmem_dealloc(tmem, BN);
+    }
+}
+
+// ---- inference: the whole network of one member in one kernel ----------------
+//
+// A block takes tiles of 128 rows through every layer: the tile's activations
+// stay in shared memory (128 x 256 BF16, K-major with 128-byte swizzle, the
+// layout the weights arrive in), the accumulator in 256 columns of TMEM, and
+// only the weights stream in (16 KB boxes of 128 neurons x 64 inputs through
+// a ring of kInferStages).  Warp 0 issues the TMA loads, warp 1 the MMAs.
+// Warps 2-9 normalise the input, apply bias and GELU to a layer's accumulator
+// and write it back as the next layer's operand, in place (every MMA of the
+// layer has completed by then); a pair of them shares 32 rows by columns.
+// What bounds it is the GELU: some 37 instructions a value, erff with a branch
+// that keeps a thread's values from overlapping, so it takes four such warps
+// per scheduler to fill the issue slots (two blocks per SM, 113 KB of shared
+// memory and half of the TMEM each).  As one GEMM launch per layer the
+// activations went through L2 and HBM between layers and the epilogue stored
+// 16-byte pieces of 32 rows at a time.  4 members of 56-256x4-55
+// through fcs_mlp_forward: 65,536 rows 1,047 -> 600 us, 1,000 rows 437 -> 292 us.
+
+constexpr int kMaxLayers = 9, kInferStages = 3, kWidth = 256;
+constexpr int kInferThreads = 320;
+constexpr int kBoxBytes = 128 * BK * 2;                    // one ring stage; one 64-column chunk of the activations
+constexpr int kInferSmem = (4 + kInferStages) * kBoxBytes + 256;
+
+struct InferArgs {
+    long long n;
+    int nIn, kPad, nOut, nOutPad, depth;
+    const float *x, *mean, *rstd;  // raw input [n][nIn] and its normalisation
+    const float* bias[kMaxLayers];
+    const float *scale, *shift;    // y = (D + b) scale + shift
+    float* y;                      // [n][nOut]
+    int* err;
+};
+
+struct InferMaps { CUtensorMap w[kMaxLayers]; };
+
+// Byte offset of element (r, k) of the activations
+__device__ __forceinline__ int act_offset(int r, int k) {
+    return (k >> 6) * kBoxBytes + r * 128 + ((((k & 63) >> 3) ^ (r & 7)) << 4) + (k & 7) * 2;
+}
+
+__global__ void __launch_bounds__(kInferThreads, 2)
+infer_kernel(const __grid_constant__ InferMaps maps, const InferArgs a) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* act = smem_raw;
+    uint8_t* ring = act + 4 * kBoxBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(ring + kInferStages * kBoxBytes);
+    uint64_t* empty = full + kInferStages;
+    uint64_t* ready = empty + kInferStages;   // the activations are written, the accumulator read
+    uint64_t* done = ready + 1;               // the layer's MMAs have completed
+    uint32_t* tmemBase = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemBase + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tiles = (int)((a.n + BM - 1) / BM);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kInferStages; s++) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        tc::mbar_init(ready, kInferThreads - 64);
+        tc::mbar_init(done, 1);
+        // the swizzle needs the tile bases on 1024 bytes
+        *abortFlag = (tc::smem_u32(smem_raw) & 1023u) != 0;
+        if (*abortFlag && a.err) atomicCAS(a.err, 0, 7);
+        tc::fence_mbar_init();
+        for (int l = 0; l <= a.depth; l++) tc::tma_prefetch_map(&maps.w[l]);
+    }
+    if (warp == 1) tc::tmem_alloc(tmemBase, kWidth);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = *tmemBase;
+    const bool run = !*abortFlag;
+
+    if (warp == 0 && lane == 0 && run) {
+        int i = 0;  // loads issued
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x)
+            for (int l = 0; ok && l <= a.depth; l++) {
+                const int chunks = (l == 0 ? a.kPad : kWidth) / BK, halves = (l == a.depth ? a.nOutPad : kWidth) / 128;
+                for (int c = 0; ok && c < chunks * halves; c++) {
+                    const int s = i % kInferStages;
+                    if (i >= kInferStages && !tc::mbar_wait(&empty[s], ((i / kInferStages) - 1) & 1, a.err, 4, abortFlag)) {
+                        ok = false;
+                        break;
+                    }
+                    tc::mbar_arrive_expect_tx(&full[s], kBoxBytes);
+                    tc::tma_load_2d(ring + s * kBoxBytes, &maps.w[l], &full[s], (c / halves) * BK, (c % halves) * 128);
+                    i++;
+                }
+            }
+        if (!ok) {
+            // given up: the loads in flight still write this block's shared memory
+            int none = 0;
+            for (int k = i > kInferStages ? i - kInferStages : 0; k < i; k++)
+                tc::mbar_wait(&full[k % kInferStages], (k / kInferStages) & 1, nullptr, 0, &none);
+        }
+    } else if (warp == 1 && lane == 0 && run) {
+        constexpr uint32_t idesc = tc::idesc_bf16_f32(BM, 128);
+        int i = 0, k = 0;  // ring stages consumed, layer under way
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x)
+            for (int l = 0; ok && l <= a.depth; l++) {
+                const int chunks = (l == 0 ? a.kPad : kWidth) / BK, halves = (l == a.depth ? a.nOutPad : kWidth) / 128;
+                ok = tc::mbar_wait(ready, k & 1, a.err, 5, abortFlag);
+                tc::tc_fence_after();
+                for (int c = 0; ok && c < chunks * halves; c++, i++) {
+                    const int s = i % kInferStages;
+                    ok = tc::mbar_wait(&full[s], (i / kInferStages) & 1, a.err, 6, abortFlag);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    const uint32_t sa = tc::smem_u32(act + (c / halves) * kBoxBytes);
+                    const uint32_t sb = tc::smem_u32(ring + s * kBoxBytes);
+#pragma unroll
+                    for (int j = 0; j < BK / 16; j++)
+                        tc::mma_bf16(tmem + (c % halves) * 128, tc::desc_k_sw128(sa + 32 * j),
+                                     tc::desc_k_sw128(sb + 32 * j), idesc, (c / halves | j) != 0);
+                    tc::mma_commit(&empty[s]);
+                }
+                tc::mma_commit(done);
+                if (!ok) {
+                    // given up: wait for the MMAs already issued, they read this block's shared memory
+                    int none = 0;
+                    tc::mbar_wait(done, k & 1, nullptr, 0, &none);
+                }
+                k++;
+            }
+    } else if (warp >= 2 && run) {
+        // a warp reads and writes its own rows (input) or rows and columns only
+        const int q = warp & 3, part = (warp - 2) >> 2, r = 32 * q + lane;
+        const uint32_t lanes = tmem + (static_cast<uint32_t>(32 * q) << 16);
+        int k = 0;  // layers finished
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+            const long long m0 = (long long)tile * BM;
+            const int rows = (int)min((long long)BM, a.n - m0);
+            // the input, normalised, zero in the padding; eight rows' loads in
+            // flight (one at a time took 25 us a tile)
+            for (int k2 = 2 * lane; k2 < a.kPad; k2 += 64) {
+                const bool in0 = k2 < a.nIn, in1 = k2 + 1 < a.nIn;
+                const float m0k = in0 ? __ldg(a.mean + k2) : 0.f, m1k = in1 ? __ldg(a.mean + k2 + 1) : 0.f;
+                const float s0k = in0 ? __ldg(a.rstd + k2) : 0.f, s1k = in1 ? __ldg(a.rstd + k2 + 1) : 0.f;
+                for (int r0 = 32 * q + 16 * part; r0 < 32 * q + 16 * part + 16; r0 += 8) {
+                    float x0[8], x1[8];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        const float* x = a.x + (m0 + r0 + u) * a.nIn + k2;
+                        x0[u] = r0 + u < rows && in0 ? x[0] : m0k;
+                        x1[u] = r0 + u < rows && in1 ? x[1] : m1k;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; u++)
+                        *reinterpret_cast<__nv_bfloat162*>(act + act_offset(r0 + u, k2)) =
+                            __floats2bfloat162_rn((x0[u] - m0k) * s0k, (x1[u] - m1k) * s1k);
+                }
+            }
+            tc::fence_async_shared();
+            tc::mbar_arrive(ready);
+            for (int l = 0; l <= a.depth; l++, k++) {
+                if (!tc::mbar_wait(done, k & 1, a.err, 3, abortFlag)) ok = false;
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc::tc_fence_after();
+                const float* bias = a.bias[l];
+                if (l < a.depth) {
+                    for (int c0 = 128 * part; c0 < 128 * part + 128; c0 += 16) {
+                        float v[16];
+                        tc::tmem_ld16(lanes + c0, v);
+                        __align__(16) __nv_bfloat162 h[8];
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const float4 b = __ldg(reinterpret_cast<const float4*>(bias + c0) + u);
+                            h[2 * u] = __floats2bfloat162_rn(gelu(v[4 * u] + b.x), gelu(v[4 * u + 1] + b.y));
+                            h[2 * u + 1] = __floats2bfloat162_rn(gelu(v[4 * u + 2] + b.z), gelu(v[4 * u + 3] + b.w));
+                        }
+#pragma unroll
+                        for (int u = 0; u < 2; u++)
+                            *reinterpret_cast<uint4*>(act + act_offset(r, c0 + 8 * u)) = reinterpret_cast<const uint4*>(h)[u];
+                    }
+                    tc::tc_fence_before();
+                    tc::fence_async_shared();
+                    tc::mbar_arrive(ready);
+                } else {
+                    // 16 columns at a time through the rows' own bytes of the
+                    // activations (free now), to leave as runs along the rows
+                    for (int c0 = 16 * part; c0 < a.nOut; c0 += 32) {
+                        float v[16];
+                        tc::tmem_ld16(lanes + c0, v);
+                        float* mine = reinterpret_cast<float*>(act + part * kBoxBytes);
+#pragma unroll
+                        for (int u = 0; u < 16; u++) {
+                            const int c = c0 + u;
+                            if (c < a.nOut)
+                                mine[r * 32 + ((u ^ r) & 15)] =
+                                    fmaf(v[u] + __ldg(bias + c), __ldg(a.scale + c), __ldg(a.shift + c));
+                        }
+                        __syncwarp();
+                        const int u = lane & 15, c = c0 + u;
+                        if (c < a.nOut) {
+#pragma unroll 4
+                            for (int rr = 32 * q + (lane >> 4); rr < 32 * q + 32; rr += 2)
+                                if (rr < rows) a.y[(m0 + rr) * a.nOut + c] = mine[rr * 32 + ((u ^ rr) & 15)];
+                        }
+                        __syncwarp();
+                    }
+                    tc::tc_fence_before();
+                }
+            }
+        }
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc(tmem, kWidth);
     }
 }
 
@@ -287,10 +501,11 @@ __global__ void rowsum_kernel(int rows, int n, const bf16* T, int ldT, float* db
 }
 
 // Adam on one layer (lr > 0) or a plain publish (lr == 0), then the BF16
-// copies W[n][k] (ld kPad) and WT[k][n] (ld nPad) of the updated weights.
+// copies W[n][k] (ld kPad) and WT[k][n] (ld nPad) of the updated weights and
+// the aligned copy of the biases.
 __global__ void adam_publish_kernel(int nOut, int nIn, int kPad, int nPad, float* W, float* b, float* mW, float* vW,
                                     float* mb, float* vb, const float* gW, const float* gb, float lr, float beta1,
-                                    float beta2, float eps, float c1, float c2, bf16* Wbf, bf16* WTbf) {
+                                    float beta2, float eps, float c1, float c2, bf16* Wbf, bf16* WTbf, float* bCopy) {
     const int total = nOut * nIn + nOut;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const bool isW = i < nOut * nIn;
@@ -311,6 +526,8 @@ __global__ void adam_publish_kernel(int nOut, int nIn, int kPad, int nPad, float
             const bf16 w = __float2bfloat16_rn(*p);
             Wbf[(size_t)n * kPad + k] = w;
             WTbf[(size_t)k * nPad + n] = w;
+        } else {
+            bCopy[n] = *p;
         }
     }
 }
@@ -376,6 +593,17 @@ cudaError_t gemm(const bf16* A, int lda, const bf16* B, int ldb, int M, int N, i
     return launch_gemm_bn<128, 3>(ma, mb, a, grid, st);
 }
 
+cudaError_t launch_infer(const InferMaps& maps, const InferArgs& a, int numSMs, cudaStream_t st) {
+    cudaError_t e = cudaFuncSetAttribute(infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(infer_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    const long long tiles = (a.n + BM - 1) / BM;
+    infer_kernel<<<(int)std::min<long long>(tiles, 2LL * numSMs), kInferThreads, kInferSmem, st>>>(maps, a);
+    return cudaGetLastError();
+}
+
 int blocks_for(long long n, int block) {
     long long b = (n + block - 1) / block;
     return (int)std::max(1LL, std::min(b, 152LL * 32));
@@ -423,6 +651,8 @@ struct Layer {
 struct Member {
     DArr<float> params, m, v;
     std::vector<DArr<bf16>> W, WT;
+    InferMaps maps;        // W of every layer, 128 x 64 boxes
+    DArr<float> bias;      // [layer][256], 16-byte aligned rows for the inference kernel
     long long step = 0;
 };
 
@@ -431,7 +661,7 @@ int round_up(int x, int m) { return (x + m - 1) / m * m; }
 }  // namespace
 
 struct fcs_mlp {
-    int device = 0;
+    int device = 0, numSMs = 0;
     cudaStream_t st = nullptr;
     fcs_mlp_shape sh{};
     std::vector<Layer> L;
@@ -481,13 +711,13 @@ static fcs_status publish(fcs_mlp* mlp, int e) {
         const Layer& y = mlp->L[l];
         adam_publish_kernel<<<blocks_for((long long)y.out * y.in + y.out, 256), 256, 0, mlp->st>>>(
             y.out, y.in, y.kPad, y.nPad, M.params.p + y.wOff, M.params.p + y.bOff, nullptr, nullptr, nullptr, nullptr,
-            nullptr, nullptr, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, M.W[l].p, M.WT[l].p);
+            nullptr, nullptr, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, M.W[l].p, M.WT[l].p, M.bias.p + 256 * l);
         MCK(cudaGetLastError());
     }
     return FCS_OK;
 }
 
-static fcs_status ensure_acts(fcs_mlp* mlp, int64_t rows, bool training) {
+static fcs_status ensure_acts(fcs_mlp* mlp, int64_t rows) {
     const int w = mlp->sh.width, k0 = mlp->L.front().kPad, no = mlp->L.back().nPad;
     const size_t r = (size_t)round_up((int)rows, 128);
     MCK(mlp->X.ensure(r * k0));
@@ -496,12 +726,6 @@ static fcs_status ensure_acts(fcs_mlp* mlp, int64_t rows, bool training) {
     mlp->Z.resize(depth);
     mlp->H.resize(depth);
     mlp->HT.resize(depth);
-    if (!training) {
-        // inference: two ping-pong hidden buffers
-        MCK(mlp->H[0].ensure(r * w));
-        if (depth > 1) MCK(mlp->H[1].ensure(r * w));
-        return FCS_OK;
-    }
     MCK(mlp->XT.ensure(r * k0));
     MCK(mlp->dOut.ensure(r * no));
     MCK(mlp->dOutT.ensure(r * no));
@@ -522,11 +746,9 @@ static GemmArgs base_args(fcs_mlp* mlp) {
     return a;
 }
 
-// Forward pass of member e over the packed input mlp->X ([n][kPad0]).
-// training: stores Z, H, H^T of every hidden layer and the normalised output
-// in mlp->Out; inference: ping-pong hidden buffers, output de-normalised into
-// y (ld n_out).
-static fcs_status forward_packed(fcs_mlp* mlp, int e, int n, bool training, float* y, cudaStream_t st) {
+// Training forward of member e over the packed input mlp->X ([n][kPad0]):
+// stores Z, H, H^T of every hidden layer and the normalised output in mlp->Out.
+static fcs_status forward_packed(fcs_mlp* mlp, int e, int n, cudaStream_t st) {
     Member& M = mlp->mem[e];
     const int depth = mlp->sh.depth, w = mlp->sh.width;
     const int ldT = round_up(n, 128);
@@ -538,32 +760,25 @@ static fcs_status forward_packed(fcs_mlp* mlp, int e, int n, bool training, floa
         a.bias = M.params.p + ly.bOff;
         if (l < depth) {
             a.mode = EPI_HIDDEN;
-            bf16* h = training ? mlp->H[l].p : mlp->H[l & 1].p;
+            bf16* h = mlp->H[l].p;
             a.h = h; a.ldh = w;
-            if (training) {
-                a.z = mlp->Z[l].p; a.ldz = w;
-                a.t = mlp->HT[l].p; a.ldt = ldT;
-            }
+            a.z = mlp->Z[l].p; a.ldz = w;
+            a.t = mlp->HT[l].p; a.ldt = ldT;
             a.nValid = ly.nPad;
             MCK(gemm(A, lda, M.W[l].p, ly.kPad, n, ly.nPad, ly.kPad, 1, a, st));
             A = h;
             lda = w;
         } else {
             a.mode = EPI_OUT;
-            a.nValid = ly.out;  // padding columns of the training output are never read
-            if (training) {
-                a.f = mlp->Out.p; a.ldf = ly.nPad;
-            } else {
-                a.f = y; a.ldf = ly.out;
-                a.outScale = mlp->outStd.p; a.outShift = mlp->outMean.p;
-            }
+            a.nValid = ly.out;  // padding columns of the output are never read
+            a.f = mlp->Out.p; a.ldf = ly.nPad;
             MCK(gemm(A, lda, M.W[l].p, ly.kPad, n, ly.nPad, ly.kPad, 1, a, st));
         }
     }
     return FCS_OK;
 }
 
-// Backward pass of member e after forward_packed(training) and the loss
+// Backward pass of member e after forward_packed and the loss
 // kernel: fills mlp->gW / mlp->gb (zeroed here).
 static fcs_status backward(fcs_mlp* mlp, int e, int n) {
     Member& M = mlp->mem[e];
@@ -645,7 +860,7 @@ extern "C" fcs_status fcs_mlp_destroy(fcs_mlp* mlp) {
     cudaSetDevice(mlp->device);
     if (mlp->st) cudaStreamSynchronize(mlp->st);
     for (auto& M : mlp->mem) {
-        M.params.release(); M.m.release(); M.v.release();
+        M.params.release(); M.m.release(); M.v.release(); M.bias.release();
         for (auto& b : M.W) b.release();
         for (auto& b : M.WT) b.release();
     }
@@ -696,6 +911,7 @@ extern "C" fcs_status fcs_mlp_create(fcs_mlp** out, int device, const fcs_mlp_sh
     fcs_mlp* mlp = new fcs_mlp();
     mlp->device = device;
     mlp->sh = *s;
+    cudaDeviceGetAttribute(&mlp->numSMs, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&mlp->st, cudaStreamNonBlocking) != cudaSuccess) {
         delete mlp;
         return FCS_ERR_CUDA;
@@ -728,13 +944,15 @@ extern "C" fcs_status fcs_mlp_create(fcs_mlp** out, int device, const fcs_mlp_sh
     std::vector<float> host(off);
     for (int e = 0; e < s->members; e++) {
         Member& M = mlp->mem[e];
-        if (M.params.ensure(off) || M.m.ensure(off) || M.v.ensure(off)) return fail(FCS_ERR_NOMEM);
+        if (M.params.ensure(off) || M.m.ensure(off) || M.v.ensure(off) || M.bias.ensure(256 * mlp->L.size()))
+            return fail(FCS_ERR_NOMEM);
         M.W.resize(mlp->L.size());
         M.WT.resize(mlp->L.size());
         for (size_t l = 0; l < mlp->L.size(); l++) {
             const Layer& y = mlp->L[l];
             if (M.W[l].ensure((size_t)y.nPad * y.kPad) || M.WT[l].ensure((size_t)y.nPad * y.kPad))
                 return fail(FCS_ERR_NOMEM);
+            if (!make_map(&M.maps.w[l], M.W[l].p, y.nPad, y.kPad, y.kPad, 128)) return fail(FCS_ERR_CUDA);
         }
         // He initialisation; the output layer starts 10x smaller
         std::mt19937_64 rng(seed + (uint64_t)e);
@@ -798,13 +1016,24 @@ fcs_status fcs::mlp_forward_device(fcs_mlp* mlp, int member, int64_t n, const fl
     if (!mlp || member < 0 || member >= mlp->sh.members) return mlp_err(mlp, FCS_ERR_INVALID, "bad member");
     if (n <= 0) return FCS_OK;
     if (n > (1LL << 24)) return mlp_err(mlp, FCS_ERR_INVALID, "too many rows");
-    fcs_status s = ensure_acts(mlp, n, false);
-    if (s != FCS_OK) return s;
-    const Layer& l0 = mlp->L[0];
-    pack_input_kernel<<<blocks_for(n * l0.kPad, 256), 256, 0, st>>>((int)n, l0.in, l0.kPad, x, nullptr, 0,
-                                                                     mlp->inMean.p, mlp->inRstd.p, mlp->X.p, nullptr, 0);
-    MCK(cudaGetLastError());
-    return forward_packed(mlp, member, (int)n, false, y, st);
+    const Member& M = mlp->mem[member];
+    InferArgs a{};
+    a.n = n;
+    a.nIn = mlp->sh.n_in;
+    a.kPad = mlp->L.front().kPad;
+    a.nOut = mlp->sh.n_out;
+    a.nOutPad = mlp->L.back().nPad;
+    a.depth = mlp->sh.depth;
+    a.x = x;
+    a.mean = mlp->inMean.p;
+    a.rstd = mlp->inRstd.p;
+    for (size_t l = 0; l < mlp->L.size(); l++) a.bias[l] = M.bias.p + 256 * l;
+    a.scale = mlp->outStd.p;
+    a.shift = mlp->outMean.p;
+    a.y = y;
+    a.err = mlp->err.p;
+    MCK(launch_infer(M.maps, a, mlp->numSMs, st));
+    return FCS_OK;
 }
 
 fcs_status fcs::mlp_check_errors(fcs_mlp* mlp) { return check_device_err(mlp); }
@@ -847,7 +1076,7 @@ static fcs_status fwd_bwd(fcs_mlp* mlp, int e, int n, const float* x, const floa
     pack_input_kernel<<<blocks_for((long long)n * l0.kPad, 256), 256, 0, st>>>(
         n, l0.in, l0.kPad, x, perm, off, mlp->inMean.p, mlp->inRstd.p, mlp->X.p, mlp->XT.p, ldT);
     MCK(cudaGetLastError());
-    fcs_status s = forward_packed(mlp, e, n, true, nullptr, st);
+    fcs_status s = forward_packed(mlp, e, n, st);
     if (s != FCS_OK) return s;
     loss_grad_kernel<<<blocks_for((long long)n * lo.nPad, 256), 256, 0, st>>>(
         n, lo.out, lo.nPad, mlp->Out.p, t, perm, off, mlp->outMean.p, mlp->outStd.p, mlp->dOut.p, mlp->dOutT.p, ldT,
@@ -862,7 +1091,7 @@ extern "C" fcs_status fcs_mlp_gradients(fcs_mlp* mlp, int32_t e, int64_t n, cons
     if (e < 0 || e >= mlp->sh.members) return mlp_err(mlp, FCS_ERR_INVALID, "bad member");
     if (n <= 0 || n % 128 || n > (1 << 20)) return mlp_err(mlp, FCS_ERR_INVALID, "n must be a positive multiple of 128");
     cudaSetDevice(mlp->device);
-    fcs_status s = ensure_acts(mlp, n, true);
+    fcs_status s = ensure_acts(mlp, n);
     if (s != FCS_OK) return s;
     MCK(mlp->xDev.ensure((size_t)n * mlp->sh.n_in));
     MCK(mlp->tDev.ensure((size_t)n * mlp->sh.n_out));
@@ -899,7 +1128,7 @@ extern "C" fcs_status fcs_mlp_train(fcs_mlp* mlp, int64_t n, const float* x, con
     if (n < o.batch) return mlp_err(mlp, FCS_ERR_INVALID, "fewer samples than one batch");
     cudaSetDevice(mlp->device);
     cudaStream_t st = mlp->st;
-    fcs_status s = ensure_acts(mlp, o.batch, true);
+    fcs_status s = ensure_acts(mlp, o.batch);
     if (s != FCS_OK) return s;
     MCK(mlp->xDev.ensure((size_t)n * mlp->sh.n_in));
     MCK(mlp->tDev.ensure((size_t)n * mlp->sh.n_out));
@@ -932,7 +1161,7 @@ extern "C" fcs_status fcs_mlp_train(fcs_mlp* mlp, int64_t n, const float* x, con
                         y.out, y.in, y.kPad, y.nPad, M.params.p + y.wOff, M.params.p + y.bOff, M.m.p + y.wOff,
                         M.v.p + y.wOff, M.m.p + y.bOff, M.v.p + y.bOff, mlp->gW.p + y.gOff, mlp->gb.p + y.gbOff,
                         (float)lr, (float)o.beta1, (float)o.beta2, (float)o.eps, c1, c2,
-                        M.W[&y - &mlp->L[0]].p, M.WT[&y - &mlp->L[0]].p);
+                        M.W[&y - &mlp->L[0]].p, M.WT[&y - &mlp->L[0]].p, M.bias.p + 256 * (&y - &mlp->L[0]));
                 }
                 MCK(cudaGetLastError());
             }

@@ -676,6 +676,28 @@ __device__ __forceinline__ ThermoScalars thermo_scalars(const Grp<G>& g, double*
     return t;
 }
 
+// Two sums sum_i a_i b_i in species order, as one thread would take them (a
+// null: the constant ac): s.rw == 1, the lane mapping's sums.  The chains run
+// in two lanes of one warp, so that the pair costs one FP64 instruction per
+// species; the group's arrays are complete before (a barrier here).
+struct SumOf { const double* a; double ac; const double* b; };
+template<int G>
+__device__ __forceinline__ void serial_sums(const Grp<G>& g, int n, const SumOf& f, const SumOf& h, double* red,
+                                            double& x, double& y) {
+    g.sync();
+    if (g.rank < 2) {
+        const SumOf s = g.rank ? h : f;
+        double v = 0;
+        #pragma unroll 8
+        for (int i = 0; i < n; i++) v = fma(s.a ? s.a[i] : s.ac, s.b[i], v);
+        red[g.rank] = v;
+    }
+    g.sync();
+    x = red[0];
+    y = red[1];
+    if constexpr (G == 32) g.sync();
+}
+
 // M_t = sum_j eff[t][j] C_j (ThirdBodyFactor1D)
 template<int G, class MT>
 __device__ __forceinline__ void third_bodies(const Grp<G>& g, const DevMech& M, const Slot<MT>& s) {
@@ -875,12 +897,22 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
     const double T = YT[ns];
     const double Tc = clampT(M, T);
     const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * T, p);
-    double part = 0;
-    for (int i = r0; i < ns; i += s.rw) {
-        const double y0 = YT[i];
-        part = fma((positive(y0) ? y0 : 0.0) * __ldg(&M.invW[i]), t.numByP, part);
+    double invrhoM = 0;
+    if (s.rw == 1) {
+        for (int i = g.rank; i < ns; i += G) {
+            const double y0 = YT[i];
+            s.C[i] = (positive(y0) ? y0 : 0.0) * __ldg(&M.invW[i]);
+        }
+        const SumOf f{nullptr, t.numByP, s.C};
+        double same;
+        serial_sums(g, ns, f, f, s.red, invrhoM, same);
+    } else {
+        for (int i = r0; i < ns; i += s.rw) {
+            const double y0 = YT[i];
+            invrhoM = fma((positive(y0) ? y0 : 0.0) * __ldg(&M.invW[i]), t.numByP, invrhoM);
+        }
+        invrhoM = gsum(g, invrhoM, s.red);
     }
-    const double invrhoM = gsum(g, part, s.red);
     const double rhoM = 1.0 / invrhoM;
     const double Tp = mode == 2 ? T : Tc;
     for (int i = g.rank; i < ns; i += G) {
@@ -902,13 +934,17 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
     net_production<G, MT>(g, M, s, out);
     g.sync();
     for (int i = g.rank; i < ns; i += G) out[i] = (__ldg(&M.W[i]) * invrhoM) * out[i];
-    if (s.rw < G) g.sync();
     double cpm = 0, dtd = 0;
-    for (int i = r0; i < ns; i += s.rw) {
-        cpm = fma(YT[i], s.Cp[i], cpm);
-        dtd = fma(s.Ha[i], out[i], dtd);
+    if (s.rw == 1) {
+        serial_sums(g, ns, SumOf{YT, 0, s.Cp}, SumOf{s.Ha, 0, out}, s.red, cpm, dtd);
+    } else {
+        if (s.rw < G) g.sync();
+        for (int i = r0; i < ns; i += s.rw) {
+            cpm = fma(YT[i], s.Cp[i], cpm);
+            dtd = fma(s.Ha[i], out[i], dtd);
+        }
+        gsum2(g, cpm, dtd, s.red);
     }
-    gsum2(g, cpm, dtd, s.red);
     if (g.rank == 0) out[ns] = -dtd / cpm;
     g.sync();
 }
@@ -1100,12 +1136,21 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * Tc, p);
     const double logT = t.logT, invT = t.invT;
     double rs = 0, mws = 0;
-    for (int i = r0; i < ns; i += s.rw) {
-        const double y0 = YT[i], y = positive(y0) ? y0 : 0.0, invW = __ldg(&M.invW[i]);
-        rs = fma(t.numByP, y * invW, rs);
-        mws = fma(y, invW, mws);
+    if (s.rw == 1) {
+        for (int i = g.rank; i < ns; i += G) {
+            const double y0 = YT[i], y = positive(y0) ? y0 : 0.0;
+            YT[i] = y;
+            s.C[i] = y * __ldg(&M.invW[i]);
+        }
+        serial_sums(g, ns, SumOf{nullptr, t.numByP, s.C}, SumOf{YT, 0, M.invW}, s.red, rs, mws);
+    } else {
+        for (int i = r0; i < ns; i += s.rw) {
+            const double y0 = YT[i], y = positive(y0) ? y0 : 0.0, invW = __ldg(&M.invW[i]);
+            rs = fma(t.numByP, y * invW, rs);
+            mws = fma(y, invW, mws);
+        }
+        gsum2(g, rs, mws, s.red);
     }
-    gsum2(g, rs, mws, s.red);
     const double rhoM = 1.0 / rs, invRhoM = rs, MW = 1.0 / mws;
     for (int i = g.rank; i < ns; i += G) {
         const double y0 = YT[i], y = positive(y0) ? y0 : 0.0, invW = __ldg(&M.invW[i]);
@@ -1126,12 +1171,16 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     g.sync();
     third_bodies<G, MT>(g, M, s);
     if constexpr (G == 32) g.sync();
-    double cpm = 0, dcpm = 0;
-    for (int i = r0; i < ns; i += s.rw) {
-        cpm = fma(YT[i], s.Cp[i], cpm);
-        dcpm = fma(YT[i], s.dCpdT[i], dcpm);
+    double cpm = 0, dcpm = 0;  // the sums' barriers publish the third bodies
+    if (s.rw == 1) {
+        serial_sums(g, ns, SumOf{YT, 0, s.Cp}, SumOf{YT, 0, s.dCpdT}, s.red, cpm, dcpm);
+    } else {
+        for (int i = r0; i < ns; i += s.rw) {
+            cpm = fma(YT[i], s.Cp[i], cpm);
+            dcpm = fma(YT[i], s.dCpdT[i], dcpm);
+        }
+        gsum2(g, cpm, dcpm, s.red);
     }
-    gsum2(g, cpm, dcpm, s.red);  // its barriers publish the third bodies
     const double CpM = cpm, dCpMdT = dcpm;
     const double logP = s.red[37];
     const JacLists& L = M.jac[s.jv];
@@ -1228,7 +1277,8 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
         }
         g.sync();  // the next chunk overwrites the values; the passes below read J
     }
-    // third-body columns, J_ij += nu_i w_t E_tj (JF* third-body block).  Up to
+    // third-body columns, J_ij += nu_i w_t E_tj (JF* third-body block; one
+    // rounding when summing as the lane mapping does).  Up to
     // 64 threads own columns: the entries come in reaction order and a
     // reaction's products E w are formed once.  More threads than columns
     // share out the elements of the rows that have terms (one more product a
@@ -1237,16 +1287,18 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     if constexpr (G <= 64) {
         for (int j = g.rank; j < ns; j += G) {
             int last = -1;
-            double wd = 0;
+            double e0 = 0, wd = 0;
             for (int e = 0; e < M.nTbInc; e++) {
                 const int v = __ldg(&M.tbInc[e]);
                 const int i = v >> 16, tb = (v >> 1) & 0x7fff;
                 if (tb != last) {
-                    wd = __ldg(&M.eff[(size_t)tb * ns + j]) * s.tbF[tb];
+                    e0 = __ldg(&M.eff[(size_t)tb * ns + j]);
+                    wd = __dmul_rn(e0, s.tbF[tb]);
                     last = tb;
                 }
                 MT& c = J[i * ld + j];
-                c = (v & 1) ? c + MT(wd) : c - MT(wd);
+                const double w = v & 1 ? s.tbF[tb] : -s.tbF[tb], d = v & 1 ? wd : -wd;
+                c = s.rw == 1 ? MT(fma(e0, w, double(c))) : MT(double(c) + d);
             }
         }
     } else {
@@ -1259,8 +1311,8 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
             #pragma unroll 2
             for (int e = e0; e < e1; e++) {
                 const int c = __ldg(M.tbTerm + e), tb = c >> 1;
-                const double wd = __dmul_rn(__ldg(&M.eff[(size_t)tb * ns + j]), s.tbF[tb]);
-                v += (c & 1) ? wd : -wd;
+                const double e0 = __ldg(&M.eff[(size_t)tb * ns + j]), w = c & 1 ? s.tbF[tb] : -s.tbF[tb];
+                v = s.rw == 1 ? fma(e0, w, v) : v + __dmul_rn(e0, w);
             }
             o = MT(v);
             r += dr;
@@ -1315,12 +1367,17 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
         }
     }
     double dtd = 0, dd = 0;
-    for (int i = r0; i < ns; i += s.rw) {
-        const double dY = f[i], tcol = double(J[i * ld + ns]);
-        dtd = fma(s.Ha[i], dY, dtd);
-        dd += dY * s.Cp[i] + tcol * s.Ha[i];
+    if (s.rw == 1) {
+        for (int i = g.rank; i < ns; i += G) s.B[i] = f[i] * s.Cp[i] + double(J[i * ld + ns]) * s.Ha[i];
+        serial_sums(g, ns, SumOf{s.Ha, 0, f}, SumOf{nullptr, 1.0, s.B}, s.red, dtd, dd);
+    } else {
+        for (int i = r0; i < ns; i += s.rw) {
+            const double dY = f[i], tcol = double(J[i * ld + ns]);
+            dtd = fma(s.Ha[i], dY, dtd);
+            dd += dY * s.Cp[i] + tcol * s.Ha[i];
+        }
+        gsum2(g, dtd, dd, s.red);
     }
-    gsum2(g, dtd, dd, s.red);
     const double dTdt = -dtd / CpM;
     g.sync();
     // temperature row (ddTdtdYT): column owners

@@ -78,3 +78,21 @@ def test_auto_equals_its_partial_sum_width(built, ns):
         ctx.set_options(mapping=mapping)
         outs.append(ctx.integrate(cells, 1e-7))
     assert np.array_equal(outs[0]["T"], outs[1]["T"]) and np.array_equal(outs[0]["Y"], outs[1]["Y"])
+
+
+@pytest.mark.parametrize("ns,solver", [(34, "OptRodas34"), (34, "OptRosenbrock23"), (50, "OptRodas34")])
+def test_auto_equals_the_lanes_on_large_batches(built, ns, solver):
+    """From three quarters of a cell per lane on AUTO sums as the lane mapping does:
+    groups (below 1.1 cells per lane) and lanes give a cell the same bits."""
+    from fcs import _lib
+    flat, cells = small_case(ns, n=16)
+    outs = []
+    for mapping, n in ((1, 16), (0, 44000), (0, 66000)):
+        ctx = _lib.Context(0)
+        ctx.load_mechanism(flat)
+        ctx.set_options(solver=solver, mapping=mapping)
+        outs.append(ctx.integrate(cells.subset(np.arange(n) % 16), 1e-8))
+    assert outs[1]["stats"]["mapping"] > 1 and outs[2]["stats"]["mapping"] == 1
+    for o in outs[1:]:
+        for k in ("T", "Y", "subDt", "RR", "status"):
+            assert np.array_equal(outs[0][k], o[k][..., :16]), k

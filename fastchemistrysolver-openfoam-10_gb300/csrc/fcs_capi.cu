@@ -219,16 +219,25 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
                        "reaction types other than (ir)reversible Arrhenius, ThirdBodyArrhenius, "
                        "ArrheniusLindemann/Troe/SRIFallOff, ArrheniusPLOG and nonEquilibriumReversible"
                        "(ThirdBody)Arrhenius are not supported by the GPU path");
-    std::vector<double> W(ns), invW(ns), Tc(ns), coef(16 * (size_t)ns, 0.0), hf(ns);
+    std::vector<double> W(ns), invW(ns), Tc(ns), coef(32 * (size_t)ns, 0.0), hf(ns), RuInvW(ns);
     double TlowMin = 1e10, ThighMax = 1, TcMin = 1e10, TcMax = 0;
     for (int i = 0; i < ns; i++) {
         if (!(d->W[i] > 0)) return set_err(ctx, FCS_ERR_INVALID, "molecular weight must be positive");
         W[i] = d->W[i];
         invW[i] = 1.0 / d->W[i];
         Tc[i] = d->T_common[i];
-        for (int j = 0; j < 7; j++) {
-            coef[16 * i + j] = d->low_coeffs[7 * i + j];
-            coef[16 * i + 8 + j] = d->high_coeffs[7 * i + j];
+        RuInvW[i] = invW[i] * kRu;
+        for (int set = 0; set < 2; set++) {
+            const double* a = (set ? d->high_coeffs : d->low_coeffs) + 7 * i;
+            double* c = &coef[32 * (size_t)i + 16 * set];
+            for (int j = 0; j < 7; j++) c[j] = a[j];
+            c[7] = a[1] * 0.5;
+            c[8] = a[2] * (1.0 / 6.0);
+            c[9] = a[2] * (1.0 / 3.0);
+            c[10] = a[3] * (1.0 / 12.0);
+            c[11] = a[3] * 0.25;
+            c[12] = a[4] * 0.05;
+            c[13] = a[4] * 0.2;
         }
         TlowMin = std::min(TlowMin, d->T_low[i]);
         ThighMax = std::max(ThighMax, d->T_high[i]);
@@ -346,6 +355,7 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
     ListBlock at;
     at.ev = at.put(lists.ev);
     at.wiw = at.put(wiw);
+    at.RuInvW = at.put(RuInvW);
     at.tbRow = at.put(lists.tbRow);
     at.tbTerm = at.put(lists.tbTerm);
     at.prod = at.put(lists.prod);
@@ -392,6 +402,7 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
     for (size_t q = 0; q + 1 < plogOff.size(); q++)
         for (int k = plogOff[q]; k + 1 < plogOff[q + 1]; k++)
             if (!(plogRow[4 * (size_t)k] <= plogRow[4 * (size_t)k + 4])) M.plogSorted = 0;
+    M.RuInvW = reinterpret_cast<const double*>(ctx->dLists.p + at.RuInvW);
     M.wiw = reinterpret_cast<const double*>(ctx->dLists.p + at.wiw);
     M.prod = at.sums(ctx->dLists.p, at.prod, lists.prod);
     for (int v = 0; v < kJacVariants; v++) {

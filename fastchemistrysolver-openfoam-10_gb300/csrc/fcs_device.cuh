@@ -66,25 +66,29 @@ __device__ __forceinline__ void gsum2(const Grp<G>& g, double& a, double& b, dou
     }
 }
 
+// Bits of |v|, ordered as the magnitudes are, NaN above infinity.
+__device__ __forceinline__ unsigned long long magnitude_bits(double v) {
+    return static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffULL;
+}
+
+// Maximum over the group of magnitude bits (a NaN anywhere wins), as a double.
 template<int G>
-__device__ __forceinline__ double gmax(const Grp<G>& g, double v, double* red) {
-    // NaN-propagating max: a NaN anywhere makes the result NaN
+__device__ __forceinline__ double gmax_bits(const Grp<G>& g, unsigned long long v, double* red) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        const double u = __shfl_xor_sync(0xffffffffu, v, o);
-        v = (u > v || u != u) ? u : v;
+        const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
+        v = u > v ? u : v;
     }
-    if constexpr (G == 32) {
-        return v;
-    } else {
+    if constexpr (G > 32) {
+        unsigned long long* r = reinterpret_cast<unsigned long long*>(red);
         g.sync();
-        if ((g.rank & 31) == 0) red[g.rank >> 5] = v;
+        if ((g.rank & 31) == 0) r[g.rank >> 5] = v;
         g.sync();
-        double s = red[0];
+        v = r[0];
 #pragma unroll
-        for (int w = 1; w < G / 32; w++) s = (red[w] > s || red[w] != red[w]) ? red[w] : s;
-        return s;
+        for (int w = 1; w < G / 32; w++) v = r[w] > v ? r[w] : v;
     }
+    return __longlong_as_double(static_cast<long long>(v));
 }
 
 // Two maxima at once of non-negative values (or NaN, which wins), compared
@@ -136,6 +140,11 @@ __device__ __forceinline__ bool positive(double x) {
 __device__ __forceinline__ bool less_than(double a, double b) {
     const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
     return x < y && ordered(y) && ordered(x & 0x7fffffffffffffffLL);
+}
+
+// max(|a|, |b|) as fmax takes it for b NaN
+__device__ __forceinline__ double larger_magnitude(double a, double b) {
+    return less_than(fabs(a), fabs(b)) ? fabs(b) : fabs(a);
 }
 
 // a <= b for b > 0 or NaN
@@ -273,26 +282,31 @@ __device__ __forceinline__ Slot<MT> make_slot(char* base, const SlotLayout& L, c
 
 __device__ __forceinline__ const double* species_coeffs(const DevMech& M, int i, double Tb) {
     // setPtrCoeffs (ThermoFunctionI.H:1-31)
-    const double* base = M.coef + 16 * i;
+    const double* base = M.coef + 32 * i;
     if (less_than(Tb, M.TcommonMin)) return base;
-    if (less_than(M.TcommonMax, Tb)) return base + 8;
-    return less_than(Tb, __ldg(&M.Tcommon[i])) ? base : base + 8;
+    if (less_than(M.TcommonMax, Tb)) return base + 16;
+    return less_than(Tb, __ldg(&M.Tcommon[i])) ? base : base + 16;
 }
 
-struct Nasa { double a0, a1, a2, a3, a4, a5, a6; };
+// A species' NASA-7 set with the products of the coefficients and the
+// polynomials' constants (formed on the host with the same rounding: eight
+// FP64 instructions per species fewer in each evaluation).
+struct Nasa { double a0, a1, a2, a3, a4, a5, a6, a1h, a2_6, a2_3, a3_12, a3_4, a4_20, a4_5; };
 
 __device__ __forceinline__ Nasa load_nasa(const double* a) {
     Nasa c;
     c.a0 = __ldg(a + 0); c.a1 = __ldg(a + 1); c.a2 = __ldg(a + 2); c.a3 = __ldg(a + 3);
     c.a4 = __ldg(a + 4); c.a5 = __ldg(a + 5); c.a6 = __ldg(a + 6);
+    c.a1h = __ldg(a + 7); c.a2_6 = __ldg(a + 8); c.a2_3 = __ldg(a + 9); c.a3_12 = __ldg(a + 10);
+    c.a3_4 = __ldg(a + 11); c.a4_20 = __ldg(a + 12); c.a4_5 = __ldg(a + 13);
     return c;
 }
 
 // exponent of exp(-G/RT) (ThermoFunctionI.H:539-636)
 __device__ __forceinline__ double gibbs_exponent(const Nasa& a, double T, double invT, double logT) {
-    double v = fma(a.a4 * 0.05, T, a.a3 * (1.0 / 12.0));
-    v = fma(v, T, a.a2 * (1.0 / 6.0));
-    v = fma(v, T, a.a1 * 0.5);
+    double v = fma(a.a4_20, T, a.a3_12);
+    v = fma(v, T, a.a2_6);
+    v = fma(v, T, a.a1h);
     v = fma(v, T, -(a.a5 * invT));
     v = v + a.a6;
     return fma(a.a0, logT - 1.0, v);
@@ -307,9 +321,9 @@ __device__ __forceinline__ double cp_of(const Nasa& a, double T, double RuInvW) 
 }
 
 __device__ __forceinline__ double ha_of(const Nasa& a, double T, double RuInvW) {
-    double v = fma(a.a4, T * 0.2, a.a3 * 0.25);
-    v = fma(v, T, a.a2 * (1.0 / 3.0));
-    v = fma(v, T, a.a1 * 0.5);
+    double v = fma(a.a4, T * 0.2, a.a3_4);
+    v = fma(v, T, a.a2_3);
+    v = fma(v, T, a.a1h);
     v = fma(v, T, a.a0);
     v = fma(v, T, a.a5);
     return RuInvW * v;
@@ -350,9 +364,13 @@ __device__ const double kExp2Table[64] = {
     1.8340080864093424, 1.8539791250833855, 1.8741676341103, 1.8945759815869656,
     1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951};
 
+// Out of range arguments; one copy of the code (inlined, CUDA's exp stood in
+// every rate expression, and the instruction cache is shared by all of them).
+static __device__ __noinline__ double exp_out_of_range(double x) { return exp(x); }
+
 __device__ __forceinline__ double fast_exp(double x) {
     // |x| <= 707 (0x4086180000000000), false for NaN
-    if ((__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x4086180000000000LL) return exp(x);
+    if ((__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x4086180000000000LL) return exp_out_of_range(x);
     const double kInvL = 92.33248261689366;          // 64/ln2
     const double kL1 = 0.010830424696223417;         // head of ln2/64 (36 bits)
     const double kL2 = 2.572804622327669e-14;        // tail
@@ -412,24 +430,6 @@ __device__ __forceinline__ double pressure_factor(const PFactor& pf, int dnu) {
 template<class Rxn>
 __device__ __forceinline__ double inv_kc_clamp(const Rxn& x) {
     return (x.nl > 3 || x.nr > 3) ? kInvKcClampG : kInvKcClamp;
-}
-
-// 1/Kc from per-species exp(-G/RT) and its inverse, no division:
-// 1/Kc = prod_reactants E * prod_products 1/E * (Pstd/(Ru T))^-dnu, with the
-// reference's lower clamp of Kc (ReactionFunctionI.H:17; RFG's for more than
-// 3 species on a side) as an upper clamp.
-__device__ __forceinline__ double inv_equilibrium_kc(const RxnInfo& x, const double* E, const double* Einv,
-                                                     const PFactor& pf) {
-    double v = E[x.sl[0]];
-    // Species loops over a reaction stay rolled: unrolled over the 4 + 8 byte
-    // slots of RxnInfo they raised the integrator's register spills.
-    #pragma unroll 1
-    for (int q = 1; q < x.nl; q++) v *= E[x.sl[q]];
-    #pragma unroll 1
-    for (int q = 0; q < x.nr; q++) v *= Einv[x.sr[q]];
-    if (x.dnu != 0) v *= pressure_factor(pf, x.dnu);
-    const double cl = inv_kc_clamp(x);
-    return less_than(cl, v) ? cl : v;
 }
 
 // ------------------------------------------------------------------------
@@ -744,8 +744,10 @@ __device__ __forceinline__ double product_over(const double* X, const uint8_t* s
     return v;
 }
 
-// 1/Kc = prod_reactants E prod_products 1/E (Pstd/(Ru T))^-dnu, clamped as
-// inv_equilibrium_kc clamps it (ReactionFunctionI.H:17)
+// 1/Kc from per-species E = exp(-G/RT) and its inverse, no division:
+// prod_reactants E prod_products 1/E (Pstd/(Ru T))^-dnu, with the reference's
+// lower clamp of Kc (ReactionFunctionI.H:17; RFG's for more than 3 species on
+// a side) as an upper clamp
 __device__ __forceinline__ double inverse_kc(const RxnEv& x, const double* E, const double* Einv, const PFactor& pf) {
     double v;
     if (three_at_most(x)) {
@@ -924,7 +926,7 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
         const double Ei = fast_exp(gibbs_exponent(a, Tc, t.invT, t.logT));
         s.B[i] = Ei;
         s.Binv[i] = 1.0 / Ei;
-        const double RuInvW = invW * kRu;
+        const double RuInvW = __ldg(&M.RuInvW[i]);
         s.Cp[i] = cp_of(a, Tp, RuInvW);
         s.Ha[i] = ha_of(a, Tp, RuInvW);
     }
@@ -963,73 +965,64 @@ __device__ __noinline__ double tc_eval(const Grp<G>& g, const DevMech& M, const 
                                        double rho, const double* Y) {
     const int ns = M.ns;
     const double Tc = clampT(M, T);
-    const double logT = log(Tc), invT = 1.0 / Tc;
+    const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * T, p);
     double sumc = 0;
     for (int i = g.rank; i < ns; i += G) {
         const double ci = rho * Y[i] / __ldg(&M.W[i]);
         s.C[i] = ci;
         sumc += ci;
         const Nasa a = load_nasa(species_coeffs(M, i, Tc));
-        s.B[i] = fast_exp(gibbs_exponent(a, Tc, invT, logT));
+        const double E = fast_exp(gibbs_exponent(a, Tc, t.invT, t.logT));
+        s.B[i] = E;
+        s.Binv[i] = 1.0 / E;
     }
     sumc = gsum(g, sumc, s.red);
     g.sync();
-    for (int t = g.rank; t < M.nTB; t += G) {
-        const double* e = M.eff + (size_t)t * ns;
-        double m = 0;
-        for (int j = 0; j < ns; j++) m = fma(__ldg(&e[j]), s.C[j], m);
-        s.Mtb[t] = m;
-    }
-    g.sync();
-    const double PByRT = kPstd / (kRu * Tc);
-    const double logP = M.nPlog ? log(p) : 0.0;
+    third_bodies<G, MT>(g, M, s);
+    const double logP = s.red[37];
     double sw = 0, sw2 = 0;
-    // The special block [spBegin, spBegin + nSp) of the packed order (first
-    // non-equilibrium to last fall-off reaction) runs in a loop of its own, so
-    // that the main loop carries neither the fall-off call nor a second
-    // Arrhenius.
-    // Tc.C:578-600: the reverse rate only through Kc; a non-equilibrium
-    // reaction counts with its forward rate alone
-    auto finish = [&](const int r, const RxnInfo& x, const double Kf) {
+    // Tc.C:578-600: the reverse rate only through Kc (1/Kc from the species'
+    // factors, clamped at 1/1.49011611938476e-8 for every kind here); a
+    // non-equilibrium reaction counts with its forward rate alone
+    auto finish = [&](const RxnEv& x, const double Kf) {
         double Kr = 0;
         if (x.rev == 1) {
-            double Kp = 1.0;
+            double v = product_over(s.B, x.sl, x.nl);
             #pragma unroll 1
-            for (int q = 0; q < x.nl; q++) Kp = Kp / s.B[x.sl[q]];
-            #pragma unroll 1
-            for (int q = 0; q < x.nr; q++) Kp = Kp * s.B[x.sr[q]];
-            double Kc = Kp * fast_pow_int(PByRT, x.dnu);
-            Kc = Kc > 1.49011611938476e-8 ? Kc : 1.49011611938476e-8;
-            Kr = Kf / Kc;
+            for (int q = 0; q < x.nr; q++) v *= s.Binv[x.sr[q]];
+            if (x.nr != x.nl) v *= pressure_factor(t.pf, x.nr - x.nl);
+            Kr = Kf * (less_than(kInvKcClampG, v) ? kInvKcClampG : v);
         }
-        double CF = s.C[x.sl[0]];
-        #pragma unroll 1
-        for (int q = 1; q < x.nl; q++) CF *= s.C[x.sl[q]];
-        double CR = s.C[x.sr[0]];
-        #pragma unroll 1
-        for (int q = 1; q < x.nr; q++) CR *= s.C[x.sr[q]];
+        double CF, CR;
+        if (three_at_most(x)) {
+            CF = product3(load3(s.C, x.sl), x.nl);
+            CR = product3(load3(s.C, x.sr), x.nr);
+        } else {
+            CF = product_over(s.C, x.sl, x.nl);
+            CR = product_over(s.C, x.sr, x.nr);
+        }
         const double wf = x.nr * (Kf * CF), wr = x.nl * (Kr * CR);
         sw += wf + wr;
         sw2 = fma(wf, wf, fma(wr, wr, sw2));
     };
-    for (int j = g.rank; j < M.nr - M.nSp; j += G) {
-        const int r = j < M.spBegin ? j : j + M.nSp;
-        const RxnInfo x = load_rx(M.rx + r);
-        double Kf;
-        if (x.kind == FCS_RXN_PLOG) {
+    #pragma unroll 1
+    for (int part = 0; part < 2; part++) {
+        const int end = part ? M.evSpecial : M.evThird;
+        #pragma unroll 1
+        for (int k = (part ? M.evThird : 0) + g.rank; k < end; k += G) {
+            const RxnEv x = load_ev(M.ev + k);
             double dk;
-            Kf = plog_rate(M, x.plog, p, logP, logT, invT, &dk);
-        } else if (x.tind) {
-            Kf = x.A;
-        } else {
-            Kf = x.A * fast_exp(fma(x.beta, logT, -(x.Ta * invT)));
+            double Kf = forward_k(M, x, p, logP, t.logT, t.invT, &dk);
+            if (x.tb >= 0) Kf *= s.Mtb[x.tb];
+            finish(x, Kf);
         }
-        if (x.tb >= 0) Kf *= s.Mtb[x.tb];
-        finish(r, x, Kf);
+        if (part == 0) g.sync();
     }
-    for (int r = M.spBegin + g.rank; r < M.spBegin + M.nSp; r += G) {
-        const RxnInfo x = load_rx(M.rx + r);
-        finish(r, x, special_rates(M, x, s.Mtb, Tc, logT, invT, false).Kf);
+    #pragma unroll 1
+    for (int k = M.evSpecial + g.rank; k < M.nr; k += G) {
+        const RxnEv x = load_ev(M.ev + k);
+        const RxnInfo xi = load_rx(M.rx + x.r);
+        finish(x, special_rates(M, xi, s.Mtb, Tc, t.logT, t.invT, false).Kf);
     }
     gsum2(g, sw, sw2, s.red);
     return sw2 == 0 ? 1e300 : sw / sw2 * sumc;
@@ -1161,8 +1154,8 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
         s.B[i] = Ei;
         s.Binv[i] = 1.0 / Ei;
         s.dBdT[i] = fma(fma(a.a5, invT, a.a0), invT,
-                        fma(fma(fma(a.a4 * 0.2, Tc, a.a3 * 0.25), Tc, a.a2 * (1.0 / 3.0)), Tc, a.a1 * 0.5));
-        const double RuInvW = invW * kRu;
+                        fma(fma(fma(a.a4_5, Tc, a.a3_4), Tc, a.a2_3), Tc, a.a1h));
+        const double RuInvW = __ldg(&M.RuInvW[i]);
         s.Cp[i] = cp_of(a, Tc, RuInvW);
         s.dCpdT[i] = RuInvW * fma(Tc, fma(Tc, fma(Tc, 4 * a.a4, 3 * a.a3), 2 * a.a2), a.a1);
         s.Ha[i] = ha_of(a, Tc, RuInvW);
@@ -1284,35 +1277,55 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     // share out the elements of the rows that have terms (one more product a
     // term, 53 species: 24,000 cycles by columns at any group size, 15,000
     // with 128 threads, 9,000 with 256).
+    // (each form in a loop of its own: chosen per term, both would be issued)
     if constexpr (G <= 64) {
         for (int j = g.rank; j < ns; j += G) {
             int last = -1;
             double e0 = 0, wd = 0;
-            for (int e = 0; e < M.nTbInc; e++) {
-                const int v = __ldg(&M.tbInc[e]);
-                const int i = v >> 16, tb = (v >> 1) & 0x7fff;
+            auto next_row = [&](int tb) {
                 if (tb != last) {
                     e0 = __ldg(&M.eff[(size_t)tb * ns + j]);
                     wd = __dmul_rn(e0, s.tbF[tb]);
                     last = tb;
                 }
-                MT& c = J[i * ld + j];
-                const double w = v & 1 ? s.tbF[tb] : -s.tbF[tb], d = v & 1 ? wd : -wd;
-                c = s.rw == 1 ? MT(fma(e0, w, double(c))) : MT(double(c) + d);
+            };
+            if (s.rw == 1) {
+                #pragma unroll 1
+                for (int e = 0; e < M.nTbInc; e++) {
+                    const int v = __ldg(&M.tbInc[e]), tb = (v >> 1) & 0x7fff;
+                    next_row(tb);
+                    const double w = s.tbF[tb];
+                    MT& c = J[(v >> 16) * ld + j];
+                    c = MT(fma(e0, __longlong_as_double(__double_as_longlong(w) ^ ((long long)(~v & 1) << 63)), double(c)));
+                }
+            } else {
+                #pragma unroll 1
+                for (int e = 0; e < M.nTbInc; e++) {
+                    const int v = __ldg(&M.tbInc[e]);
+                    next_row((v >> 1) & 0x7fff);
+                    J[(v >> 16) * ld + j] += MT(__longlong_as_double(__double_as_longlong(wd) ^ ((long long)(~v & 1) << 63)));
+                }
             }
         }
     } else {
         int r = g.rank / ns, j = g.rank - r * ns;
         const int dr = G / ns, dj = G - dr * ns;
+        const bool once = s.rw == 1;
         while (r < M.nTbRow) {
             const int i = __ldg(M.tbRow + 2 * r), e0 = __ldg(M.tbRow + 2 * r + 1), e1 = __ldg(M.tbRow + 2 * r + 3);
             MT& o = J[i * ld + j];
             double v = double(o);
-            #pragma unroll 2
-            for (int e = e0; e < e1; e++) {
-                const int c = __ldg(M.tbTerm + e), tb = c >> 1;
-                const double e0 = __ldg(&M.eff[(size_t)tb * ns + j]), w = c & 1 ? s.tbF[tb] : -s.tbF[tb];
-                v = s.rw == 1 ? fma(e0, w, v) : v + __dmul_rn(e0, w);
+            if (once) {
+                for (int e = e0; e < e1; e++) {
+                    const int c = __ldg(M.tbTerm + e), tb = c >> 1;
+                    v = fma(__ldg(&M.eff[(size_t)tb * ns + j]), c & 1 ? s.tbF[tb] : -s.tbF[tb], v);
+                }
+            } else {
+                #pragma unroll 2
+                for (int e = e0; e < e1; e++) {
+                    const int c = __ldg(M.tbTerm + e), tb = c >> 1;
+                    v += __dmul_rn(__ldg(&M.eff[(size_t)tb * ns + j]), c & 1 ? s.tbF[tb] : -s.tbF[tb]);
+                }
             }
             o = MT(v);
             r += dr;

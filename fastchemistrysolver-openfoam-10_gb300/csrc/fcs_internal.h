@@ -2,8 +2,9 @@
 // kernels of libfcs_cuda.so.
 //
 // Mechanism image in HBM (built once by pack_mechanism, read through L1):
-//   * species arrays W, invW, Tcommon and the NASA-7 sets, 16 doubles per
-//     species (low[0..6], pad, high[0..6], pad): one 128-byte line each;
+//   * species arrays W, invW, Ru/W, Tcommon and the NASA-7 sets, low then high,
+//     16 doubles each: the coefficients, then their products with the
+//     polynomials' constants;
 //   * one 64-byte RxnInfo per reaction, in the reference's type-block order
 //     (OptReaction.C:448-1175): constant Arrhenius, other Arrhenius,
 //     third-body, PLOG;
@@ -90,8 +91,9 @@ struct DevMech {
     double TlowMin, ThighMax, TcommonMin, TcommonMax;
     const double* W;        // [ns]
     const double* invW;     // [ns]
+    const double* RuInvW;   // [ns]
     const double* Tcommon;  // [ns]
-    const double* coef;     // [ns][16]
+    const double* coef;     // [ns][32]
     const RxnInfo* rx;      // [nr]
     const double* eff;      // [nTB][ns]
     const int* plogOff;     // [nPlog+1]

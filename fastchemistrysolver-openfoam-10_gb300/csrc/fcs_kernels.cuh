@@ -261,15 +261,15 @@ __device__ __noinline__ double rodas34_attempt(const Grp<G>& g, const DevMech& M
     }
     g.sync();
     if (!stage_solve<G, MT>(g, M, s, cdiag, err, tmp)) return -1.0;
-    double me = 0;
+    unsigned long long me = 0;
     for (int i = g.rank; i < n; i += G) {
         const double yt = y0[i] + dy[i] + err[i];
         yTemp[i] = yt;
-        const double tol = o.absTol + o.relTol * fmax(fabs(y0[i]), fabs(yt));
+        const double tol = o.absTol + o.relTol * larger_magnitude(y0[i], yt);
         const double e = fabs(err[i]) / tol;
-        me = (e > me || e != e) ? e : me;
+        me = max(me, magnitude_bits(e));
     }
-    return gmax(g, me, s.red);
+    return gmax_bits(g, me, s.red);
 }
 
 // OptRosenbrock34::Rosenbrock34Solve (OptRosenbrock34.C:281-678), .H:127-158
@@ -321,17 +321,17 @@ __device__ __noinline__ double ros34_attempt(const Grp<G>& g, const DevMech& M, 
     }
     g.sync();
     if (!stage_solve<G, MT>(g, M, s, cdiag, k4, tmp)) return -1.0;
-    double me = 0;
+    unsigned long long me = 0;
     for (int i = g.rank; i < n; i += G) {
         const double yt = fma(b4, k4[i], fma(b3, k3[i], fma(b2, k2[i], fma(b1, k1[i], y0[i]))));
         yTemp[i] = yt;
         const double e = fma(e4, k4[i], fma(e2, k2[i], e1 * k1[i]));
         err[i] = e;
-        const double tol = o.absTol + o.relTol * fmax(fabs(y0[i]), fabs(yt));
+        const double tol = o.absTol + o.relTol * larger_magnitude(y0[i], yt);
         const double r = fabs(e) / tol;
-        me = (r > me || r != r) ? r : me;
+        me = max(me, magnitude_bits(r));
     }
-    return gmax(g, me, s.red);
+    return gmax_bits(g, me, s.red);
 }
 
 // OptRodas23::Rodas23Solve (OptRodas23.C:202-315), constants OptRodas23.H:113-126:
@@ -376,15 +376,15 @@ __device__ __noinline__ double rodas23_attempt(const Grp<G>& g, const DevMech& M
     for (int i = g.rank; i < n; i += G) err[i] = dydx[i] + fma(c43, k3[i], fma(c42, k2[i], c41 * k1[i])) / dx;
     g.sync();
     if (!stage_solve<G, MT>(g, M, s, cdiag, err, tmp)) return -1.0;
-    double me = 0;
+    unsigned long long me = 0;
     for (int i = g.rank; i < n; i += G) {
         const double yt = y0[i] + dy[i] + err[i];
         yTemp[i] = yt;
-        const double tol = o.absTol + o.relTol * fmax(fabs(y0[i]), fabs(yt));
+        const double tol = o.absTol + o.relTol * larger_magnitude(y0[i], yt);
         const double e = fabs(err[i]) / tol;
-        me = (e > me || e != e) ? e : me;
+        me = max(me, magnitude_bits(e));
     }
-    return gmax(g, me, s.red);
+    return gmax_bits(g, me, s.red);
 }
 
 // OptRosenbrock23::Rosenbrock23Solve (OptRosenbrock23.C:208-298), constants
@@ -422,17 +422,17 @@ __device__ __noinline__ double ros23_attempt(const Grp<G>& g, const DevMech& M, 
     for (int i = g.rank; i < n; i += G) k3[i] = fma(dxd3, dfdx[i], dydx[i]) + fma(c32, k2[i], c31 * k1[i]) / dx;
     g.sync();
     if (!stage_solve<G, MT>(g, M, s, cdiag, k3, tmp)) return -1.0;
-    double me = 0;
+    unsigned long long me = 0;
     for (int i = g.rank; i < n; i += G) {
         const double yt = fma(b3, k3[i], fma(b2, k2[i], fma(b1, k1[i], y0[i])));
         yTemp[i] = yt;
         const double e = fma(e3, k3[i], fma(e2, k2[i], e1 * k1[i]));
         err[i] = e;
-        const double tol = o.absTol + o.relTol * fmax(fabs(y0[i]), fabs(yt));
+        const double tol = o.absTol + o.relTol * larger_magnitude(y0[i], yt);
         const double r = fabs(e) / tol;
-        me = (r > me || r != r) ? r : me;
+        me = max(me, magnitude_bits(r));
     }
-    return gmax(g, me, s.red);
+    return gmax_bits(g, me, s.red);
 }
 
 template<int G, class MT>
@@ -445,6 +445,20 @@ __device__ __forceinline__ double attempt_of(const Grp<G>& g, const DevMech& M, 
         case FCS_SOLVER_ROSENBROCK23: return ros23_attempt<G, MT>(g, M, o, s, sd, p, dx, invdx, cc);
         default: return rodas34_attempt<G, MT>(g, M, o, s, sd, p, dx, invdx, cc);
     }
+}
+
+// SAFE Err^-alpha of the step controller for the whole group: pow is 87 FP64
+// instructions, issued by one warp.
+template<int G>
+__device__ __forceinline__ double step_factor(const Grp<G>& g, double* red, double Err, double alpha) {
+    double v = 0;
+    if (g.rank < 32) v = 0.9 * pow(Err, -alpha);
+    if constexpr (G > 32) {
+        if (g.rank == 0) red[38] = v;
+        g.sync();
+        v = red[38];
+    }
+    return v;
 }
 
 // ODESolve + adaptiveSolve (OptRodas34.C:123-289, OptRosenbrock34.C:127-279,
@@ -488,7 +502,7 @@ __device__ int rosenbrock_integrate(const Grp<G>& g, const DevMech& M, const KOp
         int rejects = 0;
         while (Err > 1) {
             if (++rejects > o.maxRejects) return FCS_CELL_DT_UNDERFLOW;
-            const double scale = fmax(SAFE * pow(Err, -ALPHA_DEC), MIN_SCALE);
+            const double scale = fmax(step_factor<G>(g, s.red, Err, ALPHA_DEC), MIN_SCALE);
             dx *= scale;
             invdx = 1.0 / dx;
             Err = rosenbrock_attempt<G, MT>(g, M, o, s, sd, p, dx, invdx, cc);
@@ -499,7 +513,7 @@ __device__ int rosenbrock_integrate(const Grp<G>& g, const DevMech& M, const KOp
         x += dx;
         for (int i = g.rank; i < n; i += G) y0[i] = yTemp[i];
         g.sync();
-        dxTry = (Err > ratio) ? fmin(fmax(SAFE * pow(Err, -ALPHA_INC), MIN_SCALE), MAX_SCALE) * dx
+        dxTry = (Err > ratio) ? fmin(fmax(step_factor<G>(g, s.red, Err, ALPHA_INC), MIN_SCALE), MAX_SCALE) * dx
                               : safeMaxScale * dx;
         if ((x - xEnd) * (xEnd - 0.0) >= 0) {
             if (nStep > 0 && last) dxTry = dxTry0;

@@ -116,7 +116,7 @@ __device__ __forceinline__ void lane_map(int n, LA<double> out, F f, In... in) {
 // ------------------------------------------------------------------------
 // rates
 
-// 1/Kc with the reference's clamp (inv_equilibrium_kc over per-lane arrays)
+// 1/Kc with the reference's clamp (inverse_kc over per-lane arrays)
 __device__ __forceinline__ double lane_inv_kc(const RxnInfo& x, const LA<double>& E, const LA<double>& Einv,
                                               const PFactor& pf) {
     double v = E[x.sl[0]];
@@ -263,7 +263,7 @@ __device__ __noinline__ void lane_rhs(const DevMech& M, const LaneSlot& s, doubl
             const double Ei = fast_exp(gibbs_exponent(a, Tc, invT, logT));
             s.B[k] = Ei;
             s.Binv[k] = 1.0 / Ei;
-            const double RuInvW = invW * kRu;
+            const double RuInvW = __ldg(&M.RuInvW[k]);
             s.Cp[k] = cp_of(a, Tp, RuInvW);
             s.Ha[k] = ha_of(a, Tp, RuInvW);
         }
@@ -399,8 +399,8 @@ __device__ __noinline__ void lane_jac(const DevMech& M, const LaneSlot& s, doubl
         s.B[i] = Ei;
         s.Binv[i] = 1.0 / Ei;
         s.dBdT[i] = fma(fma(a.a5, invT, a.a0), invT,
-                        fma(fma(fma(a.a4 * 0.2, Tc, a.a3 * 0.25), Tc, a.a2 * (1.0 / 3.0)), Tc, a.a1 * 0.5));
-        const double RuInvW = invW * kRu;
+                        fma(fma(fma(a.a4_5, Tc, a.a3_4), Tc, a.a2_3), Tc, a.a1h));
+        const double RuInvW = __ldg(&M.RuInvW[i]);
         const double cp = cp_of(a, Tc, RuInvW);
         const double dcp = RuInvW * fma(Tc, fma(Tc, fma(Tc, 4 * a.a4, 3 * a.a3), 2 * a.a2), a.a1);
         s.Cp[i] = cp;

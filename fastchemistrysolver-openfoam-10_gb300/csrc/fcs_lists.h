@@ -81,7 +81,7 @@ struct ListBlock {
     struct Sums { size_t elem, off, con; };
     struct Jac { size_t ev, chunk; Sums sums; };
     std::vector<char> bytes;
-    size_t ev = 0, wiw = 0, tbRow = 0, tbTerm = 0;
+    size_t ev = 0, wiw = 0, RuInvW = 0, tbRow = 0, tbTerm = 0;
     Sums prod{};
     Jac jac[kJacVariants]{};
     template<class T>

@@ -14,8 +14,6 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
-#include <numeric>
-#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -26,6 +24,21 @@ namespace fcs {
 
 constexpr int kTroe = FCS_RXN_TROE_FALLOFF, kSri = FCS_RXN_SRI_FALLOFF;
 
+// Terms of sums, one after another: sum k is val[begin[k] .. begin[k + 1]).
+struct Terms {
+    std::vector<uint32_t> target, val;
+    std::vector<int> begin;
+    void start(uint32_t t) {
+        target.push_back(t);
+        begin.push_back((int)val.size());
+    }
+    void clear() {
+        target.clear();
+        val.clear();
+        begin.clear();
+    }
+};
+
 // Sums, 32 to a group: elem[32 g + lane] = target << 16 | terms, the group's
 // terms from con[off[g]] on, term k of a lane at off[g] + 32 k + lane, each
 // value index << 1 | (1: added, 0: subtracted).
@@ -35,21 +48,28 @@ struct HostSums {
     std::vector<uint32_t> con;
     int groups() const { return (int)off.size(); }
 
-    // targets[t], lists[t]: appended, longest first
-    void append(const std::vector<uint32_t>& targets, const std::vector<std::vector<uint32_t>>& lists) {
-        std::vector<int> order(targets.size());
-        std::iota(order.begin(), order.end(), 0);
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return lists[a].size() > lists[b].size(); });
-        for (size_t g = 0; g < order.size(); g += 32) {
-            const size_t len = lists[order[g]].size();
-            off.push_back((int)con.size());
+    // t's sums appended, longest first
+    void append(const Terms& t) {
+        const int n = (int)t.target.size();
+        auto begin = [&](int k) { return k < n ? t.begin[k] : (int)t.val.size(); };
+        auto length = [&](int k) { return begin(k + 1) - begin(k); };
+        int longest = 0;
+        for (int k = 0; k < n; k++) longest = std::max(longest, length(k));
+        std::vector<int> at(longest + 2, 0), order(n);
+        for (int k = 0; k < n; k++) at[longest - length(k) + 1]++;
+        for (int l = 0; l <= longest; l++) at[l + 1] += at[l];
+        for (int k = 0; k < n; k++) order[at[longest - length(k)]++] = k;
+        for (int g = 0; g < n; g += 32) {
+            const int len = length(order[g]);
             const size_t base = con.size();
-            con.resize(base + 32 * len, 0);
-            for (size_t l = 0; l < 32; l++) {
-                if (g + l >= order.size()) { elem.push_back(kNoSum); continue; }
-                const auto& v = lists[order[g + l]];
-                elem.push_back(targets[order[g + l]] << 16 | (uint32_t)v.size());
-                for (size_t k = 0; k < v.size(); k++) con[base + 32 * k + l] = v[k];
+            off.push_back((int)base);
+            con.resize(base + 32 * (size_t)len, 0);
+            for (int l = 0; l < 32; l++) {
+                if (g + l >= n) { elem.push_back(kNoSum); continue; }
+                const int k = order[g + l], m = length(k);
+                elem.push_back(t.target[k] << 16 | (uint32_t)m);
+                const uint32_t* v = t.val.data() + begin(k);
+                for (int q = 0; q < m; q++) con[base + 32 * (size_t)q + l] = v[q];
             }
         }
     }
@@ -130,10 +150,23 @@ inline int falloff_class(const RxnEv& e) { return e.kind == kTroe ? 1 : e.kind =
 
 // Reactions that take the same path next to each other, the dearest kind first.
 inline void sort_ev(std::vector<RxnEv>& v) {
-    auto key = [](const RxnEv& e) {
-        return std::make_tuple(falloff_class(e), e.plog < 0, e.tind, e.tb >= 0, e.rev, e.nl, e.nr, e.r);
-    };
-    std::sort(v.begin(), v.end(), [&](const RxnEv& x, const RxnEv& y) { return key(x) < key(y); });
+    std::vector<std::pair<uint64_t, int>> key(v.size());
+    for (size_t k = 0; k < v.size(); k++) {
+        const RxnEv& e = v[k];
+        uint64_t w = falloff_class(e);
+        w = w << 1 | (e.plog < 0);
+        w = w << 1 | (e.tind != 0);
+        w = w << 1 | (e.tb >= 0);
+        w = w << 4 | uint64_t(e.rev);
+        w = w << 8 | uint64_t(e.nl);
+        w = w << 8 | uint64_t(e.nr);
+        key[k] = {w << 32 | uint32_t(e.r), (int)k};
+    }
+    std::sort(key.begin(), key.end());
+    std::vector<RxnEv> sorted;
+    sorted.reserve(v.size());
+    for (const auto& k : key) sorted.push_back(v[k.second]);
+    v.swap(sorted);
 }
 
 // First position of fall-off class c or above in v
@@ -176,14 +209,21 @@ inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, con
         H.tbRow.push_back((int)H.tbTerm.size());
     }
     {
-        std::vector<uint32_t> tgt;
-        std::vector<std::vector<uint32_t>> terms;
+        Terms t;
         for (int i = 0; i < ns; i++) {
-            tgt.push_back(i);
-            terms.emplace_back(inc[i].begin(), inc[i].end());
+            t.start(i);
+            t.val.insert(t.val.end(), inc[i].begin(), inc[i].end());
         }
-        H.prod.append(tgt, terms);
+        H.prod.append(t);
     }
+    // scratch of a column: its terms in the order they are added, then by row
+    Terms t;
+    std::vector<uint32_t> w, tc;
+    struct Term { int row; uint32_t val; };
+    size_t longest = 0;
+    for (const auto& l : inc) longest = std::max(longest, l.size());
+    std::vector<Term> col(longest * (kMaxL + kMaxR));
+    std::vector<int> rows, count(ns, 0), where(ns, 0);
     for (int v = 0; v < kJacVariants; v++) {
         HostChunks& J = H.jac[v];
         J.size = kJacChunk[v];
@@ -207,11 +247,11 @@ inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, con
             J.values = std::max(J.values, n);
             for (RxnEv& e : main) e.ent = ent[e.r - c0];
             J.ev.insert(J.ev.end(), main.begin(), main.end());
-            std::vector<uint32_t> tgt;
-            std::vector<std::vector<uint32_t>> terms;
+            t.clear();
             for (int j = 0; j < ns; j++) {
-                std::vector<uint32_t> w, tc;
-                std::vector<std::pair<int, uint32_t>> col;  // (row, term) of column j
+                w.clear();
+                tc.clear();
+                Term* end = col.data();
                 int seen[2] = {-1, -1}, occ[2] = {0, 0};  // occurrence of j on the side so far
                 for (; at[j] < inc[j].size() && (inc[j][at[j]] >> 1) < c1; at[j]++) {
                     const int r = inc[j][at[j]] >> 1, side = inc[j][at[j]] & 1, l = r - c0;
@@ -226,26 +266,28 @@ inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, con
                         if (s[slot] == j && k-- == 0) break;
                     if (side && !x.rev) continue;
                     const uint32_t val = uint32_t(ent[l] + (side ? x.nl : 0) + slot);
-                    for (int q = 0; q < x.nl; q++) col.emplace_back(x.sl[q], val << 1);
-                    for (int q = 0; q < x.nr; q++) col.emplace_back(x.sr[q], val << 1 | 1);
+                    for (int q = 0; q < x.nl; q++) *end++ = Term{x.sl[q], val << 1};
+                    for (int q = 0; q < x.nr; q++) *end++ = Term{x.sr[q], val << 1 | 1};
                 }
                 if (!w.empty()) {
-                    tgt.push_back(uint32_t(ns) << 8 | uint32_t(j));
-                    terms.push_back(w);
-                    tgt.push_back(uint32_t(j) << 8 | uint32_t(ns));
-                    terms.push_back(tc);
+                    t.start(uint32_t(ns) << 8 | uint32_t(j));
+                    t.val.insert(t.val.end(), w.begin(), w.end());
+                    t.start(uint32_t(j) << 8 | uint32_t(ns));
+                    t.val.insert(t.val.end(), tc.begin(), tc.end());
                 }
-                std::stable_sort(col.begin(), col.end(),
-                                 [](const auto& a, const auto& b) { return a.first < b.first; });
-                for (size_t a = 0; a < col.size(); a++) {
-                    if (a == 0 || col[a].first != col[a - 1].first) {
-                        tgt.push_back(uint32_t(col[a].first) << 8 | uint32_t(j));
-                        terms.emplace_back();
-                    }
-                    terms.back().push_back(col[a].second);
+                rows.clear();
+                for (const Term* c = col.data(); c < end; c++)
+                    if (count[c->row]++ == 0) rows.push_back(c->row);
+                std::sort(rows.begin(), rows.end());
+                for (const int i : rows) {
+                    t.start(uint32_t(i) << 8 | uint32_t(j));
+                    where[i] = (int)t.val.size();
+                    t.val.resize(t.val.size() + count[i]);
+                    count[i] = 0;
                 }
+                for (const Term* c = col.data(); c < end; c++) t.val[where[c->row]++] = c->val;
             }
-            J.sums.append(tgt, terms);
+            J.sums.append(t);
             ch.groupEnd = J.sums.groups();
             J.chunk.push_back(ch);
         }

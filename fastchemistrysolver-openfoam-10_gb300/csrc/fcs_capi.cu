@@ -835,11 +835,28 @@ static fcs_status eval_impl(fcs_ctx* ctx, int64_t nc, const double* p, const dou
         if (J) { CK(ctx->bJ.ensure((size_t)n * n * nc)); dJ = ctx->bJ.p; }
         if (Qdot) { CK(ctx->bQ.ensure(nc)); dQ = ctx->bQ.p; }
     }
-    // the per-cell evaluations run on cell groups (the lane mapping is the integrator's)
+    // The per-cell evaluations run on cell groups (the lane mapping is the
+    // integrator's), the same for any number of cells.  rates() and tc()
+    // together, us, 300 | 20,000 cells: 53 species 64 threads 77 | 1,620 (32: 107
+    // | 1,620, 128: 77 | 1,807); 111 species 128 threads 97 | 3,097 (64: 117 |
+    // 2,975, 256: 105 | 4,128); 200 species 128 threads 152 | 6,045 (64: 195 |
+    // 5,894, 256: 153 | 6,977).
+    const int wide = ctx->M.n <= 128 ? 256 : 512;  // with a matrix
     const int group = ctx->opt.mapping > FCS_MAPPING_LANE ? ctx->opt.mapping
-                                                          : ctx->M.n <= 64 ? 64 : ctx->M.n <= 128 ? 256 : 512;
+                      : ctx->M.n <= 64                    ? 64
+                      : mode == 1                         ? wide
+                                                          : 128;
     Shape sh;
-    if (!make_shape(ctx, group, false, nc, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape");
+    if (mode == 1) {
+        if (!make_shape(ctx, group, false, nc, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape");
+    } else {
+        if (ctx->M.n > 256) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape");
+        sh.L = make_source_layout(ns, ctx->M.nr, ctx->M.nTB);
+        sh.L.rw = sum_threads(ctx, group, false, nc);
+        sh.global = (size_t)sh.L.bytes > ctx->maxSmemPerBlock;
+        sh.lc.group = group;
+        sh.lc.block = group == 32 ? 128 : group;
+    }
     const int gpb = sh.lc.block / sh.lc.group;
     sh.lc.grid = (int)((nc + gpb - 1) / gpb);
     char* gws = nullptr;
@@ -848,8 +865,11 @@ static fcs_status eval_impl(fcs_ctx* ctx, int64_t nc, const double* p, const dou
             return set_err(ctx, FCS_ERR_NOMEM, "workspace allocation failed");
         gws = ctx->gws.p;
     }
-    const KOpts ko = kopts(ctx->opt);
-    CK(launch_eval(sh.lc, sh.mixed, ctx->M, ko, sh.L, nc, dp, dT, drho, dY, dout, dJ, dQ, mode, gws, st));
+    if (mode == 1)
+        CK(launch_jacobian(sh.lc, ctx->M, kopts(ctx->opt), sh.L, nc, dp, dT, dY, dout, dJ, gws, st));
+    else
+        CK(launch_sources(sh.lc, ctx->M, sh.L, nc, dp, dT, drho, dY, dout, dQ,
+                          mode == 0 ? SRC_RHS : mode == 2 ? SRC_RATES : SRC_TC, gws, st));
     if (!dev) {
         CK(cudaMemcpyAsync(out, dout, nout * 8, cudaMemcpyDeviceToHost, st));
         if (J) CK(cudaMemcpyAsync(J, dJ, (size_t)n * n * nc * 8, cudaMemcpyDeviceToHost, st));

@@ -222,6 +222,23 @@ __host__ __device__ inline SlotLayout make_layout(int ns, int nr, int nTB, bool 
     return L;
 }
 
+// What a cell's rates, right-hand side or time scale need: no matrix, two
+// vectors, five species arrays, the net rates, M of the third bodies and the
+// reduction scratch.  6 KB instead of 34 for 53 species, so that registers and
+// not shared memory limit the cells of an SM.  The other offsets are not used.
+inline SlotLayout make_source_layout(int ns, int nr, int nTB) {
+    SlotLayout L{};
+    const int n = ns + 1;
+    int o = 0;
+    L.offVec = o;   o = align16(o + 2 * n * 8);
+    L.offSp = o;    o = align16(o + 5 * ns * 8);
+    L.offRx = o;    o = align16(o + (nr > 0 ? nr : 1) * 8);
+    L.offTb = o;    o = align16(o + (nTB > 0 ? nTB : 1) * 8);
+    L.offRed = o;   o = align16(o + 48 * 8);
+    L.bytes = o;
+    return L;
+}
+
 template<class MT>
 struct Slot {
     int ld, n, ns;

@@ -101,16 +101,15 @@ cudaError_t launch_integrate(const LaunchCfg& lc, bool mixed, const DevMech& M, 
     }
 }
 
-cudaError_t launch_eval(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,
-                        const SlotLayout& L, long long nc, const double* p, const double* T,
-                        const double* rho, const double* Y, double* out, double* J, double* Qdot,
-                        int mode, char* gws, cudaStream_t st) {
+cudaError_t launch_jacobian(const LaunchCfg& lc, const DevMech& M, const KOpts& o, const SlotLayout& L,
+                            long long nc, const double* p, const double* T, const double* Y, double* out,
+                            double* J, char* gws, cudaStream_t st) {
     switch (lc.group) {
-        case 32: return launch_eval_g<32>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
-        case 64: return launch_eval_g<64>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
-        case 128: return launch_eval_g<128>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
-        case 256: return launch_eval_g<256>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
-        case 512: return launch_eval_g<512>(lc, mixed, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
+        case 32: return launch_jacobian_g<32>(lc, M, o, L, nc, p, T, Y, out, J, gws, st);
+        case 64: return launch_jacobian_g<64>(lc, M, o, L, nc, p, T, Y, out, J, gws, st);
+        case 128: return launch_jacobian_g<128>(lc, M, o, L, nc, p, T, Y, out, J, gws, st);
+        case 256: return launch_jacobian_g<256>(lc, M, o, L, nc, p, T, Y, out, J, gws, st);
+        case 512: return launch_jacobian_g<512>(lc, M, o, L, nc, p, T, Y, out, J, gws, st);
         default: return cudaErrorInvalidValue;
     }
 }

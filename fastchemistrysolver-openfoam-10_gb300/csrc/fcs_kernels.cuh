@@ -934,13 +934,12 @@ integrate_kernel(const DevMech M, const KOpts o, const SlotLayout L, CellIO io, 
     }
 }
 
-// f(y) per cell: one group per cell, Y read-only (copied into the slot)
-template<int G, class MT>
+// J and f(y) per cell: one group per cell, Y read-only (copied into the slot)
+template<int G>
 __global__ void __launch_bounds__(G == 32 ? 256 : G)
-eval_kernel(const DevMech M, const KOpts o, const SlotLayout L, long long nc, const double* __restrict__ p,
-            const double* __restrict__ T, const double* __restrict__ rho, const double* __restrict__ Y,
-            double* __restrict__ out,
-            double* __restrict__ Jout, double* __restrict__ Qdot, int mode, char* __restrict__ gws) {
+jacobian_kernel(const DevMech M, const KOpts o, const SlotLayout L, long long nc, const double* __restrict__ p,
+                const double* __restrict__ T, const double* __restrict__ Y, double* __restrict__ out,
+                double* __restrict__ Jout, char* __restrict__ gws) {
     extern __shared__ __align__(16) char smem[];
     Grp<G> g;
     g.rank = threadIdx.x % G;
@@ -949,7 +948,7 @@ eval_kernel(const DevMech M, const KOpts o, const SlotLayout L, long long nc, co
     const long long c = (long long)blockIdx.x * groupsPerBlock + gidInBlock;
     char* base = gws ? gws + (size_t)(blockIdx.x * groupsPerBlock + gidInBlock) * L.bytes
                      : smem + (size_t)gidInBlock * L.bytes;
-    const Slot<MT> s = make_slot<MT>(base, L, M);
+    const Slot<double> s = make_slot<double>(base, L, M);
     if (c >= nc) return;  // whole group exits together
     const int ns = M.ns, n = M.n;
     double* y = s.v(0);
@@ -960,26 +959,13 @@ eval_kernel(const DevMech M, const KOpts o, const SlotLayout L, long long nc, co
         s.red[37] = M.nPlog ? log(p[c]) : 0.0;
     }
     g.sync();
-    if (mode == 0) {
-        rhs_eval<G, MT>(g, M, s, p[c], y, f, 1);
-    } else if (mode == 1) {
-        const Slot<double> sd = make_slot<double>(base, L, M);
-        jac_eval<G, double>(g, M, sd, p[c], y, f, sd.J, o.jacobian, false, 0.0);
-        for (int idx = g.rank; idx < n * n; idx += G) {
-            const int i = idx / n, j = idx - i * n;
-            Jout[(size_t)c * n * n + idx] = sd.J[(size_t)i * s.ld + j];
-        }
-    } else if (mode == 2) {
-        const double qd = rates_eval<G, MT>(g, M, s, p[c], T[c], rho[c], y, f);
-        if (Qdot && g.rank == 0) Qdot[c] = qd;
-    } else {
-        const double tc = tc_eval<G, MT>(g, M, s, p[c], T[c], rho[c], y);
-        if (g.rank == 0) out[c] = tc;
-        return;
+    jac_eval<G, double>(g, M, s, p[c], y, f, s.J, o.jacobian, false, 0.0);
+    for (int idx = g.rank; idx < n * n; idx += G) {
+        const int i = idx / n, j = idx - i * n;
+        Jout[(size_t)c * n * n + idx] = s.J[(size_t)i * s.ld + j];
     }
     g.sync();
-    const int nout = mode == 2 ? ns : n;
-    for (int i = g.rank; i < nout; i += G) out[(size_t)i * nc + c] = f[i];
+    for (int i = g.rank; i < n; i += G) out[(size_t)i * nc + c] = f[i];
 }
 
 // ------------------------------------------------------------------------
@@ -1011,18 +997,17 @@ inline cudaError_t launch_integrate_t(const LaunchCfg& lc, const DevMech& M, con
     return cudaGetLastError();
 }
 
-template<int G, class MT>
-inline cudaError_t launch_eval_t(const LaunchCfg& lc, const DevMech& M, const KOpts& o, const SlotLayout& L,
-                                 long long nc, const double* p, const double* T, const double* rho,
-                                 const double* Y, double* out, double* J, double* Qdot, int mode, char* gws,
-                                 cudaStream_t st) {
-    auto k = eval_kernel<G, MT>;
+template<int G>
+inline cudaError_t launch_jacobian_t(const LaunchCfg& lc, const DevMech& M, const KOpts& o, const SlotLayout& L,
+                                     long long nc, const double* p, const double* T, const double* Y, double* out,
+                                     double* J, char* gws, cudaStream_t st) {
+    auto k = jacobian_kernel<G>;
     const size_t sm = gws ? 0 : (size_t)L.bytes * (lc.block / G);
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
     }
-    k<<<lc.grid, lc.block, sm, st>>>(M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws);
+    k<<<lc.grid, lc.block, sm, st>>>(M, o, L, nc, p, T, Y, out, J, gws);
     return cudaGetLastError();
 }
 

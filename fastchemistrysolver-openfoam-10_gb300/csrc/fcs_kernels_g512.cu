@@ -13,12 +13,10 @@ cudaError_t launch_integrate_g<512>(const LaunchCfg& lc, bool mixed, const DevMe
 }
 
 template<>
-cudaError_t launch_eval_g<512>(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,
-                             const SlotLayout& L, long long nc, const double* p, const double* T,
-                             const double* rho, const double* Y, double* out, double* J, double* Qdot,
-                             int mode, char* gws, cudaStream_t st) {
-    return mixed ? launch_eval_t<512, float>(lc, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st)
-                 : launch_eval_t<512, double>(lc, M, o, L, nc, p, T, rho, Y, out, J, Qdot, mode, gws, st);
+cudaError_t launch_jacobian_g<512>(const LaunchCfg& lc, const DevMech& M, const KOpts& o, const SlotLayout& L,
+                                 long long nc, const double* p, const double* T, const double* Y, double* out,
+                                 double* J, char* gws, cudaStream_t st) {
+    return launch_jacobian_t<512>(lc, M, o, L, nc, p, T, Y, out, J, gws, st);
 }
 
 template<>

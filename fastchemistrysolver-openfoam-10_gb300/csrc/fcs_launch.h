@@ -59,10 +59,14 @@ struct LaunchCfg {
 cudaError_t launch_integrate(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,
                              const SlotLayout& L, const CellIO& io, const WorkQueue& q, char* gws,
                              cudaStream_t st);
-cudaError_t launch_eval(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,
-                        const SlotLayout& L, long long nc, const double* p, const double* T,
-                        const double* rho, const double* Y, double* out, double* J, double* Qdot,
-                        int mode, char* gws, cudaStream_t st);
+cudaError_t launch_jacobian(const LaunchCfg& lc, const DevMech& M, const KOpts& o, const SlotLayout& L,
+                            long long nc, const double* p, const double* T, const double* Y, double* out,
+                            double* J, char* gws, cudaStream_t st);
+// Per-cell evaluations without a matrix (fcs_sources.cu), L from make_source_layout.
+enum SourceMode { SRC_RHS, SRC_RATES, SRC_TC };
+cudaError_t launch_sources(const LaunchCfg& lc, const DevMech& M, const SlotLayout& L, long long nc,
+                           const double* p, const double* T, const double* rho, const double* Y, double* out,
+                           double* Qdot, SourceMode mode, char* gws, cudaStream_t st);
 cudaError_t launch_classify(const CellIO& io, int ns, double Treact, int* order, int* count,
                             cudaStream_t st);
 cudaError_t integrate_attributes(int group, bool mixed, int* maxThreads, int* regs);
@@ -89,10 +93,9 @@ cudaError_t launch_integrate_g(const LaunchCfg& lc, bool mixed, const DevMech& M
                                const SlotLayout& L, const CellIO& io, const WorkQueue& q, char* gws,
                                cudaStream_t st);
 template<int G>
-cudaError_t launch_eval_g(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,
-                          const SlotLayout& L, long long nc, const double* p, const double* T,
-                          const double* rho, const double* Y, double* out, double* J, double* Qdot,
-                          int mode, char* gws, cudaStream_t st);
+cudaError_t launch_jacobian_g(const LaunchCfg& lc, const DevMech& M, const KOpts& o, const SlotLayout& L,
+                              long long nc, const double* p, const double* T, const double* Y, double* out,
+                              double* J, char* gws, cudaStream_t st);
 template<int G>
 cudaError_t integrate_attributes_g(bool mixed, int* maxThreads, int* regs);
 

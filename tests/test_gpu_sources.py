@@ -1,0 +1,45 @@
+"""Source terms, right-hand side and chemical time scale at the edges of their
+launches (cells per block, threads per cell, cells of a grid), against the
+oracle.
+
+Tolerances: a net rate is a difference of its forward and reverse parts, summed
+over the reactions of a species, so its error is bounded by the rounding of the
+largest species' rate: 1e-10 of that (test_gpu_parity.py bounds the rates the
+same way); the time scale is a quotient of positive sums, 1e-10 relative."""
+import numpy as np
+import pytest
+
+import fcs
+from fcs.workloads import RU
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ns", [10, 32, 63, 64, 130])
+@pytest.mark.parametrize("n", [1, 5, 257])
+def test_sources_match_oracle(ns, n):
+    import oracle
+    from fcs import _lib
+    flat = fcs.flatten(fcs.synthetic_mechanism(name=f"src_{ns}", n_species=ns, n_reactions=3 * ns, n_third_body=2,
+                                               n_plog=1, seed=2000 + ns))
+    rng = np.random.default_rng(n)
+    T, p = rng.uniform(900.0, 2000.0, n), rng.uniform(1e5, 1e6, n)
+    Y = np.ascontiguousarray(rng.dirichlet(np.full(ns, 0.5), size=n).T)
+    rho = p / (RU * T * (Y / flat.W[:, None]).sum(axis=0))
+    port = oracle.Port(flat)
+    RR0, Q0 = port.rates(p, T, rho, Y)
+    f0, t0 = port.rhs(p, T, Y), port.tc(p, T, rho, Y)
+    ctx = _lib.Context(0)
+    ctx.load_mechanism(flat)
+    for mapping in (0, 32, 64, 128, 256):
+        ctx.set_options(mapping=mapping)
+        RR, Q = ctx.rates(p, T, rho, Y)
+        assert (np.abs(RR - RR0) <= 1e-10 * np.abs(RR0).max(axis=0)).all()
+        hf = np.abs(RR0).max(axis=0) * 1e9 * ns  # |Hf| stays below 1e9 J/kg
+        assert (np.abs(Q - Q0) <= 1e-10 * hf).all()
+        f = ctx.rhs(p, T, Y)
+        assert (np.abs(f - f0)[:ns] <= 1e-10 * np.abs(f0[:ns]).max(axis=0)).all()
+        # dT/dt sums Ha dY / cp: |Ha| / cp below 1e5 K
+        assert (np.abs(f - f0)[ns] <= 1e-10 * (np.abs(f0[ns]) + 1e5 * np.abs(f0[:ns]).max(axis=0))).all()
+        np.testing.assert_allclose(ctx.tc(p, T, rho, Y), t0, rtol=1e-10)
+    ctx.close()

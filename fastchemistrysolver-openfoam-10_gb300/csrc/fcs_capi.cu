@@ -504,6 +504,7 @@ bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, S
     const size_t smemCap = ctx->maxSmemPerBlock;
     int maxThreads = 0, regs = 0;
     if (integrate_attributes(group, mixed, &maxThreads, &regs) != cudaSuccess) return false;
+    if (!integrate) regs = kJacobianRegs;
     // Cells resident per SM for a layout: groups per block (group 32 packs up
     // to 8 cells into a block), blocks per SM by shared memory and registers.
     struct Res { int gpb, perSM; bool global; int cells; };
@@ -525,8 +526,9 @@ bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, S
     // chunks of 256 (12 KB) would keep four.
     Res res{};
     for (int v = kJacVariants - 1; v >= 0; v--) {
-        const SlotLayout L = make_layout(ctx->M.ns, ctx->M.nr, ctx->M.nTB, mixed, seulex, 1,
-                                         std::max(ctx->M.nr, ctx->M.jac[v].values));
+        const SlotLayout L = integrate ? make_layout(ctx->M.ns, ctx->M.nr, ctx->M.nTB, mixed, seulex, 1,
+                                                     std::max(ctx->M.nr, ctx->M.jac[v].values))
+                                       : make_jacobian_layout(ctx->M.ns, ctx->M.nTB, ctx->M.jac[v].values);
         const Res r = residency(L);
         if (v < kJacVariants - 1 && (r.global || (!res.global && r.cells <= res.cells))) continue;
         sh.L = L;
@@ -804,6 +806,25 @@ extern "C" fcs_status fcs_integrate_lts(fcs_ctx* ctx, int64_t n, const double* d
 // ------------------------------------------------------------------------
 // per-cell evaluations
 
+// Threads per cell of the evaluations under AUTO.  Without a matrix 64 up to 63
+// species, 128 above, for any number of cells; rates() and tc() together, us,
+// 300 | 20,000 cells: 53 species 64 threads 77 | 1,620 (32: 107 | 1,620, 128:
+// 77 | 1,807); 111 species 128 threads 97 | 3,097 (64: 117 | 2,975, 256: 105 |
+// 4,128); 200 species 128 threads 152 | 6,045 (64: 195 | 5,894, 256: 153 | 6,977).
+// Jacobians, us, 30 | 300 | 3,000 cells: 10 species 64 threads 37 | 38 | 130
+// (128: 36 | 38 | 166); 16 with fall-off 128 threads 53 | 60 | 375 (64: 70 | 71 |
+// 385); 53: 64 threads 128 | 131 | 509, 128 threads 77 | 86 | 524; 111: 256
+// threads 173 | 209 | 1,917 (128: 209 | 234 | 2,180); 200: 256 threads 320 | 506 |
+// 4,588, 512 threads 254 | 528 | 5,064.
+static int jacobian_group(fcs_ctx* ctx, long long cells) {
+    const int n = ctx->M.n;
+    const double perSM = (double)cells / std::max(1, ctx->numSMs);
+    if (n <= 32) return ctx->M.nSp > 0 ? 128 : 64;
+    if (n <= 64) return perSM > 9 ? 64 : 128;
+    if (n <= 128) return 256;
+    return perSM > 1 ? 256 : 512;
+}
+
 static fcs_status eval_impl(fcs_ctx* ctx, int64_t nc, const double* p, const double* T, const double* rho,
                             const double* Y, double* out, double* J, double* Qdot, int mode, int32_t flags) {
     if (!ctx) return FCS_ERR_INVALID;
@@ -835,17 +856,10 @@ static fcs_status eval_impl(fcs_ctx* ctx, int64_t nc, const double* p, const dou
         if (J) { CK(ctx->bJ.ensure((size_t)n * n * nc)); dJ = ctx->bJ.p; }
         if (Qdot) { CK(ctx->bQ.ensure(nc)); dQ = ctx->bQ.p; }
     }
-    // The per-cell evaluations run on cell groups (the lane mapping is the
-    // integrator's), the same for any number of cells.  rates() and tc()
-    // together, us, 300 | 20,000 cells: 53 species 64 threads 77 | 1,620 (32: 107
-    // | 1,620, 128: 77 | 1,807); 111 species 128 threads 97 | 3,097 (64: 117 |
-    // 2,975, 256: 105 | 4,128); 200 species 128 threads 152 | 6,045 (64: 195 |
-    // 5,894, 256: 153 | 6,977).
-    const int wide = ctx->M.n <= 128 ? 256 : 512;  // with a matrix
+    // the per-cell evaluations run on cell groups (the lane mapping is the integrator's)
     const int group = ctx->opt.mapping > FCS_MAPPING_LANE ? ctx->opt.mapping
-                      : ctx->M.n <= 64                    ? 64
-                      : mode == 1                         ? wide
-                                                          : 128;
+                      : mode == 1                         ? jacobian_group(ctx, nc)
+                                                          : ctx->M.n <= 64 ? 64 : 128;
     Shape sh;
     if (mode == 1) {
         if (!make_shape(ctx, group, false, nc, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape");

@@ -239,6 +239,22 @@ inline SlotLayout make_source_layout(int ns, int nr, int nTB) {
     return L;
 }
 
+// A Jacobian without the step around it: no stage vectors, pivots or scratch of
+// the solves.  values: doubles of a chunk (or of the net rates).
+inline SlotLayout make_jacobian_layout(int ns, int nTB, int values) {
+    SlotLayout L{};
+    const int n = ns + 1;
+    L.ld = n | 1;
+    int o = align16(n * L.ld * 8);
+    L.offVec = o;   o = align16(o + 2 * n * 8);
+    L.offSp = o;    o = align16(o + 7 * ns * 8);
+    L.offRx = o;    o = align16(o + values * 8);
+    L.offTb = o;    o = align16(o + 2 * (nTB > 0 ? nTB : 1) * 8);
+    L.offRed = o;   o = align16(o + 48 * 8);
+    L.bytes = o;
+    return L;
+}
+
 template<class MT>
 struct Slot {
     int ld, n, ns;

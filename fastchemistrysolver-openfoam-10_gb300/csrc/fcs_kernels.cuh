@@ -934,9 +934,12 @@ integrate_kernel(const DevMech M, const KOpts o, const SlotLayout L, CellIO io, 
     }
 }
 
-// J and f(y) per cell: one group per cell, Y read-only (copied into the slot)
+// J and f(y) per cell: one group per cell, Y read-only (copied into the slot).
+// Bounded by the latency of its sums: in the integrator's slot one cell of 111
+// species resided per SM, without the vectors of the step two do (2,001 cells
+// 1.50 -> 1.36 ms).
 template<int G>
-__global__ void __launch_bounds__(G == 32 ? 256 : G)
+__global__ void __launch_bounds__(G == 32 ? 256 : G, 65536 / kJacobianRegs / (G == 32 ? 256 : G))
 jacobian_kernel(const DevMech M, const KOpts o, const SlotLayout L, long long nc, const double* __restrict__ p,
                 const double* __restrict__ T, const double* __restrict__ Y, double* __restrict__ out,
                 double* __restrict__ Jout, char* __restrict__ gws) {

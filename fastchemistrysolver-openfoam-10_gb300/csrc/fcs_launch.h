@@ -59,6 +59,7 @@ struct LaunchCfg {
 cudaError_t launch_integrate(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,
                              const SlotLayout& L, const CellIO& io, const WorkQueue& q, char* gws,
                              cudaStream_t st);
+constexpr int kJacobianRegs = 128;  // the Jacobian kernel is compiled for no more
 cudaError_t launch_jacobian(const LaunchCfg& lc, const DevMech& M, const KOpts& o, const SlotLayout& L,
                             long long nc, const double* p, const double* T, const double* Y, double* out,
                             double* J, char* gws, cudaStream_t st);

@@ -43,3 +43,34 @@ def test_sources_match_oracle(ns, n):
         assert (np.abs(f - f0)[ns] <= 1e-10 * (np.abs(f0[ns]) + 1e5 * np.abs(f0[:ns]).max(axis=0))).all()
         np.testing.assert_allclose(ctx.tc(p, T, rho, Y), t0, rtol=1e-10)
     ctx.close()
+
+
+@pytest.mark.parametrize("ns,special", [(10, 0), (14, 4), (34, 0), (63, 0), (64, 0), (112, 0), (130, 0), (200, 0)])
+def test_jacobian_matches_oracle_on_every_group(ns, special):
+    """AUTO takes other groups for few cells than for many: the same bits.  Against
+    the oracle 1e-11 of a cell's largest element (test_gpu_parity.py: 1e-12 of the
+    largest, for up to 111 species)."""
+    import oracle
+    from fcs import _lib
+    flat = fcs.flatten(fcs.synthetic_mechanism(name=f"jac_{ns}", n_species=ns, n_reactions=3 * ns, n_third_body=2,
+                                               n_plog=1, n_falloff=(special, 0, 0), seed=3000 + ns))
+    n = 3
+    rng = np.random.default_rng(ns)
+    T, p = rng.uniform(900.0, 2000.0, n), rng.uniform(1e5, 1e6, n)
+    Y = np.ascontiguousarray(rng.dirichlet(np.full(ns, 0.5), size=n).T)
+    J0, f0 = oracle.Port(flat).jacobian(p, T, Y)
+    ctx = _lib.Context(0)
+    ctx.load_mechanism(flat)
+    for mapping in (0, 32, 64, 128, 256):
+        ctx.set_options(mapping=mapping)
+        J, f = ctx.jacobian(p, T, Y)
+        assert (np.abs(J - J0) <= 1e-11 * np.abs(J0).max(axis=(1, 2), keepdims=True)).all()
+        if mapping == 0:
+            few = J, f
+    ctx.set_options(mapping=0)
+    many = np.arange(10 * 152 if ns < 64 else 320) % n
+    J, f = ctx.jacobian(p[many], T[many], np.ascontiguousarray(Y[:, many]))
+    np.testing.assert_array_equal(J[:n], few[0])
+    np.testing.assert_array_equal(J[-n:], few[0][many[-n:]])
+    np.testing.assert_array_equal(f[:, :n], few[1])
+    ctx.close()

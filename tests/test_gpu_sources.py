@@ -74,3 +74,30 @@ def test_jacobian_matches_oracle_on_every_group(ns, special):
     np.testing.assert_array_equal(J[-n:], few[0][many[-n:]])
     np.testing.assert_array_equal(f[:, :n], few[1])
     ctx.close()
+
+
+@pytest.mark.parametrize("falloff", [(0, 1, 0), (1, 8, 9), (2, 9, 8), (0, 0, 33)])
+def test_falloff_rates_match_oracle(falloff):
+    """Few Troe or SRI reactions are shared out over four lanes each, more take one
+    lane each."""
+    import oracle
+    from fcs import _lib
+    flat = fcs.flatten(fcs.synthetic_mechanism(name="fall", n_species=20, n_reactions=60, n_third_body=2, n_plog=1,
+                                               n_falloff=falloff, seed=77))
+    n = 33
+    rng = np.random.default_rng(5)
+    T, p = rng.uniform(900.0, 2000.0, n), 10.0 ** rng.uniform(3.0, 7.0, n)
+    Y = np.ascontiguousarray(rng.dirichlet(np.full(20, 0.5), size=n).T)
+    rho = p / (RU * T * (Y / flat.W[:, None]).sum(axis=0))
+    port = oracle.Port(flat)
+    RR0, _ = port.rates(p, T, rho, Y)
+    J0, _ = port.jacobian(p, T, Y)
+    ctx = _lib.Context(0)
+    ctx.load_mechanism(flat)
+    for mapping in (0, 32, 64, 128, 256):
+        ctx.set_options(mapping=mapping)
+        RR, _ = ctx.rates(p, T, rho, Y)
+        assert (np.abs(RR - RR0) <= 1e-10 * np.abs(RR0).max(axis=0)).all()
+        J, _ = ctx.jacobian(p, T, Y)
+        assert (np.abs(J - J0) <= 1e-10 * np.abs(J0).max(axis=(1, 2), keepdims=True)).all()
+    ctx.close()

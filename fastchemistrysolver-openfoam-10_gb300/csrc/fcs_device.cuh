@@ -986,7 +986,7 @@ __device__ __forceinline__ void net_production(const Grp<G>& g, const DevMech& M
 // Bound by the count of FP64 warp instructions (19 cycles each per SM) when
 // the SM is full of cells and by their latency when it holds one.  Reactions
 // sorted by path, sums by length, scalars side by side, compares on integers:
-// 877 -> 735 instructions on 53 species with 64 threads, fcs_rhs on
+// 877 -> 723 instructions on 53 species with 64 threads, fcs_rhs on
 // 2,001 cells 0.19 -> 0.15 ms.
 
 template<int G, class MT>
@@ -1171,7 +1171,7 @@ __device__ __noinline__ double rates_eval(const Grp<G>& g, const DevMech& M, con
 // net production (collected in the temperature row) and dq/dT (in the
 // temperature column).  The former column owners walked incidence lists of
 // unequal length in which reactants and products took different branches:
-// 3,011 FP64 warp instructions on 53 species with 64 threads, now 2,143, and
+// 3,011 FP64 warp instructions on 53 species with 64 threads, now 2,043, and
 // 2,000 such matrices 0.65 -> 0.50 ms.
 
 // d q / d C of every occurrence of x's species, into v (reactants, then

@@ -869,7 +869,8 @@ static fcs_status eval_impl(fcs_ctx* ctx, int64_t nc, const double* p, const dou
         sh.L.rw = sum_threads(ctx, group, false, nc);
         sh.global = (size_t)sh.L.bytes > ctx->maxSmemPerBlock;
         sh.lc.group = group;
-        sh.lc.block = group == 32 ? 128 : group;
+        const int cells = sh.global ? 1 : (int)std::min<size_t>(kSourceCells32, ctx->maxSmemPerBlock / sh.L.bytes);
+        sh.lc.block = group == 32 ? 32 * cells : group;
     }
     const int gpb = sh.lc.block / sh.lc.group;
     sh.lc.grid = (int)((nc + gpb - 1) / gpb);

@@ -64,6 +64,7 @@ cudaError_t launch_jacobian(const LaunchCfg& lc, const DevMech& M, const KOpts& 
                             long long nc, const double* p, const double* T, const double* Y, double* out,
                             double* J, char* gws, cudaStream_t st);
 // Per-cell evaluations without a matrix (fcs_sources.cu), L from make_source_layout.
+constexpr int kSourceCells32 = 4;  // most cells in a block of 32-thread groups
 enum SourceMode { SRC_RHS, SRC_RATES, SRC_TC };
 cudaError_t launch_sources(const LaunchCfg& lc, const DevMech& M, const SlotLayout& L, long long nc,
                            const double* p, const double* T, const double* rho, const double* Y, double* out,

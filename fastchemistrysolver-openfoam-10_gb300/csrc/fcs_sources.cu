@@ -14,7 +14,6 @@
 
 namespace fcs {
 
-constexpr int kSourceCells32 = 4;  // cells of a block of 32-thread groups
 constexpr int kSourceRegs = 80;    // 128 (as compiled without a bound): 5.48 ms, 64: 5.18 with spills for 32 threads
 
 template<int G>

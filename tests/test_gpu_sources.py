@@ -101,3 +101,26 @@ def test_falloff_rates_match_oracle(falloff):
         J, _ = ctx.jacobian(p, T, Y)
         assert (np.abs(J - J0) <= 1e-10 * np.abs(J0).max(axis=(1, 2), keepdims=True)).all()
     ctx.close()
+
+
+def test_groups_of_32_with_a_large_slot():
+    """7,500 reactions: four cells' net rates exceed a block's shared memory, so
+    fewer cells share a block; the rates have the bits of the larger groups."""
+    from fcs import _lib
+    flat = fcs.flatten(fcs.synthetic_mechanism(name="many", n_species=60, n_reactions=7500, n_third_body=2, n_plog=1,
+                                               seed=9))
+    n = 9
+    rng = np.random.default_rng(n)
+    T, p = rng.uniform(900.0, 2000.0, n), rng.uniform(1e5, 1e6, n)
+    Y = np.ascontiguousarray(rng.dirichlet(np.full(60, 0.5), size=n).T)
+    rho = p / (RU * T * (Y / flat.W[:, None]).sum(axis=0))
+    ctx = _lib.Context(0)
+    ctx.load_mechanism(flat)
+    out = []
+    for mapping in (32, 64, 256):
+        ctx.set_options(mapping=mapping)
+        out.append(ctx.rates(p, T, rho, Y)[0])
+    np.testing.assert_array_equal(out[0], out[1])
+    np.testing.assert_array_equal(out[0], out[2])
+    assert np.isfinite(out[0]).all() and np.abs(out[0]).max() > 0
+    ctx.close()

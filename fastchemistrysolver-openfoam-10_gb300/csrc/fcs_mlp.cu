@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "../../include/fcs_mlp.h"
+#include "fcs_infer_layout.h"
 #include "fcs_mlp_internal.h"
 #include "fcs_tc.cuh"
 
@@ -234,6 +235,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
 constexpr int kMaxLayers = 9, kInferStages = 3, kWidth = 256;
 constexpr int kInferThreads = 320;
 constexpr int kBoxBytes = 128 * BK * 2;                    // one ring stage; one 64-column chunk of the activations
+static_assert(kBoxBytes == kActChunkBytes, "a weight box and an activation chunk are both 128 x 64 BF16");
 constexpr int kInferSmem = (4 + kInferStages) * kBoxBytes + 256;
 
 struct InferArgs {
@@ -247,11 +249,6 @@ struct InferArgs {
 };
 
 struct InferMaps { CUtensorMap w[kMaxLayers]; };
-
-// Byte offset of element (r, k) of the activations
-__device__ __forceinline__ int act_offset(int r, int k) {
-    return (k >> 6) * kBoxBytes + r * 128 + ((((k & 63) >> 3) ^ (r & 7)) << 4) + (k & 7) * 2;
-}
 
 __global__ void __launch_bounds__(kInferThreads, 2)
 infer_kernel(const __grid_constant__ InferMaps maps, const InferArgs a) {
@@ -340,7 +337,7 @@ infer_kernel(const __grid_constant__ InferMaps maps, const InferArgs a) {
                 k++;
             }
     } else if (warp >= 2 && run) {
-        // a warp reads and writes its own rows (input) or rows and columns only
+        // who writes what, and why no barrier between the warps is needed: fcs_infer_layout.h
         const int q = warp & 3, part = (warp - 2) >> 2, r = 32 * q + lane;
         const uint32_t lanes = tmem + (static_cast<uint32_t>(32 * q) << 16);
         int k = 0;  // layers finished
@@ -354,7 +351,7 @@ infer_kernel(const __grid_constant__ InferMaps maps, const InferArgs a) {
                 const bool in0 = k2 < a.nIn, in1 = k2 + 1 < a.nIn;
                 const float m0k = in0 ? __ldg(a.mean + k2) : 0.f, m1k = in1 ? __ldg(a.mean + k2 + 1) : 0.f;
                 const float s0k = in0 ? __ldg(a.rstd + k2) : 0.f, s1k = in1 ? __ldg(a.rstd + k2 + 1) : 0.f;
-                for (int r0 = 32 * q + 16 * part; r0 < 32 * q + 16 * part + 16; r0 += 8) {
+                for (int r0 = input_row(q, part); r0 < input_row(q, part) + 16; r0 += 8) {
                     float x0[8], x1[8];
 #pragma unroll
                     for (int u = 0; u < 8; u++) {
@@ -395,25 +392,28 @@ infer_kernel(const __grid_constant__ InferMaps maps, const InferArgs a) {
                     tc::fence_async_shared();
                     tc::mbar_arrive(ready);
                 } else {
-                    // 16 columns at a time through the rows' own bytes of the
-                    // activations (free now), to leave as runs along the rows
+                    // 16 columns at a time through this warp's input bytes of
+                    // the next tile, to leave as runs along the rows
                     for (int c0 = 16 * part; c0 < a.nOut; c0 += 32) {
                         float v[16];
                         tc::tmem_ld16(lanes + c0, v);
-                        float* mine = reinterpret_cast<float*>(act + part * kBoxBytes);
 #pragma unroll
                         for (int u = 0; u < 16; u++) {
                             const int c = c0 + u;
                             if (c < a.nOut)
-                                mine[r * 32 + ((u ^ r) & 15)] =
+                                *reinterpret_cast<float*>(act + stage_offset(q, part, lane, u)) =
                                     fmaf(v[u] + __ldg(bias + c), __ldg(a.scale + c), __ldg(a.shift + c));
                         }
                         __syncwarp();
                         const int u = lane & 15, c = c0 + u;
                         if (c < a.nOut) {
-#pragma unroll 4
-                            for (int rr = 32 * q + (lane >> 4); rr < 32 * q + 32; rr += 2)
-                                if (rr < rows) a.y[(m0 + rr) * a.nOut + c] = mine[rr * 32 + ((u ^ rr) & 15)];
+#pragma unroll 8
+                            for (int i = 0; i < 16; i++) {
+                                const int rr = 16 * (lane >> 4) + i;
+                                if (32 * q + rr < rows)
+                                    a.y[(m0 + 32 * q + rr) * a.nOut + c] =
+                                        *reinterpret_cast<const float*>(act + stage_offset(q, part, rr, u));
+                            }
                         }
                         __syncwarp();
                     }

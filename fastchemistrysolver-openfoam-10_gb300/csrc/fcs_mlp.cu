@@ -1066,6 +1066,12 @@ extern "C" fcs_status fcs_mlp_forward(fcs_mlp* mlp, int32_t e, int64_t n, const 
         MCK(cudaMemcpyAsync(mlp->xDev.p, x, (size_t)n * mlp->sh.n_in * 4, cudaMemcpyHostToDevice, mlp->st));
         dx = mlp->xDev.p;
         dy = mlp->yDev.p;
+    } else if (const uintptr_t x0 = (uintptr_t)x, y0 = (uintptr_t)y;
+               x0 < y0 + (size_t)n * mlp->sh.n_out * 4 && y0 < x0 + (size_t)n * mlp->sh.n_in * 4) {
+        // in place: the kernel stores a tile's rows while other tiles still read theirs
+        MCK(mlp->xDev.ensure((size_t)n * mlp->sh.n_in));
+        MCK(cudaMemcpyAsync(mlp->xDev.p, x, (size_t)n * mlp->sh.n_in * 4, cudaMemcpyDeviceToDevice, mlp->st));
+        dx = mlp->xDev.p;
     }
     fcs_status s = fcs::mlp_forward_device(mlp, e, n, dx, dy, mlp->st);
     if (s != FCS_OK) return s;

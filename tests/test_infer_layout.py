@@ -41,3 +41,24 @@ def test_every_row_of_several_tiles_per_block(n_in, n_out, n):
     for _ in range(3):
         np.testing.assert_array_equal(mlp.forward(0, x), parts)
     mlp.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_in,n_out,shift", [(56, 55, 0), (13, 12, 128), (20, 64, 0)])
+def test_forward_in_place(n_in, n_out, shift):
+    """Device arrays that overlap: the result is that of separate arrays."""
+    import __graft_entry__
+    __graft_entry__.build()
+    import torch
+    from fcs import _lib
+    n = 3000
+    mlp = _lib.Mlp(n_in, n_out, width=256, depth=2, members=1, seed=4)
+    x = np.random.default_rng(n_in).normal(0, 1, (n, n_in)).astype(np.float32)
+    buf = torch.zeros(n * max(n_in, n_out) + shift, dtype=torch.float32, device="cuda")
+    buf[:n * n_in] = torch.from_numpy(x.ravel()).cuda()
+    torch.cuda.synchronize()
+    at = buf.data_ptr()
+    mlp._check(mlp.L.fcs_mlp_forward(mlp.h, 0, n, at, at + 4 * shift, _lib.PTR_DEVICE))
+    y = buf[shift:shift + n * n_out].cpu().numpy().reshape(n, n_out)
+    np.testing.assert_array_equal(y, mlp.forward(0, x))
+    mlp.close()

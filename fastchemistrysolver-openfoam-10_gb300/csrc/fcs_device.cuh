@@ -8,6 +8,15 @@
 // scalars that steer control flow (error norms, step sizes) come out of
 // butterfly reductions, so every thread of a group holds bit-identical values
 // and takes the same branches.
+//
+// Code size: on a full SM the warps are spread over all phases of a step and
+// share one instruction cache.  A loop that strides by the group runs once or
+// twice, so it is kept rolled (left alone, the compiler unrolls it by four);
+// the solves of small groups load four columns ahead instead of eight, and the
+// mixed kernel has one right-hand side for its FP32 and its FP64 attempts.  34
+// species, Seulex, 64 threads, 4,560 cells: mixed 125 -> 98 ms, FP64 81 -> 72
+// (of 26 cycles per instruction 11 had been spent waiting for it); 53 species,
+// Rodas34 mixed 128 -> 110.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -791,6 +800,7 @@ __device__ __forceinline__ void serial_sums(const Grp<G>& g, int n, const SumOf&
 template<int G, class MT>
 __device__ __forceinline__ void third_bodies(const Grp<G>& g, const DevMech& M, const Slot<MT>& s) {
     const int ns = M.ns;
+    #pragma unroll 1
     for (int t = g.rank; t < M.nTB; t += G) {
         const double* e = M.eff + (size_t)t * ns;
         double m = 0;
@@ -970,6 +980,7 @@ __device__ __forceinline__ double sum_terms(const uint32_t* __restrict__ con, in
 template<int G, class MT>
 __device__ __forceinline__ void net_production(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double* out) {
     const int lane = g.rank & 31;
+    #pragma unroll 1
     for (int k = g.rank >> 5; k < M.prod.groups; k += G / 32) {
         const uint32_t e = __ldg(M.prod.elem + 32 * k + lane);
         const int n = e & 0xffff, most = __shfl_sync(0xffffffffu, n, 0), i = e >> 16;
@@ -999,6 +1010,7 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
     const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * T, p);
     double invrhoM = 0;
     if (s.rw == 1) {
+        #pragma unroll 1
         for (int i = g.rank; i < ns; i += G) {
             const double y0 = YT[i];
             s.C[i] = (positive(y0) ? y0 : 0.0) * __ldg(&M.invW[i]);
@@ -1007,6 +1019,7 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
         double same;
         serial_sums(g, ns, f, f, s.red, invrhoM, same);
     } else {
+        #pragma unroll 1
         for (int i = r0; i < ns; i += s.rw) {
             const double y0 = YT[i];
             invrhoM = fma((positive(y0) ? y0 : 0.0) * __ldg(&M.invW[i]), t.numByP, invrhoM);
@@ -1015,6 +1028,7 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
     }
     const double rhoM = 1.0 / invrhoM;
     const double Tp = mode == 2 ? T : Tc;
+    #pragma unroll 1
     for (int i = g.rank; i < ns; i += G) {
         const double invW = __ldg(&M.invW[i]);
         const double y0 = YT[i], y = positive(y0) ? y0 : 0.0;
@@ -1033,12 +1047,14 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
     g.sync();
     net_production<G, MT>(g, M, s, out);
     g.sync();
+    #pragma unroll 1
     for (int i = g.rank; i < ns; i += G) out[i] = (__ldg(&M.W[i]) * invrhoM) * out[i];
     double cpm = 0, dtd = 0;
     if (s.rw == 1) {
         serial_sums(g, ns, SumOf{YT, 0, s.Cp}, SumOf{s.Ha, 0, out}, s.red, cpm, dtd);
     } else {
         if (s.rw < G) g.sync();
+        #pragma unroll 1
         for (int i = r0; i < ns; i += s.rw) {
             cpm = fma(YT[i], s.Cp[i], cpm);
             dtd = fma(s.Ha[i], out[i], dtd);
@@ -1065,6 +1081,7 @@ __device__ __noinline__ double tc_eval(const Grp<G>& g, const DevMech& M, const 
     const double Tc = clampT(M, T);
     const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * T, p);
     double sumc = 0;
+    #pragma unroll 1
     for (int i = g.rank; i < ns; i += G) {
         const double ci = rho * Y[i] / __ldg(&M.W[i]);
         s.C[i] = ci;
@@ -1137,6 +1154,7 @@ __device__ __noinline__ double rates_eval(const Grp<G>& g, const DevMech& M, con
     const int ns = M.ns;
     const double Tc = clampT(M, T);
     const ThermoScalars t = thermo_scalars(g, s.red, Tc, kRu * Tc, p);
+    #pragma unroll 1
     for (int i = g.rank; i < ns; i += G) {
         s.C[i] = rho * Y[i] / __ldg(&M.W[i]);
         const Nasa a = load_nasa(species_coeffs(M, i, Tc));
@@ -1149,9 +1167,11 @@ __device__ __noinline__ double rates_eval(const Grp<G>& g, const DevMech& M, con
     g.sync();
     net_production<G, MT>(g, M, s, RR);
     g.sync();
+    #pragma unroll 1
     for (int i = g.rank; i < ns; i += G) RR[i] = RR[i] * __ldg(&M.W[i]);
     if (s.rw < G) g.sync();
     double qd = 0;
+    #pragma unroll 1
     for (int i = g.rank < s.rw ? g.rank : ns; i < ns; i += s.rw) qd -= __ldg(&M.hf[i]) * RR[i];
     qd = gsum(g, qd, s.red);
     g.sync();
@@ -1228,6 +1248,7 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     const double logT = t.logT, invT = t.invT;
     double rs = 0, mws = 0;
     if (s.rw == 1) {
+        #pragma unroll 1
         for (int i = g.rank; i < ns; i += G) {
             const double y0 = YT[i], y = positive(y0) ? y0 : 0.0;
             YT[i] = y;
@@ -1235,6 +1256,7 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
         }
         serial_sums(g, ns, SumOf{nullptr, t.numByP, s.C}, SumOf{YT, 0, M.invW}, s.red, rs, mws);
     } else {
+        #pragma unroll 1
         for (int i = r0; i < ns; i += s.rw) {
             const double y0 = YT[i], y = positive(y0) ? y0 : 0.0, invW = __ldg(&M.invW[i]);
             rs = fma(t.numByP, y * invW, rs);
@@ -1243,6 +1265,7 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
         gsum2(g, rs, mws, s.red);
     }
     const double rhoM = 1.0 / rs, invRhoM = rs, MW = 1.0 / mws;
+    #pragma unroll 1
     for (int i = g.rank; i < ns; i += G) {
         const double y0 = YT[i], y = positive(y0) ? y0 : 0.0, invW = __ldg(&M.invW[i]);
         YT[i] = y;
@@ -1266,6 +1289,7 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     if (s.rw == 1) {
         serial_sums(g, ns, SumOf{YT, 0, s.Cp}, SumOf{YT, 0, s.dCpdT}, s.red, cpm, dcpm);
     } else {
+        #pragma unroll 1
         for (int i = r0; i < ns; i += s.rw) {
             cpm = fma(YT[i], s.Cp[i], cpm);
             dcpm = fma(YT[i], s.dCpdT[i], dcpm);
@@ -1380,6 +1404,7 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     // with 128 threads, 9,000 with 256).
     // (each form in a loop of its own: chosen per term, both would be issued)
     if constexpr (G <= 64) {
+        #pragma unroll 1
         for (int j = g.rank; j < ns; j += G) {
             int last = -1;
             double e0 = 0, wd = 0;
@@ -1436,10 +1461,12 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     }
     // dB/dT is free now: the column factors of the conversion
     double* mj = s.dBdT;
+    #pragma unroll 1
     for (int j = g.rank; j < ns; j += G) mj[j] = MW * __ldg(&M.invW[j]);
     g.sync();
     // rows: production rate and temperature column; K_i for the conversion
     double* rowK = s.dCpdT;
+    #pragma unroll 1
     for (int i = g.rank; i < ns; i += G) {
         MT* row = J + i * ld;
         const double w = double(J[ns * ld + i]), tc = double(row[ns]);
@@ -1482,9 +1509,11 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     }
     double dtd = 0, dd = 0;
     if (s.rw == 1) {
+        #pragma unroll 1
         for (int i = g.rank; i < ns; i += G) s.B[i] = f[i] * s.Cp[i] + double(J[i * ld + ns]) * s.Ha[i];
         serial_sums(g, ns, SumOf{s.Ha, 0, f}, SumOf{nullptr, 1.0, s.B}, s.red, dtd, dd);
     } else {
+        #pragma unroll 1
         for (int i = r0; i < ns; i += s.rw) {
             const double dY = f[i], tcol = double(J[i * ld + ns]);
             dtd = fma(s.Ha[i], dY, dtd);
@@ -1495,6 +1524,7 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     const double dTdt = -dtd / CpM;
     g.sync();
     // temperature row (ddTdtdYT): column owners
+    #pragma unroll 1
     for (int j = g.rank; j < ns; j += G) {
         double v = 0;
         #pragma unroll 8
@@ -1509,6 +1539,7 @@ __device__ __noinline__ void jac_eval(const Grp<G>& g, const DevMech& M, const S
     if (g.rank == 0) f[ns] = dTdt;
     if (iterate) {
         g.sync();
+        #pragma unroll 1
         for (int i = g.rank; i < n; i += G) {
             const double a = i == ns ? -((-dd - dTdt * dCpMdT) / CpM) : double(J[i * ld + i]);
             J[i * ld + i] = MT(a + shift);
@@ -1627,6 +1658,7 @@ __device__ __noinline__ void lu_factor(const Grp<G>& g, MT* A, int n, int ld, in
     constexpr int W = G / 32, kAhead = 12;
     const int lane = g.rank & 31, warp = g.rank >> 5;
     const int br = (lane >> 2) & 3, bc = lane & 3;
+    #pragma unroll 1
     for (int i = g.rank; i < n; i += G) piv[i] = i;
     if (warp == 0) {
         const int size = n < 4 ? n : 4;
@@ -1646,6 +1678,7 @@ __device__ __noinline__ void lu_factor(const Grp<G>& g, MT* A, int n, int ld, in
         if (m > 0) {
             const MT r0 = MT(invD[k0]), r1 = MT(invD[k0 + 1]), r2 = MT(invD[k0 + 2]), r3 = MT(invD[k0 + 3]);
             const MT u01 = P[1], u02 = P[2], u03 = P[3], u12 = P[ld + 2], u13 = P[ld + 3], u23 = P[2 * ld + 3];
+            #pragma unroll 1
             for (int i = k1 + g.rank; i < n; i += G) {
                 MT* x = A + i * ld + k0;
                 const MT l0 = x[0] * r0;
@@ -1669,6 +1702,7 @@ __device__ __noinline__ void lu_factor(const Grp<G>& g, MT* A, int n, int ld, in
             // the rows above took the first m threads: start with the next warp
             const int first = G == 32 ? g.rank : (g.rank + G - ((m + 31) & ~31) % G) % G;
             const int cols = moved ? m + k0 : m;
+            #pragma unroll 1
             for (int t = first; t < cols; t += G) {
                 MT* x = A + k0 * ld + (t < m ? k1 + t : t - m);
                 MT x0 = x[f0 * ld], x1 = x[f1 * ld], x2 = size > 2 ? x[f2 * ld] : MT(0), x3 = size > 3 ? x[f3 * ld] : MT(0);
@@ -1738,21 +1772,21 @@ __device__ __noinline__ void lu_factor(const Grp<G>& g, MT* A, int n, int ld, in
     }
 }
 
-// Eight columns of one row, and the update of one unknown by them, in order.
-template<class MT, class VT>
+// Columns of one row, D at a time, and the update of one unknown by them, in order.
+template<int D, class MT, class VT>
 __device__ __forceinline__ VT solve_columns(const MT* row, const VT* x, int cols, int step, VT v) {
     #pragma unroll 1
-    for (int c = 0; c < cols; c += 8) {
-        MT a[8];
-        VT y[8];
+    for (int c = 0; c < cols; c += D) {
+        MT a[D];
+        VT y[D];
         #pragma unroll
-        for (int q = 0; q < 8; q++) {
+        for (int q = 0; q < D; q++) {
             const int k = (c + q < cols ? c + q : c) * step;
             a[q] = row[k];
             y[q] = x[k];
         }
         #pragma unroll
-        for (int q = 0; q < 8; q++)
+        for (int q = 0; q < D; q++)
             if (c + q < cols) v = fma(-VT(a[q]), y[q], v);
     }
     return v;
@@ -1772,11 +1806,11 @@ __device__ __forceinline__ VT solve_columns(const MT* row, const VT* x, int cols
 // solves it while the other warps update the blocks behind it, one barrier a
 // block.  Cycles per solve, one cell per SM, against one warp sweeping whole
 // columns: 53 species, 64 threads 36,500 -> 26,400; 111 species, 256 threads
-// 99,000 -> 59,000; 200 species (global workspace), 256 threads 796,000 ->
+// 99,000 -> 58,000; 200 species (global workspace), 256 threads 796,000 ->
 // 188,000.  Six 53-species cells per SM: 40,800 -> 30,500.
-template<int G, class MT, class VT>
-__device__ __noinline__ void lu_solve(const Grp<G>& g, const MT* A, int n, int ld, const int* perm,
-                                      const double* invD, VT* b) {
+template<int D, int G, class MT, class VT>
+__device__ __noinline__ void lu_solve_ahead(const Grp<G>& g, const MT* A, int n, int ld, const int* perm,
+                                            const double* invD, VT* b) {
     constexpr int W = G / 32, U = (256 + G - 1) / G;
     const unsigned FULL = 0xffffffffu;
     const int lane = g.rank & 31, warp = g.rank >> 5, nb = (n + 31) >> 5;
@@ -1804,14 +1838,14 @@ __device__ __noinline__ void lu_solve(const Grp<G>& g, const MT* A, int n, int l
             const int i = 32 * kb + lane, cols = n - 32 * kb < 32 ? n - 32 * kb : 32;
             const MT* row = A + (i < n ? i : n - 1) * ld;
             VT v = b[i < n ? i : n - 1];
-            if (kb > 0) v = solve_columns<MT, VT>(row + 32 * (kb - 1), x, 32, 1, v);
+            if (kb > 0) v = solve_columns<D, MT, VT>(row + 32 * (kb - 1), x, 32, 1, v);
             #pragma unroll 1
-            for (int c = 0; c < cols; c += 8) {
-                MT a[8];
+            for (int c = 0; c < cols; c += D) {
+                MT a[D];
                 #pragma unroll
-                for (int q = 0; q < 8; q++) a[q] = row[32 * kb + (c + q < cols ? c + q : c)];
+                for (int q = 0; q < D; q++) a[q] = row[32 * kb + (c + q < cols ? c + q : c)];
                 #pragma unroll
-                for (int q = 0; q < 8; q++) {
+                for (int q = 0; q < D; q++) {
                     if (c + q < cols - 1) {
                         const VT xj = __shfl_sync(FULL, v, c + q);
                         const VT w = fma(-VT(a[q]), xj, v);
@@ -1823,9 +1857,10 @@ __device__ __noinline__ void lu_solve(const Grp<G>& g, const MT* A, int n, int l
         }
         if (kb > 0) {
             int rb = kb + 1 + (warp - (kb + 1) % W + W) % W;  // this warp's next block after kb
+            #pragma unroll 1
             for (; rb < nb; rb += W) {
                 const int i = 32 * rb + lane;
-                if (i < n) b[i] = solve_columns<MT, VT>(A + i * ld + 32 * (kb - 1), x, 32, 1, b[i]);
+                if (i < n) b[i] = solve_columns<D, MT, VT>(A + i * ld + 32 * (kb - 1), x, 32, 1, b[i]);
             }
         }
         if (kb + 1 < nb) g.sync();
@@ -1839,15 +1874,15 @@ __device__ __noinline__ void lu_solve(const Grp<G>& g, const MT* A, int n, int l
             const int i = 32 * kb + lane, cols = n - 32 * kb < 32 ? n - 32 * kb : 32;
             const MT* row = A + (i < n ? i : n - 1) * ld;
             VT v = b[i < n ? i : n - 1];
-            if (kb + 1 < nb) v = solve_columns<MT, VT>(row + last, b + last, had, -1, v);
+            if (kb + 1 < nb) v = solve_columns<D, MT, VT>(row + last, b + last, had, -1, v);
             const VT inv = VT(invD[i < n ? i : n - 1]);
             #pragma unroll 1
-            for (int c = cols - 1; c >= 0; c -= 8) {
-                MT a[8];
+            for (int c = cols - 1; c >= 0; c -= D) {
+                MT a[D];
                 #pragma unroll
-                for (int q = 0; q < 8; q++) a[q] = row[32 * kb + (c - q >= 0 ? c - q : c)];
+                for (int q = 0; q < D; q++) a[q] = row[32 * kb + (c - q >= 0 ? c - q : c)];
                 #pragma unroll
-                for (int q = 0; q < 8; q++) {
+                for (int q = 0; q < D; q++) {
                     if (c - q >= 0) {
                         const VT xj = __shfl_sync(FULL, v * inv, c - q);
                         const VT w = fma(-VT(a[q]), xj, v);
@@ -1859,14 +1894,28 @@ __device__ __noinline__ void lu_solve(const Grp<G>& g, const MT* A, int n, int l
         }
         if (kb + 1 < nb) {
             int rb = warp;
+            #pragma unroll 1
             for (; rb < kb; rb += W) {
                 const int i = 32 * rb + lane;
-                b[i] = solve_columns<MT, VT>(A + i * ld + last, b + last, had, -1, b[i]);
+                b[i] = solve_columns<D, MT, VT>(A + i * ld + last, b + last, had, -1, b[i]);
             }
         }
         if (kb > 0) g.sync();
     }
     g.sync();
+}
+
+// Loads of eight columns ahead hide the latency of a slot in L2 (201 unknowns,
+// 256 threads: 144,000 cycles, with four 178,000); in shared memory four give
+// the same time (54 unknowns: 25,500 and 25,900 cycles) in half the code, which
+// counts where small groups fill an SM.
+template<int G, class MT, class VT>
+__device__ __forceinline__ void lu_solve(const Grp<G>& g, const MT* A, int n, int ld, const int* perm,
+                                         const double* invD, VT* b) {
+    if constexpr (G < 256) {
+        if (__isShared(A)) return lu_solve_ahead<4, G, MT, VT>(g, A, n, ld, perm, invD, b);
+    }
+    lu_solve_ahead<8, G, MT, VT>(g, A, n, ld, perm, invD, b);
 }
 
 }  // namespace fcs

@@ -207,7 +207,7 @@ __device__ __noinline__ double rodas34_attempt(const Grp<G>& g, const DevMech& M
     if (!stage_solve<G, MT>(g, M, s, cdiag, k1, tmp)) return -1.0;
     for (int i = g.rank; i < n; i += G) yTemp[i] = fma(a21, k1[i], y0[i]);
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     {
         const double dxd2 = dx * d2, e1 = c21 * invdx;
         for (int i = g.rank; i < n; i += G) k2[i] = fma(e1, k1[i], fma(dxd2, dfdx[i], dydx[i]));
@@ -216,7 +216,7 @@ __device__ __noinline__ double rodas34_attempt(const Grp<G>& g, const DevMech& M
     if (!stage_solve<G, MT>(g, M, s, cdiag, k2, tmp)) return -1.0;
     for (int i = g.rank; i < n; i += G) yTemp[i] = fma(a32, k2[i], fma(a31, k1[i], y0[i]));
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     {
         const double dxd3 = dx * d3, e1 = c31 * invdx, e2 = c32 * invdx;
         for (int i = g.rank; i < n; i += G) k3[i] = fma(e2, k2[i], fma(e1, k1[i], fma(dxd3, dfdx[i], dydx[i])));
@@ -225,7 +225,7 @@ __device__ __noinline__ double rodas34_attempt(const Grp<G>& g, const DevMech& M
     if (!stage_solve<G, MT>(g, M, s, cdiag, k3, tmp)) return -1.0;
     for (int i = g.rank; i < n; i += G) yTemp[i] = fma(a43, k3[i], fma(a42, k2[i], fma(a41, k1[i], y0[i])));
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     {
         const double dxd4 = dx * d4, e1 = c41 * invdx, e2 = c42 * invdx, e3 = c43 * invdx;
         for (int i = g.rank; i < n; i += G)
@@ -239,7 +239,7 @@ __device__ __noinline__ double rodas34_attempt(const Grp<G>& g, const DevMech& M
         yTemp[i] = y0[i] + d;
     }
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     {
         const double e1 = c51 * invdx, e2 = c52 * invdx, e3 = c53 * invdx, e4 = c54 * invdx;
         for (int i = g.rank; i < n; i += G)
@@ -253,7 +253,7 @@ __device__ __noinline__ double rodas34_attempt(const Grp<G>& g, const DevMech& M
         yTemp[i] = y0[i] + d;
     }
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 2);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 2);
     {
         const double e1 = c61 * invdx, e2 = c62 * invdx, e3 = c63 * invdx, e4 = c64 * invdx, e5 = c65 * invdx;
         for (int i = g.rank; i < n; i += G)
@@ -298,7 +298,7 @@ __device__ __noinline__ double ros34_attempt(const Grp<G>& g, const DevMech& M, 
     if (!stage_solve<G, MT>(g, M, s, cdiag, k1, tmp)) return -1.0;
     for (int i = g.rank; i < n; i += G) yTemp[i] = fma(a21, k1[i], y0[i]);
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     {
         const double dxd2 = dx * d2, f1 = c21 * invdx;
         for (int i = g.rank; i < n; i += G) k2[i] = fma(f1, k1[i], fma(dxd2, dfdx[i], dydx[i]));
@@ -307,7 +307,7 @@ __device__ __noinline__ double ros34_attempt(const Grp<G>& g, const DevMech& M, 
     if (!stage_solve<G, MT>(g, M, s, cdiag, k2, tmp)) return -1.0;
     for (int i = g.rank; i < n; i += G) yTemp[i] = fma(a32, k2[i], fma(a31, k1[i], y0[i]));
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     {
         const double dxd3 = dx * d3, f1 = c31 * invdx, f2 = c32 * invdx;
         for (int i = g.rank; i < n; i += G) k3[i] = fma(f2, k2[i], fma(f1, k1[i], fma(dxd3, dfdx[i], dydx[i])));
@@ -363,7 +363,7 @@ __device__ __noinline__ double rodas23_attempt(const Grp<G>& g, const DevMech& M
         yTemp[i] = y0[i] + dy[i];
     }
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     for (int i = g.rank; i < n; i += G) k3[i] = dydx[i] + fma(c32, k2[i], c31 * k1[i]) / dx;
     g.sync();
     if (!stage_solve<G, MT>(g, M, s, cdiag, k3, tmp)) return -1.0;
@@ -372,7 +372,7 @@ __device__ __noinline__ double rodas23_attempt(const Grp<G>& g, const DevMech& M
         yTemp[i] = y0[i] + dy[i];
     }
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     for (int i = g.rank; i < n; i += G) err[i] = dydx[i] + fma(c43, k3[i], fma(c42, k2[i], c41 * k1[i])) / dx;
     g.sync();
     if (!stage_solve<G, MT>(g, M, s, cdiag, err, tmp)) return -1.0;
@@ -415,7 +415,7 @@ __device__ __noinline__ double ros23_attempt(const Grp<G>& g, const DevMech& M, 
     if (!stage_solve<G, MT>(g, M, s, cdiag, k1, tmp)) return -1.0;
     for (int i = g.rank; i < n; i += G) yTemp[i] = fma(a21, k1[i], y0[i]);
     g.sync();
-    rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+    rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
     for (int i = g.rank; i < n; i += G) k2[i] = fma(dxd2, dfdx[i], dydx[i]) + c21 * k1[i] / dx;
     g.sync();
     if (!stage_solve<G, MT>(g, M, s, cdiag, k2, tmp)) return -1.0;
@@ -561,8 +561,8 @@ struct SeulexState {
 // returns 1 on success, 0 when the sequence diverged (step reject), 2 when the
 // mixed-precision solve needs FP64
 template<int G, class MT>
-__device__ __noinline__ int seul(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double p,
-                     const SeulexConst& sc, SeulexState& st, double dxTot, int k, CellCounters& cc) {
+__device__ __noinline__ int seul(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, const Slot<double>& sd,
+                     double p, const SeulexConst& sc, SeulexState& st, double dxTot, int k, CellCounters& cc) {
     const int n = M.n;
     double *y0_ = s.v(1), *ySeq = s.v(2), *scale = s.v(3), *yTemp = s.v(4), *dy = s.v(5), *dydx = s.v(6);
     double* tmp = s.v(11);
@@ -571,7 +571,7 @@ __device__ __noinline__ int seul(const Grp<G>& g, const DevMech& M, const Slot<M
     const double invdx = nSteps / dxTot;
     factor_iteration<G, MT>(g, M, s, invdx);
     cc.lu++;
-    rhs_eval<G, MT>(g, M, s, p, y0_, dy, 1);
+    rhs_eval<G, double>(g, M, sd, p, y0_, dy, 1);
     cc.rhs++;
     if (!stage_solve<G, MT>(g, M, s, invdx, dy, tmp)) return 2;
     cc.solves++;
@@ -585,7 +585,7 @@ __device__ __noinline__ int seul(const Grp<G>& g, const DevMech& M, const Slot<M
             for (int i = r0; i < n; i += s.rw) { const double q = dy[i] / scale[i]; a += q * q; }
             a = gsum(g, a, s.red);
             const double dy1 = sqrt(a);
-            rhs_eval<G, MT>(g, M, s, p, yTemp, dydx, 1);
+            rhs_eval<G, double>(g, M, sd, p, yTemp, dydx, 1);
             cc.rhs++;
             for (int i = g.rank; i < n; i += G) dy[i] = dydx[i] - dy[i] * invdx;
             g.sync();
@@ -603,7 +603,7 @@ __device__ __noinline__ int seul(const Grp<G>& g, const DevMech& M, const Slot<M
             st.theta = dy2 / fmax(1.0, dy1 + kSmall);
             if (st.theta > 1.0) return 0;
         }
-        rhs_eval<G, MT>(g, M, s, p, yTemp, dy, 1);
+        rhs_eval<G, double>(g, M, sd, p, yTemp, dy, 1);
         cc.rhs++;
         if (!stage_solve<G, MT>(g, M, s, invdx, dy, tmp)) return 2;
         cc.solves++;
@@ -656,7 +656,7 @@ __device__ __noinline__ void seulex_step(const Grp<G>& g, const DevMech& M, cons
         double errOld = 0;
         cc.attempts++;
         for (k = 0; k <= st.kTarg + 1; k++) {
-            const int ok = seul<G, MT>(g, M, s, p, sc, st, dx, k, cc);
+            const int ok = seul<G, MT>(g, M, s, sd, p, sc, st, dx, k, cc);
             if (ok == 2) { step.needFp64 = true; return; }
             if (ok == 0) { step.reject = true; dxNew = fabs(dx) * 0.5; break; }
             if (k == 0) {

@@ -1074,6 +1074,18 @@ __device__ __noinline__ void rhs_eval(const Grp<G>& g, const DevMech& M, const S
 // 1.49011611938476e-8; tc = sum(w) / sum(w^2) * sum(c).  Returns tc to every
 // thread.
 
+// 1/Kc of a reaction whose factors leave the range of doubles (inf, or NaN from
+// inf times 0): the quotient factor by factor; NaN ends on the clamp.
+static __device__ __noinline__ double inverse_kc_by_division(const RxnEv& x, const double* E, const PFactor& pf) {
+    double Kc = 1.0;
+    #pragma unroll 1
+    for (int q = 0; q < x.nl; q++) Kc = Kc / E[x.sl[q]];
+    #pragma unroll 1
+    for (int q = 0; q < x.nr; q++) Kc = Kc * E[x.sr[q]];
+    Kc *= fast_pow_int(pf.P, x.nr - x.nl);
+    return 1.0 / (Kc > kKcClampG ? Kc : kKcClampG);
+}
+
 template<int G, class MT>
 __device__ __noinline__ double tc_eval(const Grp<G>& g, const DevMech& M, const Slot<MT>& s, double p, double T,
                                        double rho, const double* Y) {
@@ -1106,7 +1118,11 @@ __device__ __noinline__ double tc_eval(const Grp<G>& g, const DevMech& M, const 
             #pragma unroll 1
             for (int q = 0; q < x.nr; q++) v *= s.Binv[x.sr[q]];
             if (x.nr != x.nl) v *= pressure_factor(t.pf, x.nr - x.nl);
-            Kr = Kf * (less_than(kInvKcClampG, v) ? kInvKcClampG : v);
+            // v > clamp on the integer pipe; v is a product of positive factors or NaN
+            const unsigned long long bits = __double_as_longlong(v);
+            if (bits > (unsigned long long)__double_as_longlong(kInvKcClampG))
+                v = bits < 0x7ff0000000000000ULL ? kInvKcClampG : inverse_kc_by_division(x, s.B, t.pf);
+            Kr = Kf * v;
         }
         double CF, CR;
         if (three_at_most(x)) {

@@ -560,26 +560,44 @@ fcs_status fcs::ensure_gws(fcs_ctx* ctx, const Shape& sh) {
     return FCS_OK;
 }
 
-// AUTO's threads per cell, from the mechanism and the cells per SM (Rodas34,
-// FP64, GB300).  Few cells: enough threads to shorten one cell's chain of
-// dependent work; many: as few as fill their lanes, so that more cells reside
-// and fewer FP64 instructions are issued twice.
+// AUTO's threads per cell, from the mechanism, the cells per SM and, above 31
+// species, the cells that reside (GB300; Rodas34 in FP64 where nothing is said).
+// Few cells: enough threads to shorten one cell's chain of dependent work;
+// many: as few as fill their lanes, so that more cells reside and fewer FP64
+// instructions are issued twice.
 //   up to 31 species      1 cell per SM: 10 species 64 threads 12.6 ms (32: 16.4, 128: 12.6); 16 species
 //                         with fall-off 128 threads 41.3 ms (64: 51.5, 256: 44.8)
 //                         7 per SM: 10 species 32 threads 18.2 ms (64: 20.8); 20: 37.4 (64: 46.7)
-//                         13 per SM: 16 species with fall-off 64 threads 182 ms (32: 185, 128: 227)
+//                         13 per SM: 16 species with fall-off 64 threads 182 ms (32: 185, 128: 227); Seulex,
+//                         14 per SM, 32 threads 32.0 ms (64: 38.2, 128: 47.8), 29 per SM 65.6 (64: 77)
 //   up to 63 (53 species) 1 per SM: 128 threads 25.9 ms (64: 30.4, 256: 26.8); 6: 34.1 (64: 36.0);
 //                         12: 64 threads 50.6 ms (128: 56.0); 24: 88.6 (128: 111)
-//   up to 127 (111)       one cell resides: 256 threads 99.8 ms (128: 112, 512: 108)
+//   from 9 per SM on      64 threads where more cells reside with them than with 128 (53 and 64 species), else
+//                         128: 63 species mixed 87.1 ms (64: 98.4), 80 species 73.0 (64: 84.0)
+//   up to 127             256 threads, one block of which resides (255 registers), where no second cell of 128
+//                         threads fits (111 species, 13 per SM: 218 ms, 64: 361, 128: 243) or few cells are
+//                         left to run side by side: 2 per SM, 64 species 19.5 ms (128: 21.9), 96 species 40.9
+//                         (128: 50.5).  Against them two residents of 128 threads pay from 4 per SM on, three
+//                         from 3: 64 species 20.5 ms (256: 27.6), 80: 26.6 (31.6), 96 with 3 per SM 54.7 (44.3),
+//                         with 4 53.5 (57.0); 13 per SM: 64 species 52.2 (256: 115), 96: 120 (181);
+//                         Seulex of 111 species, two residents in global memory: 264 (362)
 //   above (200)           one cell per SM: 512 threads 132 ms (256: 140)
 int fcs::auto_group(fcs_ctx* ctx, long long cells) {
     if (ctx->opt.mapping) return ctx->opt.mapping;
     const int n = ctx->M.n;
     const double perSM = (double)cells / std::max(1, ctx->numSMs);
-    if (n <= 32) return ctx->M.nSp > 0 ? (perSM > 4 ? 64 : 128) : (perSM > 4 ? 32 : 64);
-    if (n <= 64) return perSM > 9 ? 64 : 128;
-    if (n <= 128) return 256;
-    return 512;
+    if (n <= 32) {
+        if (ctx->M.nSp > 0 && perSM > 9 && ctx->opt.solver == FCS_SOLVER_SEULEX) return 32;
+        return ctx->M.nSp > 0 ? (perSM > 4 ? 64 : 128) : (perSM > 4 ? 32 : 64);
+    }
+    if (n > 128) return 512;
+    auto resident = [&](int group) {
+        Shape sh;
+        return make_shape(ctx, group, true, FCS_NOALLOC_MAX_CELLS, sh) ? sh.lc.perSM : 0;
+    };
+    const int r128 = resident(128);
+    if (n > 64 && (r128 <= resident(256) || perSM * r128 <= 7)) return 256;
+    return perSM > 9 && resident(64) > r128 ? 64 : 128;
 }
 
 // AUTO chooses the lane mapping for a Rosenbrock-family step with cells enough

@@ -92,7 +92,7 @@ enum { FCS_JACOBIAN_EXACT = 0, FCS_JACOBIAN_FAST = 1 };
  * small is redone in FP64.  Rates, thermo, equilibrium constants, the
  * Jacobian assembly, state and the step controller stay FP64. */
 enum { FCS_PRECISION_FP64 = 0, FCS_PRECISION_MIXED = 1 };
-/* Cell-to-thread mapping: AUTO chooses by mechanism size and cells.  LANE: one thread
+/* Cell-to-thread mapping: AUTO chooses by mechanism, cells and resident cells.  LANE: one thread
  * per cell, the cells' working sets in a global-memory workspace interleaved
  * across the lanes of a warp (Rosenbrock-family solvers, FP64 or mixed); the others:
  * a group of 32..256 threads per cell with its working set in shared memory
@@ -319,8 +319,8 @@ fcs_status fcs_integrate_lts(fcs_ctx* ctx, int64_t n_cells, const double* delta_
  *     contexts) race on that array and must be serialised by the caller;
  *     consecutive calls from one thread are safe (each call returns after its
  *     work has finished);
- *   - the mapping is fcs_options.mapping, else one chosen by the mechanism
- *     size alone, so that a run launches one kernel variant;
+ *   - the mapping is fcs_options.mapping, else one chosen by the mechanism,
+ *     solver and precision alone, so that a run launches one kernel variant;
  *   - the first call on a device looks up the array's address (which may load
  *     this library's device code); make it before any stream capture begins.
  */

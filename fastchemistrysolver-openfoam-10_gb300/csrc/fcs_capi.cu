@@ -493,13 +493,14 @@ static int sum_threads(fcs_ctx* ctx, int group, bool integrate, long long cells)
 }
 
 // Build the launch shape for a group size; returns false when impossible.
-bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, Shape& sh) {
+bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, Shape& sh, long long kernelCells) {
     if (group == FCS_MAPPING_LANE) return make_lane_shape(ctx, integrate, sh);
     const fcs_options& o = ctx->opt;
     const bool mixed = o.precision == FCS_PRECISION_MIXED;
     const bool seulex = integrate && o.solver == FCS_SOLVER_SEULEX;
     sh.mixed = mixed;
     sh.lc.group = group;
+    sh.lc.dense = false;
     if (ctx->M.n > 256) return false;  // the solves keep <= 256 unknowns per warp lane set
     const size_t smemCap = ctx->maxSmemPerBlock;
     int maxThreads = 0, regs = 0;
@@ -508,7 +509,7 @@ bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, S
     // Cells resident per SM for a layout: groups per block (group 32 packs up
     // to 8 cells into a block), blocks per SM by shared memory and registers.
     struct Res { int gpb, perSM; bool global; int cells; };
-    auto residency = [&](const SlotLayout& L) {
+    auto residency = [&](const SlotLayout& L, int regs) {
         Res r;
         r.gpb = 1;
         if (group == 32) r.gpb = (int)std::max<size_t>(1, std::min<size_t>(8, smemCap / (size_t)L.bytes));
@@ -524,16 +525,38 @@ bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, S
     // chunks fill more threads and need fewer barriers.  53 species at 64
     // threads: chunks of 64 reactions (3 KB of values) keep six cells per SM,
     // chunks of 256 (12 KB) would keep four.
-    Res res{};
-    for (int v = kJacVariants - 1; v >= 0; v--) {
-        const SlotLayout L = integrate ? make_layout(ctx->M.ns, ctx->M.nr, ctx->M.nTB, mixed, seulex, 1,
-                                                     std::max(ctx->M.nr, ctx->M.jac[v].values))
-                                       : make_jacobian_layout(ctx->M.ns, ctx->M.nTB, ctx->M.jac[v].values);
-        const Res r = residency(L);
-        if (v < kJacVariants - 1 && (r.global || (!res.global && r.cells <= res.cells))) continue;
-        sh.L = L;
-        sh.L.jv = v;
-        res = r;
+    auto fit = [&](int regs, SlotLayout& best) {
+        Res res{};
+        for (int v = kJacVariants - 1; v >= 0; v--) {
+            const SlotLayout L = integrate ? make_layout(ctx->M.ns, ctx->M.nr, ctx->M.nTB, mixed, seulex, 1,
+                                                         std::max(ctx->M.nr, ctx->M.jac[v].values))
+                                           : make_jacobian_layout(ctx->M.ns, ctx->M.nTB, ctx->M.jac[v].values);
+            const Res r = residency(L, regs);
+            if (v < kJacVariants - 1 && (r.global || (!res.global && r.cells <= res.cells))) continue;
+            best = L;
+            best.jv = v;
+            res = r;
+        }
+        return res;
+    };
+    Res res = fit(regs, sh.L);
+    // 256 threads as the compiler likes them take 255 registers, one block per
+    // SM; compiled for 128 registers a cell alone is slower (111 species 66.5 ->
+    // 68.8 ms, 80 species with two cells per SM 22.0 -> 25.2), but where a second
+    // cell fits and many come, two run side by side: 80 species, ten cells per
+    // SM, 100.7 -> 68.1 ms, 53 species 96.9 -> 62.5.
+    // From four per SM on (34 species, four per SM: 11.0 -> 11.5; 64: 35.7 -> 23.7).
+    if (integrate && group == 256 && std::max(cells, kernelCells) > 4LL * ctx->numSMs) {
+        int regs2 = 0, threads2 = 0;
+        SlotLayout L2;
+        if (integrate_attributes_dense256(mixed, &threads2, &regs2) == cudaSuccess && threads2 >= 256) {
+            const Res two = fit(regs2, L2);
+            if (two.cells > res.cells) {
+                res = two;
+                sh.L = L2;
+                sh.lc.dense = true;
+            }
+        }
     }
     sh.L.rw = sum_threads(ctx, group, integrate, cells);
     sh.global = res.global;
@@ -596,7 +619,7 @@ int fcs::auto_group(fcs_ctx* ctx, long long cells) {
         return make_shape(ctx, group, true, FCS_NOALLOC_MAX_CELLS, sh) ? sh.lc.perSM : 0;
     };
     const int r128 = resident(128);
-    if (n > 64 && (r128 <= resident(256) || perSM * r128 <= 7)) return 256;
+    if (n > 64 && (r128 < 2 || perSM * r128 <= 7)) return 256;
     return perSM > 9 && resident(64) > r128 ? 64 : 128;
 }
 

@@ -118,7 +118,8 @@ fcs_status refuse_if_async_pending(fcs_ctx* ctx);
 fcs_status check_device_array(fcs_ctx* ctx, const void* ptr, const char* name, size_t align);
 KOpts kopts(const fcs_options& o);
 // Launch shape of a group size for this many cells; false when impossible.
-bool make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, Shape& sh);
+// kernelCells: the cells the kernel is chosen for, when they are others.
+bool make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, Shape& sh, long long kernelCells = 0);
 // The option's mapping, else AUTO's threads per cell for this many cells.
 int auto_group(fcs_ctx* ctx, long long cells);
 // AUTO mapping: the lane mapping for this many reacting cells?

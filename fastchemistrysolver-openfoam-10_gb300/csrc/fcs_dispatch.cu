@@ -95,7 +95,9 @@ cudaError_t launch_integrate(const LaunchCfg& lc, bool mixed, const DevMech& M, 
         case 32: return launch_integrate_g<32>(lc, mixed, M, o, L, io, q, gws, st);
         case 64: return launch_integrate_g<64>(lc, mixed, M, o, L, io, q, gws, st);
         case 128: return launch_integrate_g<128>(lc, mixed, M, o, L, io, q, gws, st);
-        case 256: return launch_integrate_g<256>(lc, mixed, M, o, L, io, q, gws, st);
+        case 256:
+            return lc.dense ? launch_integrate_dense256(lc, mixed, M, o, L, io, q, gws, st)
+                            : launch_integrate_g<256>(lc, mixed, M, o, L, io, q, gws, st);
         case 512: return launch_integrate_g<512>(lc, mixed, M, o, L, io, q, gws, st);
         default: return cudaErrorInvalidValue;
     }

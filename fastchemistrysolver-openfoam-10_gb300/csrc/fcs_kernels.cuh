@@ -830,9 +830,11 @@ __device__ int seulex_integrate(const Grp<G>& g, const DevMech& M, const KOpts& 
 
 __device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned long long)__double_as_longlong(v); }
 
-// Persistent integration kernel: cell groups pull work from queue->head.
-template<int G, class MT>
-__global__ void __launch_bounds__(G == 32 ? 256 : G)
+// Persistent integration kernel: cell groups pull work from queue->head.  B:
+// blocks per SM that the registers have to leave room for (0: as the compiler
+// chooses).
+template<int G, class MT, int B = 0>
+__global__ void __launch_bounds__(G == 32 ? 256 : G, B)
 integrate_kernel(const DevMech M, const KOpts o, const SlotLayout L, CellIO io, WorkQueue q,
                  char* __restrict__ gws) {
     extern __shared__ __align__(16) char smem[];
@@ -974,11 +976,11 @@ jacobian_kernel(const DevMech M, const KOpts o, const SlotLayout L, long long nc
 // ------------------------------------------------------------------------
 // host-side launchers (instantiations)
 
-template<int G, class MT>
+template<int G, class MT, int B = 0>
 inline cudaError_t launch_integrate_t(const LaunchCfg& lc, const DevMech& M, const KOpts& o,
                                       const SlotLayout& L, const CellIO& io, const WorkQueue& q,
                                       char* gws, cudaStream_t st) {
-    auto k = integrate_kernel<G, MT>;
+    auto k = integrate_kernel<G, MT, B>;
     const size_t sm = gws ? 0 : (size_t)L.bytes * (lc.block / G);
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -1014,10 +1016,10 @@ inline cudaError_t launch_jacobian_t(const LaunchCfg& lc, const DevMech& M, cons
     return cudaGetLastError();
 }
 
-template<int G, class MT>
+template<int G, class MT, int B = 0>
 inline cudaError_t attrs_t(int* maxThreadsOut, int* regsOut) {
     cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, integrate_kernel<G, MT>);
+    cudaError_t e = cudaFuncGetAttributes(&a, integrate_kernel<G, MT, B>);
     if (e != cudaSuccess) return e;
     *maxThreadsOut = a.maxThreadsPerBlock;
     *regsOut = a.numRegs;

@@ -54,6 +54,7 @@ struct LaunchCfg {
     int block;                 // threads per block
     int grid;                  // blocks
     int perSM;                 // blocks meant to reside per SM
+    bool dense = false;        // 256 threads: the kernel with room for two blocks per SM
 };
 
 cudaError_t launch_integrate(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,
@@ -100,5 +101,10 @@ cudaError_t launch_jacobian_g(const LaunchCfg& lc, const DevMech& M, const KOpts
                               double* J, char* gws, cudaStream_t st);
 template<int G>
 cudaError_t integrate_attributes_g(bool mixed, int* maxThreads, int* regs);
+// fcs_kernels_g256d.cu
+cudaError_t launch_integrate_dense256(const LaunchCfg& lc, bool mixed, const DevMech& M, const KOpts& o,
+                                      const SlotLayout& L, const CellIO& io, const WorkQueue& q, char* gws,
+                                      cudaStream_t st);
+cudaError_t integrate_attributes_dense256(bool mixed, int* maxThreads, int* regs);
 
 }  // namespace fcs

@@ -116,7 +116,7 @@ extern "C" fcs_status fcs_integrate_noalloc(fcs_ctx* ctx, int64_t nc, double dt,
     // could make the driver enlarge its local-memory reservation.
     const int group = auto_group(ctx, FCS_NOALLOC_MAX_CELLS);
     Shape sh;
-    if (!make_shape(ctx, group, true, nActive, sh))
+    if (!make_shape(ctx, group, true, nActive, sh, FCS_NOALLOC_MAX_CELLS))
         return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
     if (sh.global)
         return set_err(ctx, FCS_ERR_UNSUPPORTED,

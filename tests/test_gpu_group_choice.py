@@ -41,3 +41,21 @@ def test_one_resident_cell_keeps_the_wide_group(ns):
     ctx.load_mechanism(flat)
     out = ctx.integrate(cells.subset(np.arange(10 * 152) % 8), 1e-8)
     assert out["stats"]["mapping"] == 256
+
+
+@pytest.mark.parametrize("ns,solver,precision", [(12, "OptRodas34", "fp64"), (34, "OptSeulex", "mixed"),
+                                                 (65, "OptRosenbrock23", "fp64"), (80, "OptRodas34", "mixed"),
+                                                 (100, "OptRodas34", "fp64"), (111, "OptSeulex", "fp64")])
+def test_two_blocks_of_256_threads_give_the_bits_of_one(ns, solver, precision):
+    """Many cells take the kernel compiled for two blocks per SM."""
+    import __graft_entry__
+    __graft_entry__.build()
+    from fcs import _lib
+    flat, cells = small_case(ns, n=8)
+    ctx = _lib.Context(0)
+    ctx.load_mechanism(flat)
+    ctx.set_options(solver=solver, precision=precision, mapping=256)
+    a, b = [ctx.integrate(cells.subset(np.arange(n) % 8), 1e-7) for n in (8, 5 * 152)]
+    assert a["stats"]["mapping"] == 256 == b["stats"]["mapping"] and (a["status"] == 0).all()
+    for k in ("T", "Y", "subDt", "RR", "status"):
+        assert np.array_equal(a[k], b[k][..., :8]) and np.array_equal(a[k], b[k][..., -8:]), k

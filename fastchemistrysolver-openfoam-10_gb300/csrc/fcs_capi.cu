@@ -11,9 +11,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <map>
+#include <new>
+#include <stdexcept>
 #include <string>
-#include <tuple>
 #include <vector>
 
 #include "../../include/fcs.h"
@@ -187,9 +187,7 @@ extern "C" fcs_status fcs_mechanism_size(const fcs_ctx* ctx, int32_t* ns, int32_
 // mechanism packing: type-block order of OptReaction::readInfo
 // (OptReaction.C:448-1175), species incidence lists in reaction order.
 
-extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc* d) {
-    if (!ctx || !d) return FCS_ERR_INVALID;
-    if (fcs_status s = refuse_if_async_pending(ctx)) return s;
+static fcs_status load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc* d) {
     const int ns = d->n_species, nr = d->n_reactions;
     if (ns < 1 || nr < 0) return set_err(ctx, FCS_ERR_INVALID, "bad species/reaction count");
     if (ns > 255) return set_err(ctx, FCS_ERR_UNSUPPORTED, "the GPU path handles up to 255 species");
@@ -340,8 +338,6 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
         incv.insert(incv.end(), inc[i].begin(), inc[i].end());
     }
     if (incv.empty()) incv.push_back(0);
-    for (const auto& v : inc)  // a sum's length has 16 bits in the lists, a Jacobian element's terms two per entry
-        if (v.size() > 32767) return set_err(ctx, FCS_ERR_UNSUPPORTED, "a species takes part in too many reactions");
     int spBegin = 0, nSp = 0;
     for (int k = 0; k < nr; k++)
         if (rx[k].fo >= 0 || rx[k].nq >= 0) {
@@ -419,6 +415,18 @@ extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc*
         ctx->gexec = nullptr;
     }
     return FCS_OK;
+}
+
+extern "C" fcs_status fcs_load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc* d) {
+    if (!ctx || !d) return FCS_ERR_INVALID;
+    if (fcs_status s = refuse_if_async_pending(ctx)) return s;
+    try {
+        return load_mechanism(ctx, d);
+    } catch (const std::bad_alloc&) {
+        return set_err(ctx, FCS_ERR_NOMEM, "out of host memory");
+    } catch (const std::length_error& e) {
+        return set_err(ctx, FCS_ERR_UNSUPPORTED, e.what());
+    }
 }
 
 // ------------------------------------------------------------------------

@@ -983,7 +983,9 @@ __device__ __forceinline__ void net_production(const Grp<G>& g, const DevMech& M
     #pragma unroll 1
     for (int k = g.rank >> 5; k < M.prod.groups; k += G / 32) {
         const uint32_t e = __ldg(M.prod.elem + 32 * k + lane);
-        const int n = e & 0xffff, most = __shfl_sync(0xffffffffu, n, 0), i = e >> 16;
+        int n = e & 0xffff;
+        if (n == kLongSum) n = __ldg(M.prod.len + 32 * k + lane);
+        const int most = __shfl_sync(0xffffffffu, n, 0), i = e >> 16;
         const double v = sum_terms(M.prod.con + __ldg(M.prod.off + k) + lane, n, most, s.q, 0.0);
         if (i != 0xffff) out[i] = v;
     }

@@ -68,12 +68,14 @@ struct JacChunk { int special, troe, sri, group0, groupEnd, pad[3]; };
 constexpr int kJacVariants = 3;
 constexpr int kJacChunk[kJacVariants] = {16, 64, 256};
 constexpr uint32_t kNoSum = 0xffff0000u;
+constexpr uint32_t kLongSum = 0xffffu;
 
 struct SumLists {
     int groups;
     const uint32_t* elem;
     const int* off;
     const uint32_t* con;
+    const uint32_t* len;    // terms of the sums whose 16-bit count is kLongSum
 };
 
 struct JacLists {

@@ -12,8 +12,10 @@
 //     end together.
 #pragma once
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 #include <cstring>
+#include <stdexcept>
 #include <utility>
 #include <vector>
 
@@ -41,9 +43,11 @@ struct Terms {
 
 // Sums, 32 to a group: elem[32 g + lane] = target << 16 | terms, the group's
 // terms from con[off[g]] on, term k of a lane at off[g] + 32 k + lane, each
-// value index << 1 | (1: added, 0: subtracted).
+// value index << 1 | (1: added, 0: subtracted).  From kLongSum terms on (a
+// species' production only: a Jacobian chunk's sums have at most 36,864)
+// elem says kLongSum and len[32 g + lane] how many.
 struct HostSums {
-    std::vector<uint32_t> elem;
+    std::vector<uint32_t> elem, len;
     std::vector<int> off;
     std::vector<uint32_t> con;
     int groups() const { return (int)off.size(); }
@@ -60,14 +64,19 @@ struct HostSums {
         for (int l = 0; l <= longest; l++) at[l + 1] += at[l];
         for (int k = 0; k < n; k++) order[at[longest - length(k)]++] = k;
         for (int g = 0; g < n; g += 32) {
-            const int len = length(order[g]);
+            const int most = length(order[g]);
             const size_t base = con.size();
+            if (base + 32 * (size_t)most > INT_MAX) throw std::length_error("reaction lists exceed 2^31 terms");
             off.push_back((int)base);
-            con.resize(base + 32 * (size_t)len, 0);
+            con.resize(base + 32 * (size_t)most, 0);
             for (int l = 0; l < 32; l++) {
                 if (g + l >= n) { elem.push_back(kNoSum); continue; }
                 const int k = order[g + l], m = length(k);
-                elem.push_back(t.target[k] << 16 | (uint32_t)m);
+                elem.push_back(t.target[k] << 16 | std::min<uint32_t>(m, kLongSum));
+                if ((uint32_t)m >= kLongSum) {
+                    len.resize(elem.size());
+                    len.back() = (uint32_t)m;
+                }
                 const uint32_t* v = t.val.data() + begin(k);
                 for (int q = 0; q < m; q++) con[base + 32 * (size_t)q + l] = v[q];
             }
@@ -98,7 +107,7 @@ struct HostLists {
 
 // The lists as one block of device memory, each part on a 16-byte boundary.
 struct ListBlock {
-    struct Sums { size_t elem, off, con; };
+    struct Sums { size_t elem, off, con, len; };
     struct Jac { size_t ev, chunk; Sums sums; };
     std::vector<char> bytes;
     size_t ev = 0, wiw = 0, RuInvW = 0, tbRow = 0, tbTerm = 0;
@@ -116,11 +125,13 @@ struct ListBlock {
         o.elem = put(s.elem);
         o.off = put(s.off);
         o.con = put(s.con);
+        o.len = put(s.len);
         return o;
     }
     static SumLists sums(const char* base, const Sums& o, const HostSums& s) {
         return SumLists{s.groups(), reinterpret_cast<const uint32_t*>(base + o.elem),
-                        reinterpret_cast<const int*>(base + o.off), reinterpret_cast<const uint32_t*>(base + o.con)};
+                        reinterpret_cast<const int*>(base + o.off), reinterpret_cast<const uint32_t*>(base + o.con),
+                        reinterpret_cast<const uint32_t*>(base + o.len)};
     }
 };
 

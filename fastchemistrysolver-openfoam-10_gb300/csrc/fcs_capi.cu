@@ -493,9 +493,10 @@ static bool lane_sums(fcs_ctx* ctx, long long cells) {
 }
 
 // Threads that carry the partial sums of a group's reductions: fixed by the
-// mechanism, so that the results do not depend on the group AUTO chooses.
+// mechanism, so that the results do not depend on the group AUTO (or, for the
+// evaluations, the lane mapping) chooses.
 static int sum_threads(fcs_ctx* ctx, int group, bool integrate, long long cells) {
-    if (ctx->opt.mapping) return group;
+    if (ctx->opt.mapping > FCS_MAPPING_LANE) return group;
     if (integrate && lane_sums(ctx, cells)) return 1;
     return std::min(group, ctx->M.n <= 128 ? 64 : 128);
 }

@@ -59,3 +59,23 @@ def test_two_blocks_of_256_threads_give_the_bits_of_one(ns, solver, precision):
     assert a["stats"]["mapping"] == 256 == b["stats"]["mapping"] and (a["status"] == 0).all()
     for k in ("T", "Y", "subDt", "RR", "status"):
         assert np.array_equal(a[k], b[k][..., :8]) and np.array_equal(a[k], b[k][..., -8:]), k
+
+
+@pytest.mark.parametrize("ns", [34, 65, 100, 127, 130])
+def test_evaluations_have_the_same_bits_under_the_lane_mapping(ns):
+    """The lane mapping is the integrator's; the evaluations run on groups whose sums
+    are those of 64 threads up to 127 species, of 128 above."""
+    import __graft_entry__
+    __graft_entry__.build()
+    from fcs import _lib
+    flat, cells = small_case(ns, n=40)
+    outs = []
+    for mapping in (0, 1, 64 if ns <= 127 else 128):
+        ctx = _lib.Context(0)
+        ctx.load_mechanism(flat)
+        ctx.set_options(mapping=mapping)
+        outs.append((*ctx.rates(cells.p, cells.T, cells.rho0, cells.Y), ctx.rhs(cells.p, cells.T, cells.Y),
+                     *ctx.jacobian(cells.p, cells.T, cells.Y)))
+    for o in outs[1:]:
+        for x, y in zip(outs[0], o):
+            np.testing.assert_array_equal(x, y)

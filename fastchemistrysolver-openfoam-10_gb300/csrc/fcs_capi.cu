@@ -161,8 +161,8 @@ extern "C" fcs_status fcs_set_options(fcs_ctx* ctx, const fcs_options* o) {
     if (!(o->abs_tol > 0) || !(o->rel_tol > 0)) return set_err(ctx, FCS_ERR_INVALID, "tolerances must be positive");
     if (o->max_steps <= 0 || o->max_rejects <= 0) return set_err(ctx, FCS_ERR_INVALID, "maxSteps must be positive");
     const int m = o->mapping;
-    if (m != 0 && m != 1 && m != 32 && m != 64 && m != 128 && m != 256)
-        return set_err(ctx, FCS_ERR_INVALID, "mapping must be auto, lane (1), 32, 64, 128 or 256");
+    if (m != 0 && m != 1 && m != 32 && m != 64 && m != 128 && m != 256 && m != 512)
+        return set_err(ctx, FCS_ERR_INVALID, "mapping must be auto, lane (1), 32, 64, 128, 256 or 512");
     ctx->opt = *o;
     return FCS_OK;
 }

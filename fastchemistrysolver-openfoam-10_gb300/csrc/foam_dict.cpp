@@ -597,6 +597,7 @@ fcs_status read_chemistry_properties(const char* path, fcs_options* o, double* i
             else if (w == "block64") o->mapping = FCS_MAPPING_BLOCK64;
             else if (w == "block128") o->mapping = FCS_MAPPING_BLOCK128;
             else if (w == "block256") o->mapping = FCS_MAPPING_BLOCK256;
+            else if (w == "block512") o->mapping = FCS_MAPPING_BLOCK512;
             else return FCS_ERR_PARSE;
         }
         if (gd->find("maxRejects") && !as_count(gd->find("maxRejects"), o->max_rejects)) return FCS_ERR_PARSE;

@@ -14,6 +14,7 @@
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/fcs.h"
@@ -187,6 +188,43 @@ extern "C" fcs_status fcs_mechanism_size(const fcs_ctx* ctx, int32_t* ns, int32_
 // mechanism packing: type-block order of OptReaction::readInfo
 // (OptReaction.C:448-1175), species incidence lists in reaction order.
 
+// Cells of a slot of this size that shared memory lets reside per SM: groups
+// per block (groups of 32 threads pack up to eight cells into a block) and
+// blocks per SM.  A slot larger than a block's shared memory lies in global
+// memory, two blocks per SM.
+struct SmemFit { int gpb, perSM; bool global; };
+static SmemFit smem_fit(const fcs_ctx* ctx, size_t bytes, bool warps) {
+    SmemFit f;
+    f.gpb = warps ? (int)std::max<size_t>(1, std::min<size_t>(8, ctx->maxSmemPerBlock / bytes)) : 1;
+    f.global = bytes > ctx->maxSmemPerBlock;
+    f.perSM = f.global ? 2 : (int)std::max<size_t>(1, (228 * 1024) / (bytes * f.gpb + 1024));
+    return f;
+}
+
+// The Jacobian chunkings that a launch shape can take (make_shape: the largest
+// chunk that does not cost a resident cell): the largest, and those that fit
+// an SM otherwise than the next larger one.  Registers only take residents
+// away.  200 species need one of three (their slots are in global memory), 111
+// two: loading 2.9 -> 1.2 and 1.4 -> 1.0 ms.
+static void wanted_chunkings(const fcs_ctx* ctx, int ns, int nr, int nTB, const std::vector<RxnInfo>& rx, bool* want) {
+    int values[kJacVariants];
+    for (int v = 0; v < kJacVariants; v++) {
+        values[v] = chunk_values(rx, nr, kJacChunk[v]);
+        want[v] = v == kJacVariants - 1;
+    }
+    for (int form = 0; form < 5; form++)  // the Jacobian's own slot; the integrators' per precision and solver
+        for (const bool warps : {false, true}) {
+            auto cells = [&](int v) {
+                const SlotLayout L = form == 4 ? make_jacobian_layout(ns, nTB, values[v])
+                                               : make_layout(ns, nr, nTB, form & 1, form & 2, 1, std::max(nr, values[v]));
+                const SmemFit f = smem_fit(ctx, (size_t)L.bytes, warps);
+                return std::make_tuple(f.global, f.gpb, f.perSM);
+            };
+            for (int v = 0; v + 1 < kJacVariants; v++)
+                if (cells(v) != cells(v + 1)) want[v] = true;
+        }
+}
+
 static fcs_status load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc* d) {
     const int ns = d->n_species, nr = d->n_reactions;
     if (ns < 1 || nr < 0) return set_err(ctx, FCS_ERR_INVALID, "bad species/reaction count");
@@ -344,7 +382,9 @@ static fcs_status load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc* d) {
             if (nSp == 0) spBegin = k;
             nSp = k + 1 - spBegin;
         }
-    const HostLists lists = build_lists(ns, rx, nr, inc, spBegin, nSp);
+    bool want[kJacVariants];
+    wanted_chunkings(ctx, ns, nr, nTB, rx, want);
+    const HostLists lists = build_lists(ns, rx, nr, inc, spBegin, nSp, want);
     std::vector<double> wiw((size_t)ns * ns);
     for (int i = 0; i < ns; i++)
         for (int j = 0; j < ns; j++) wiw[(size_t)i * ns + j] = W[i] * invW[j];
@@ -405,7 +445,7 @@ static fcs_status load_mechanism(fcs_ctx* ctx, const fcs_mechanism_desc* d) {
         const HostChunks& j = lists.jac[v];
         M.jac[v].size = j.size;
         M.jac[v].values = j.values;
-        M.jac[v].ev = reinterpret_cast<const RxnEv*>(ctx->dLists.p + at.jac[v].ev);
+        M.jac[v].ev = want[v] ? reinterpret_cast<const RxnEv*>(ctx->dLists.p + at.jac[v].ev) : nullptr;
         M.jac[v].chunk = reinterpret_cast<const JacChunk*>(ctx->dLists.p + at.jac[v].chunk);
         M.jac[v].sums = at.sums(ctx->dLists.p, at.jac[v].sums, j.sums);
     }
@@ -511,22 +551,17 @@ bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, S
     sh.lc.group = group;
     sh.lc.dense = false;
     if (ctx->M.n > 256) return false;  // the solves keep <= 256 unknowns per warp lane set
-    const size_t smemCap = ctx->maxSmemPerBlock;
     int maxThreads = 0, regs = 0;
     if (integrate_attributes(group, mixed, &maxThreads, &regs) != cudaSuccess) return false;
     if (!integrate) regs = kJacobianRegs;
-    // Cells resident per SM for a layout: groups per block (group 32 packs up
-    // to 8 cells into a block), blocks per SM by shared memory and registers.
+    // Cells resident per SM for a layout, by shared memory and registers.
     struct Res { int gpb, perSM; bool global; int cells; };
     auto residency = [&](const SlotLayout& L, int regs) {
         Res r;
-        r.gpb = 1;
-        if (group == 32) r.gpb = (int)std::max<size_t>(1, std::min<size_t>(8, smemCap / (size_t)L.bytes));
-        r.global = (size_t)L.bytes > smemCap;
-        const int block = group * r.gpb;
-        const int bySmem = r.global ? 2 : (int)std::max<size_t>(1, (228 * 1024) / ((size_t)L.bytes * r.gpb + 1024));
-        const int byRegs = std::max(1, 65536 / std::max(1, regs * block));
-        r.perSM = std::max(1, std::min(bySmem, byRegs));
+        const SmemFit f = smem_fit(ctx, (size_t)L.bytes, group == 32);
+        r.gpb = f.gpb;
+        r.global = f.global;
+        r.perSM = std::min(f.perSM, std::max(1, 65536 / std::max(1, regs * group * r.gpb)));
         r.cells = r.gpb * r.perSM;
         return r;
     };
@@ -537,6 +572,7 @@ bool fcs::make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, S
     auto fit = [&](int regs, SlotLayout& best) {
         Res res{};
         for (int v = kJacVariants - 1; v >= 0; v--) {
+            if (!ctx->M.jac[v].ev) continue;  // wanted_chunkings
             const SlotLayout L = integrate ? make_layout(ctx->M.ns, ctx->M.nr, ctx->M.nTB, mixed, seulex, 1,
                                                          std::max(ctx->M.nr, ctx->M.jac[v].values))
                                            : make_jacobian_layout(ctx->M.ns, ctx->M.nTB, ctx->M.jac[v].values);

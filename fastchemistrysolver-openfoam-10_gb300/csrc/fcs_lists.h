@@ -187,10 +187,23 @@ inline int first_of(const std::vector<RxnEv>& v, int c) {
     return k;
 }
 
+// Values of a chunk of `size` reactions: their net rates, dq/dT and d q / d C
+// of every occurrence that has one; the most any chunk needs.
+inline int chunk_values(const std::vector<RxnInfo>& rx, int nr, int size) {
+    int most = 0;
+    for (int c0 = 0; c0 < nr; c0 += size) {
+        int n = 2 * size;
+        for (int r = c0; r < std::min(nr, c0 + size); r++) n += rx[r].nl + (rx[r].rev ? rx[r].nr : 0);
+        most = std::max(most, n);
+    }
+    return most;
+}
+
 // rx: the packed reactions; inc[i]: (reaction << 1 | product) of species i in
-// reaction order; [spBegin, spBegin + nSp): the special block.
+// reaction order; [spBegin, spBegin + nSp): the special block; want: the
+// chunkings to build (all when null).
 inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, const std::vector<std::vector<int>>& inc,
-                             int spBegin, int nSp) {
+                             int spBegin, int nSp, const bool* want = nullptr) {
     HostLists H;
     auto special = [&](int r) { return r >= spBegin && r < spBegin + nSp; };
     std::vector<RxnEv> part[3];
@@ -238,6 +251,8 @@ inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, con
     for (int v = 0; v < kJacVariants; v++) {
         HostChunks& J = H.jac[v];
         J.size = kJacChunk[v];
+        J.values = chunk_values(rx, nr, J.size);
+        if (want && !want[v]) continue;
         std::vector<size_t> at(ns, 0);  // position in inc[i]
         for (int c0 = 0; c0 < nr; c0 += J.size) {
             const int c1 = std::min(nr, c0 + J.size);
@@ -255,7 +270,6 @@ inline HostLists build_lists(int ns, const std::vector<RxnInfo>& rx, int nr, con
                 ent[r - c0] = n;
                 n += rx[r].nl + (rx[r].rev ? rx[r].nr : 0);
             }
-            J.values = std::max(J.values, n);
             for (RxnEv& e : main) e.ent = ent[e.r - c0];
             J.ev.insert(J.ev.end(), main.begin(), main.end());
             t.clear();

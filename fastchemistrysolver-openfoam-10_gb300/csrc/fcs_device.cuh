@@ -1,6 +1,6 @@
 // fcs_device.cuh -- device building blocks of the per-cell stiff integrator.
 //
-// Execution model: a *cell group* of G threads (G = 32: one warp; G = 64..256:
+// Execution model: a *cell group* of G threads (G = 32: one warp; G = 64..512:
 // one thread block) owns one cell at a time and keeps the whole per-cell
 // working set in a private slot of shared memory (or of global memory when it
 // does not fit): the Jacobian / LU matrices, the stage vectors, the species
@@ -176,13 +176,13 @@ struct SlotLayout {
     int offScale;      // row / column equilibration factors [2n] double (mixed precision)
     int offPiv;        // [n] int
     int offRx;         // max(4 rc, values) doubles: the net rates, or one Jacobian chunk (fcs_lists.h)
-    int rc;
-    int offCur;        // [ns] int scratch
+    int rc;            // a quarter of the least doubles at offRx, in [1, nr]
+    int offCur;        // [ns] ints, free
     int jv;            // Jacobian chunking (kJacChunk) the region at offRx holds
     int rw;            // threads that carry the partial sums of the group's reductions
     int offTb;         // M (third-body concentration), third-body column weight [nTB] each
     int offTable;      // Seulex extrapolation table [12][n] doubles
-    int offRed;        // 48 doubles of reduction / broadcast scratch (32..36 thermo scalars, 37 log p, 38 LU)
+    int offRed;        // 48 doubles of reduction / broadcast scratch (32..36 thermo scalars, 37 log p, 38..39 LU, 38 step factor, 40 queue)
     int bytes;         // total, multiple of 16
 };
 
@@ -277,7 +277,6 @@ struct Slot {
     double *dr, *dc;
     int* piv;
     double* q;                     // net rates by packed reaction, or a Jacobian chunk's values
-    int* cur;                      // ns ints of scratch
     int jv, rw;
     double *Mtb, *tbF;
     double* table;
@@ -310,7 +309,6 @@ __device__ __forceinline__ Slot<MT> make_slot(char* base, const SlotLayout& L, c
     s.q = reinterpret_cast<double*>(base + L.offRx);
     s.jv = L.jv;
     s.rw = L.rw;
-    s.cur = reinterpret_cast<int*>(base + L.offCur);
     double* tb = reinterpret_cast<double*>(base + L.offTb);
     const int nt = M.nTB > 0 ? M.nTB : 1;
     s.Mtb = tb; s.tbF = tb + nt;

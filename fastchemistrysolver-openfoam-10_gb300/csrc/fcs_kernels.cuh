@@ -2,13 +2,12 @@
 // fcs_kernels.cuh -- sm_103a kernels of the per-cell stiff chemistry path.
 //
 //   integrate_kernel : persistent kernel; each cell group pulls cells from a
-//                      device work queue and runs OptRodas34 /
-//                      OptRosenbrock34 / OptSeulex with the reference's step
-//                      size control over one CFD step
-//   rhs_kernel       : f(y) per cell (FastChemistryModel::derivatives)
-//   jac_kernel       : J(y), f(y) per cell (FastChemistryModel::jacobian)
-//   rates_kernel     : calculate()/Qdot source terms per cell
-//   classify_kernel  : Treact skip + active-cell queue
+//                      device work queue and runs one of the five solvers with
+//                      the reference's step size control over one CFD step
+//   jacobian_kernel  : J(y), f(y) per cell (FastChemistryModel::jacobian)
+//
+// Source terms, right-hand side and time scale: fcs_sources.cu; Treact skip and
+// the queue: fcs_dispatch.cu.
 //
 // Precision: MT = double is the FP64 method; MT = float is the mixed method
 // (Jacobian storage and LU in FP32, one FP64-residual refinement sweep per

@@ -47,11 +47,8 @@ extern "C" fcs_status fcs_integrate_async(fcs_ctx* ctx, int64_t nc, double dt, c
     if (sorted) CK(ctx->bBin.ensure(std::max<int64_t>(nc, 1)));
     if (!ctx->hStats) CK(cudaMallocHost(&ctx->hStats, (ST_COUNT + 1) * sizeof(long long)));
     if (!ctx->evAsync) CK(cudaEventCreateWithFlags(&ctx->evAsync, cudaEventDisableTiming));
-    const int group = lane_auto(ctx, nc) ? (int)FCS_MAPPING_LANE : auto_group(ctx, nc);
-    Shape sh;
-    if (!make_shape(ctx, group, true, nc, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
-    fcs_status s = ensure_gws(ctx, sh);
-    if (s != FCS_OK) return s;
+    StepPlan plan;
+    if (fcs_status s = plan_step(ctx, nc, sorted, plan)) return s;
 
     CellIO io{};
     io.nCells = nc;
@@ -69,13 +66,13 @@ extern "C" fcs_status fcs_integrate_async(fcs_ctx* ctx, int64_t nc, double dt, c
     CK(cudaMemsetAsync(ctx->bHead.p, 0, QC_COUNT * sizeof(int), st));
     if (sorted) {
         CK(launch_classify_binned(io, ns, ctx->opt.T_react, ctx->bBin.p, ctx->bHead.p, st));
-        CK(launch_queue(nc, ctx->bBin.p, ctx->bHead.p, ctx->bOrder.p, st));
+        CK(launch_queue(nc, ctx->bBin.p, ctx->bHead.p, ctx->bOrder.p,
+                        lane_choice(ctx, nc, io.attemptsValid, ctx->bStats.p), st));
     } else {
         CK(launch_classify(io, ns, ctx->opt.T_react, ctx->bOrder.p, ctx->bHead.p + QC_LEN, st));
     }
-    WorkQueue q{ctx->bHead.p + QC_HEAD, ctx->bOrder.p, 0, ctx->bHead.p + QC_LEN};
     CK(cudaEventRecord(ctx->ev0, st));
-    CK(launch_integrate(sh.lc, sh.mixed, ctx->M, kopts(ctx->opt), sh.L, io, q, sh.global ? ctx->gws.p : nullptr, st));
+    CK(launch_step(ctx, plan, io, ctx->bOrder.p, ctx->bHead.p, st));
     CK(cudaEventRecord(ctx->ev1, st));
     CK(cudaMemcpyAsync(ctx->hStats, ctx->bStats.p, ST_COUNT * sizeof(long long), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(ctx->hStats + ST_COUNT, ctx->bMin.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
@@ -84,7 +81,7 @@ extern "C" fcs_status fcs_integrate_async(fcs_ctx* ctx, int64_t nc, double dt, c
     ctx->asyncPending = true;
     ctx->attN = nc;
     ctx->asyncDt = dt;
-    ctx->asyncGroup = group;
+    ctx->asyncPlan = plan;
     return FCS_OK;
 }
 
@@ -128,7 +125,7 @@ static fcs_status sync_impl(fcs_ctx* ctx, double timeout_ms, fcs_step_stats* sta
         stats->fp64_fallbacks = hs[ST_FALLBACK];
         stats->kernel_ms = ms;
         stats->call_ms = cms;
-        stats->mapping = ctx->asyncGroup;
+        stats->mapping = ctx->asyncPlan.mapping(hs);
         stats->reserved = 0;
     }
     if (dtMin) {

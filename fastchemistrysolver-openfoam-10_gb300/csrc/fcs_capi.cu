@@ -671,18 +671,59 @@ int fcs::auto_group(fcs_ctx* ctx, long long cells) {
 // AUTO chooses the lane mapping for a Rosenbrock-family step with cells enough
 // to occupy most of its lanes (at fewer cells its lanes idle and the cell
 // groups, which spread one cell over many threads, are faster).  FP64 steps of
-// 32 to 63 species take it from 1.1 cells per lane on: below, a lane has one
-// cell or none, and all of them wait for the dearest, while the groups share
-// the cells out; they take the sums over species in the lanes' order then, so
-// that results do not depend on the choice.  53 species, 44,801 cells of a later
-// step (75 attempts at most, 27 on average): lanes 1.81 s, groups 1.10 s; 65,536
-// cells of a first step (255 on average): lanes 10.5 s, groups 11.9.
-bool fcs::lane_auto(fcs_ctx* ctx, long long cells) {
-    if (!lane_sums(ctx, cells)) return false;
-    const long long lanes = lane_count(ctx);
+// 32 to 63 species take it from 1.1 cells per lane on (53 species, 65,536 cells
+// of a first step, 255 attempts on average: lanes 10.5 s, groups 11.9).  Below,
+// a lane has one cell or none, and all of them wait for the dearest, while the
+// groups share the cells out: the cells' predicted costs decide
+// (lanes_are_faster; without the binned queue there are none, and the lanes
+// run).  The groups take the sums over species in the lanes' order then, so that
+// results do not depend on the choice.
+LaneUse fcs::lane_auto(fcs_ctx* ctx, long long cells, bool binned) {
+    if (!lane_sums(ctx, cells)) return LaneUse::no;
     const int n = ctx->M.n;
-    if (n > 32 && n <= 64 && ctx->opt.precision == FCS_PRECISION_FP64) return cells * 10 >= 11 * lanes;
-    return true;
+    if (n <= 32 || n > 64 || ctx->opt.precision != FCS_PRECISION_FP64 || !binned) return LaneUse::yes;
+    return cells * 10 >= 11 * lane_count(ctx) ? LaneUse::yes : LaneUse::by_cost;
+}
+
+// For a call of this many cells, reacting or not.
+LaneChoice fcs::lane_choice(fcs_ctx* ctx, long long cells, int attemptsValid, long long* stats) {
+    LaneChoice c;
+    if (lane_auto(ctx, cells, true) == LaneUse::no) return c;
+    c.lanes = lane_count(ctx);
+    c.attemptsValid = attemptsValid;
+    c.stats = stats;
+    return c;
+}
+
+fcs_status fcs::plan_step(fcs_ctx* ctx, long long cells, bool binned, StepPlan& plan) {
+    const LaneUse use = lane_auto(ctx, cells, binned);
+    plan.byCost = use == LaneUse::by_cost;
+    plan.group = use == LaneUse::yes ? (int)FCS_MAPPING_LANE : auto_group(ctx, cells);
+    if (!make_shape(ctx, plan.group, true, cells, plan.sh) ||
+        (plan.byCost && !make_shape(ctx, FCS_MAPPING_LANE, true, cells, plan.lanes)))
+        return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
+    // one workspace: only one of the two integrates cells
+    fcs_status s = ensure_gws(ctx, plan.sh);
+    if (s == FCS_OK && plan.byCost) s = ensure_gws(ctx, plan.lanes);
+    return s;
+}
+
+// Where costs decide, both kernels are launched on queues of their own, one of
+// length 0.
+cudaError_t fcs::launch_step(fcs_ctx* ctx, const StepPlan& plan, const CellIO& io, const int* order, int* counters,
+                             cudaStream_t st) {
+    const KOpts ko = kopts(ctx->opt);
+    WorkQueue q{counters + QC_HEAD, order, 0, counters + QC_LEN};
+    if (plan.byCost) {
+        q.nDev = counters + QC_LEN_LANES;
+        const cudaError_t e =
+            launch_integrate(plan.lanes.lc, plan.lanes.mixed, ctx->M, ko, plan.lanes.L, io, q, ctx->gws.p, st);
+        if (e != cudaSuccess) return e;
+        q.head = counters + QC_HEAD_GROUPS;
+        q.nDev = counters + QC_LEN_GROUPS;
+    }
+    return launch_integrate(plan.sh.lc, plan.sh.mixed, ctx->M, ko, plan.sh.L, io, q,
+                            plan.sh.global ? ctx->gws.p : nullptr, st);
 }
 
 // ------------------------------------------------------------------------
@@ -761,25 +802,23 @@ static fcs_status integrate_impl(fcs_ctx* ctx, int64_t nc, double dt, const doub
         if (!sorted) return launch_classify(io, ns, ctx->opt.T_react, ctx->bOrder.p, ctx->bHead.p + QC_LEN, st);
         if ((e = launch_classify_binned(io, ns, ctx->opt.T_react, ctx->bBin.p, ctx->bHead.p, st)) != cudaSuccess)
             return e;
-        return launch_queue(nc, ctx->bBin.p, ctx->bHead.p, ctx->bOrder.p, st);
+        return launch_queue(nc, ctx->bBin.p, ctx->bHead.p, ctx->bOrder.p,
+                            lane_choice(ctx, nc, io.attemptsValid, ctx->bStats.p), st);
     };
     long long* hs = ctx->hStats;
     unsigned long long hminv = 0;
     unsigned long long* hmin = &hminv;
     long long hsLocal[ST_COUNT];
     int group = 0;
+    StepPlan plan;  // of a graph
     if (graph) {
         // one CUDA graph per step shape: replayed while the arrays, sizes and
         // options stay the same, re-captured when any of them changes
         if (!ctx->hStats) CK(cudaMallocHost(&ctx->hStats, (ST_COUNT + 1) * sizeof(long long)));
         hs = ctx->hStats;
         hmin = reinterpret_cast<unsigned long long*>(ctx->hStats + ST_COUNT);
-        group = lane_auto(ctx, nc) ? (int)FCS_MAPPING_LANE : auto_group(ctx, nc);
-        Shape sh;
-        if (!make_shape(ctx, group, true, nc, sh))
-            return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
-        fcs_status s = ensure_gws(ctx, sh);
-        if (s != FCS_OK) return s;
+        if (fcs_status s = plan_step(ctx, nc, sorted, plan)) return s;
+        group = plan.group;
         GraphKey key;
         std::memset(&key, 0, sizeof(key));
         key.p = p; key.rho0 = rho0; key.T = T; key.Y = Y; key.sub = sub; key.RR = RR; key.status = status;
@@ -795,9 +834,7 @@ static fcs_status integrate_impl(fcs_ctx* ctx, int64_t nc, double dt, const doub
             ctx->gexec = nullptr;
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             cudaError_t e = enqueue_prologue();
-            WorkQueue q{ctx->bHead.p + QC_HEAD, ctx->bOrder.p, 0, ctx->bHead.p + QC_LEN};
-            if (e == cudaSuccess)
-                e = launch_integrate(sh.lc, sh.mixed, ctx->M, ko, sh.L, io, q, sh.global ? ctx->gws.p : nullptr, st);
+            if (e == cudaSuccess) e = launch_step(ctx, plan, io, ctx->bOrder.p, ctx->bHead.p, st);
             if (e == cudaSuccess) e = cudaMemcpyAsync(hs, ctx->bStats.p, ST_COUNT * sizeof(long long), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaMemcpyAsync(hmin, ctx->bMin.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
             cudaGraph_t gr = nullptr;
@@ -818,10 +855,13 @@ static fcs_status integrate_impl(fcs_ctx* ctx, int64_t nc, double dt, const doub
         CK(cudaEventRecord(ctx->ev1, st));
     } else {
         CK(enqueue_prologue());
-        int nActive = 0;
-        CK(cudaMemcpyAsync(&nActive, ctx->bHead.p + QC_LEN, sizeof(int), cudaMemcpyDeviceToHost, st));
+        int len[2] = {0, 0};  // the queue, and the lanes' share where costs decide
+        CK(cudaMemcpyAsync(len, ctx->bHead.p + QC_LEN, sizeof(len), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        group = lane_auto(ctx, nActive) ? (int)FCS_MAPPING_LANE : auto_group(ctx, nActive);
+        const int nActive = len[0];
+        const LaneUse use = lane_auto(ctx, nActive, sorted);
+        group = use == LaneUse::yes || (use == LaneUse::by_cost && len[1] > 0) ? (int)FCS_MAPPING_LANE
+                                                                                : auto_group(ctx, nActive);
         Shape sh;
         if (!make_shape(ctx, group, true, nActive, sh))
             return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
@@ -863,7 +903,7 @@ static fcs_status integrate_impl(fcs_ctx* ctx, int64_t nc, double dt, const doub
         stats->fp64_fallbacks = hs[ST_FALLBACK];
         stats->kernel_ms = ms;
         stats->call_ms = cms;
-        stats->mapping = group;
+        stats->mapping = graph ? plan.mapping(hs) : group;
         stats->reserved = 0;
     }
     if (dtMin) {

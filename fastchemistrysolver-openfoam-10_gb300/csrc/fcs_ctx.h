@@ -63,6 +63,15 @@ struct Shape {
     bool mixed;
 };
 
+// A step whose queue length the host does not know: the shape for `cells`, and
+// where costs decide the lane mapping's beside it, with their workspaces.
+struct StepPlan {
+    Shape sh, lanes;
+    bool byCost = false;
+    int group = 0;
+    int mapping(const long long* stats) const { return byCost && stats[ST_LANES] ? (int)FCS_MAPPING_LANE : group; }
+};
+
 }  // namespace fcs
 
 struct fcs_ctx {
@@ -100,7 +109,7 @@ struct fcs_ctx {
     cudaEvent_t evAsync = nullptr;
     bool asyncPending = false;
     double asyncDt = 0;
-    int asyncGroup = 0;
+    fcs::StepPlan asyncPlan;
 };
 
 namespace fcs {
@@ -122,8 +131,14 @@ KOpts kopts(const fcs_options& o);
 bool make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, Shape& sh, long long kernelCells = 0);
 // The option's mapping, else AUTO's threads per cell for this many cells.
 int auto_group(fcs_ctx* ctx, long long cells);
-// AUTO mapping: the lane mapping for this many reacting cells?
-bool lane_auto(fcs_ctx* ctx, long long cells);
+// AUTO mapping: the lane mapping for this many reacting cells, or their costs to
+// decide (LaneChoice)?
+enum class LaneUse { no, yes, by_cost };
+LaneUse lane_auto(fcs_ctx* ctx, long long cells, bool binned);
+LaneChoice lane_choice(fcs_ctx* ctx, long long cells, int attemptsValid, long long* stats);
+fcs_status plan_step(fcs_ctx* ctx, long long cells, bool binned, StepPlan& plan);
+cudaError_t launch_step(fcs_ctx* ctx, const StepPlan& plan, const CellIO& io, const int* order, int* counters,
+                        cudaStream_t st);
 // Global-memory workspace for shapes whose slot exceeds shared memory.
 fcs_status ensure_gws(fcs_ctx* ctx, const Shape& sh);
 

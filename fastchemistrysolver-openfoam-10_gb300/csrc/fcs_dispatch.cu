@@ -50,7 +50,30 @@ __global__ void classify_bin_kernel(CellIO io, int ns, double Treact, int* bin, 
         if (hist[b]) atomicAdd(&counters[QC_BINS + b], hist[b]);
 }
 
-__global__ void queue_kernel(long long nc, const int* __restrict__ bin, int* counters, int* __restrict__ order) {
+// Lanes or groups.  A lane takes a cell from its start to its end, so that a
+// step of about a cell per lane lasts as long as the dearest cell; the groups
+// share the cells out and last as long as all of them together.  So the dearest
+// cell's cost times the lanes stands against the sum times the ratio of the two
+// rates, 1.7 to 1.9 for 53 and 63 species, 2.4 for 34, 2.2 for 45 with fall-off.
+// 54,000 cells of 58,368 lanes: attempts up to 1.25 to 1.4 times their mean, 34 |
+// 45 | 53 | 63 species, lanes 1.7 | 3.6 | 3.3 | 4.2 s, groups 2.7 | 5.8 | 4.0 | 5.8; up
+// to 2.2 (53) to 4 times, lanes 0.40 | 0.86 | 1.03 | 1.98 s, groups 0.29 | 0.80 | 0.79 |
+// 1.07.  Cells all in the lowest bin (a sub-step as long as the step, eight
+// attempts at most) say nothing of their spread: groups.
+__device__ bool lanes_are_faster(const int* __restrict__ cells, const LaneChoice& choice) {
+    float sum = 0, dearest = 0;
+    int highest = 0;
+    for (int b = 0; b < kQueueBins; b++) {
+        if (!cells[b]) continue;
+        dearest = exp2f(choice.attemptsValid ? (b + 24.5f) / 8 : b + 0.5f);
+        sum += cells[b] * dearest;
+        highest = b;
+    }
+    return highest > 0 && dearest * (float)choice.lanes <= 1.9f * sum;
+}
+
+__global__ void queue_kernel(long long nc, const int* __restrict__ bin, int* counters, int* __restrict__ order,
+                             const LaneChoice choice) {
     __shared__ int start[kQueueBins];
     if (threadIdx.x == 0) {
         int s = 0;
@@ -58,7 +81,15 @@ __global__ void queue_kernel(long long nc, const int* __restrict__ bin, int* cou
             start[b] = s;
             s += counters[QC_BINS + b];
         }
-        if (blockIdx.x == 0) counters[QC_LEN] = s;
+        if (blockIdx.x == 0) {
+            counters[QC_LEN] = s;
+            if (choice.lanes > 0) {
+                const bool lanes = lanes_are_faster(counters + QC_BINS, choice);
+                counters[QC_LEN_LANES] = lanes ? s : 0;
+                counters[QC_LEN_GROUPS] = lanes ? 0 : s;
+                choice.stats[ST_LANES] = lanes;
+            }
+        }
     }
     __syncthreads();
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nc;
@@ -78,12 +109,13 @@ cudaError_t launch_classify_binned(const CellIO& io, int ns, double Treact, int*
     return cudaGetLastError();
 }
 
-cudaError_t launch_queue(long long nc, const int* bin, int* counters, int* order, cudaStream_t st) {
+cudaError_t launch_queue(long long nc, const int* bin, int* counters, int* order, const LaneChoice& choice,
+                         cudaStream_t st) {
     const int block = 256;
     long long blocks = (nc + block - 1) / block;
     if (blocks > 152 * 8) blocks = 152 * 8;
     if (blocks < 1) blocks = 1;
-    queue_kernel<<<(int)blocks, block, 0, st>>>(nc, bin, counters, order);
+    queue_kernel<<<(int)blocks, block, 0, st>>>(nc, bin, counters, order, choice);
     return cudaGetLastError();
 }
 

@@ -364,14 +364,8 @@ extern "C" fcs_status fcs_integrate_gated(fcs_ctx* ctx, int64_t nc, double dt, c
     CK(cudaMemsetAsync(g->counters.p, 0, QC_COUNT * sizeof(int), st));
     CK(cudaMemsetAsync(g->gstats.p, 0, GS_COUNT * sizeof(unsigned long long), st));
     // the fallback cells run with the plain method's mapping for this batch
-    const int group = lane_auto(ctx, nc) ? (int)FCS_MAPPING_LANE : auto_group(ctx, nc);
-    Shape sh;
-    if (!make_shape(ctx, group, true, nc, sh)) return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
-    if (sh.global) {
-        const size_t groups = (size_t)sh.lc.grid * (sh.lc.block / sh.lc.group);
-        if (ctx->gws.ensure(groups * (size_t)sh.L.bytes) != cudaSuccess)
-            return set_err(ctx, FCS_ERR_NOMEM, "global workspace allocation failed");
-    }
+    StepPlan plan;
+    if (fcs_status s = plan_step(ctx, nc, true, plan)) return s;
     if (nc > 0) {
         // T <= Treact: skipped exactly as by fcs_integrate (its queue is not used here)
         CK(launch_classify(io, ns, ctx->opt.T_react, ctx->bOrder.p, ctx->bHead.p + 1, st));
@@ -398,11 +392,9 @@ extern "C" fcs_status fcs_integrate_gated(fcs_ctx* ctx, int64_t nc, double dt, c
         const long long wTot = nc * 32;
         gate_kernel<<<(int)((wTot + 255) / 256), 256, 0, st>>>(a);
         CK(cudaGetLastError());
-        CK(launch_queue(nc, g->bin.p, g->counters.p, g->order.p, st));
+        CK(launch_queue(nc, g->bin.p, g->counters.p, g->order.p, lane_choice(ctx, nc, attValid, ctx->bStats.p), st));
         CK(cudaEventRecord(ctx->ev0, st));
-        WorkQueue q{g->counters.p + QC_HEAD, g->order.p, 0, g->counters.p + QC_LEN};
-        const KOpts ko = kopts(ctx->opt);
-        CK(launch_integrate(sh.lc, sh.mixed, ctx->M, ko, sh.L, io, q, sh.global ? ctx->gws.p : nullptr, st));
+        CK(launch_step(ctx, plan, io, g->order.p, g->counters.p, st));
         CK(cudaEventRecord(ctx->ev1, st));
         const long long aTot = (long long)auditCap * 32;
         audit_kernel<<<(int)((aTot + 255) / 256), 256, 0, st>>>(ns, nc, auditCap, g->counters.p, g->auditCell.p,
@@ -449,7 +441,7 @@ extern "C" fcs_status fcs_integrate_gated(fcs_ctx* ctx, int64_t nc, double dt, c
         stats->fp64_fallbacks = hs[ST_FALLBACK];
         stats->kernel_ms = ms;
         stats->call_ms = cms;
-        stats->mapping = group;
+        stats->mapping = plan.mapping(hs);
         stats->reserved = 0;
     }
     if (gst) {

@@ -132,6 +132,6 @@ struct KOpts {
 
 // Per-cell status / counters layout in the stats buffer (int64 each).
 enum { ST_CELLS = 0, ST_SKIPPED, ST_FAILED, ST_ATTEMPTS, ST_ACCEPTED, ST_JAC, ST_LU,
-       ST_RHS, ST_SOLVES, ST_FALLBACK, ST_COUNT };
+       ST_RHS, ST_SOLVES, ST_FALLBACK, ST_LANES, ST_COUNT };  // ST_LANES: the queue went to the lane mapping
 
 }  // namespace fcs

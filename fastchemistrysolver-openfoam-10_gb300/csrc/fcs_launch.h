@@ -34,11 +34,20 @@ struct WorkQueue {
     const int* nDev;           // if set, the queue length is read from device memory instead
 };
 
-// Work-queue counters (int) of the binned queue: next position, length,
-// cells per bin, cells placed per bin, and a spare counter for callers.
+// Work-queue counters (int) of the binned queue: next position, length, the
+// length for the lanes and for the groups (LaneChoice: one of them 0) with the
+// groups' own position, cells per bin, cells placed per bin, and a spare counter
+// for callers.
 constexpr int kQueueBins = 64;
-enum { QC_HEAD = 0, QC_LEN = 1, QC_BINS = 2, QC_FILL = QC_BINS + kQueueBins, QC_AUX = QC_FILL + kQueueBins,
-       QC_COUNT };
+enum { QC_HEAD = 0, QC_LEN = 1, QC_LEN_LANES = 2, QC_LEN_GROUPS = 3, QC_HEAD_GROUPS = 4, QC_BINS = 5,
+       QC_FILL = QC_BINS + kQueueBins, QC_AUX = QC_FILL + kQueueBins, QC_COUNT };
+
+// Lanes or cell groups, by the cells' predicted costs (queue_kernel).
+struct LaneChoice {
+    long long lanes = 0;       // of the lane mapping's grid; 0: no choice wanted
+    int attemptsValid = 0;     // the bins are attempt_bin's
+    long long* stats = nullptr;
+};
 
 #ifdef __CUDACC__
 // Queue bin of a cell whose previous integration took `attempts` attempted
@@ -80,8 +89,10 @@ cudaError_t integrate_attributes(int group, bool mixed, int* maxThreads, int* re
 // (bin = floor(log2), 0..31); bin[c] = -1 for skipped cells.
 cudaError_t launch_classify_binned(const CellIO& io, int ns, double Treact, int* bin, int* counters,
                                    cudaStream_t st);
-// order[] = cells with bin >= 0, highest bin first; counters[QC_LEN] = their count.
-cudaError_t launch_queue(long long nc, const int* bin, int* counters, int* order, cudaStream_t st);
+// order[] = cells with bin >= 0, highest bin first; counters[QC_LEN] = their count;
+// with a choice, counters[QC_LEN_LANES] or [QC_LEN_GROUPS] as well.
+cudaError_t launch_queue(long long nc, const int* bin, int* counters, int* order, const LaneChoice& choice,
+                         cudaStream_t st);
 
 // The lane-per-cell integrator (fcs_lane.cu): lc.group == 1, lc.block
 // threads per block, one cell per thread; gws holds make_lane_layout(...).words

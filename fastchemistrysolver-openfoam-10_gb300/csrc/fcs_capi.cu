@@ -650,12 +650,14 @@ fcs_status fcs::ensure_gws(fcs_ctx* ctx, const Shape& sh) {
 //                         with 4 53.5 (57.0); 13 per SM: 64 species 52.2 (256: 115), 96: 120 (181);
 //                         Seulex of 111 species, two residents in global memory: 264 (362)
 //   above (200)           one cell per SM: 512 threads 132 ms (256: 140)
-int fcs::auto_group(fcs_ctx* ctx, long long cells) {
+// anyCount: one group for calls of few and of many cells (many, except that 32
+// threads under Seulex cost few cells 22.8 ms where 64 take 13.0).
+int fcs::auto_group(fcs_ctx* ctx, long long cells, bool anyCount) {
     if (ctx->opt.mapping) return ctx->opt.mapping;
     const int n = ctx->M.n;
     const double perSM = (double)cells / std::max(1, ctx->numSMs);
     if (n <= 32) {
-        if (ctx->M.nSp > 0 && perSM > 9 && ctx->opt.solver == FCS_SOLVER_SEULEX) return 32;
+        if (ctx->M.nSp > 0 && perSM > 9 && !anyCount && ctx->opt.solver == FCS_SOLVER_SEULEX) return 32;
         return ctx->M.nSp > 0 ? (perSM > 4 ? 64 : 128) : (perSM > 4 ? 32 : 64);
     }
     if (n > 128) return 512;

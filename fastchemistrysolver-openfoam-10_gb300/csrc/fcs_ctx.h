@@ -130,7 +130,7 @@ KOpts kopts(const fcs_options& o);
 // kernelCells: the cells the kernel is chosen for, when they are others.
 bool make_shape(fcs_ctx* ctx, int group, bool integrate, long long cells, Shape& sh, long long kernelCells = 0);
 // The option's mapping, else AUTO's threads per cell for this many cells.
-int auto_group(fcs_ctx* ctx, long long cells);
+int auto_group(fcs_ctx* ctx, long long cells, bool anyCount = false);
 // AUTO mapping: the lane mapping for this many reacting cells, or their costs to
 // decide (LaneChoice)?
 enum class LaneUse { no, yes, by_cost };

@@ -114,7 +114,7 @@ extern "C" fcs_status fcs_integrate_noalloc(fcs_ctx* ctx, int64_t nc, double dt,
 
     // AUTO as for many cells, whatever the call's count: another kernel variant
     // could make the driver enlarge its local-memory reservation.
-    const int group = auto_group(ctx, FCS_NOALLOC_MAX_CELLS);
+    const int group = auto_group(ctx, FCS_NOALLOC_MAX_CELLS, true);
     Shape sh;
     if (!make_shape(ctx, group, true, nActive, sh, FCS_NOALLOC_MAX_CELLS))
         return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");

@@ -23,11 +23,10 @@ constexpr int act_offset(int r, int k) {
 // First of the 16 rows whose input warp (q, part) writes
 constexpr int input_row(int q, int part) { return 32 * q + 16 * part; }
 
-// Byte offset of the float staged for column u (of 16) of row 32 q + r: rows r
-// and r + 16 share the 128 bytes of the warp's input row r & 15.  The lanes of
-// a column, and of rows r and r + 16, fall on 32 different banks.
-constexpr int stage_offset(int q, int part, int r, int u) {
-    return (input_row(q, part) + (r & 15)) * 128 + (r >> 4) * 64 + ((u ^ r) & 15) * 4;
-}
+// Where it stages: floats from its input rows' first bytes on, column u (of 16)
+// of row 32 q + r at stage_index(r, u), rows r and r + 1 in 128 bytes.  The lanes
+// of a column, and of rows r and r + 1, fall on 32 different banks.
+constexpr int stage_offset(int q, int part) { return input_row(q, part) * 128; }
+constexpr int stage_index(int r, int u) { return (r & 31) * 16 + ((u ^ (r >> 1)) & 15); }
 
 }  // namespace fcs

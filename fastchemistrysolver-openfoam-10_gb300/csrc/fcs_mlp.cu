@@ -230,7 +230,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
 // activations went through L2 and HBM between layers and the epilogue stored
 // 16-byte pieces of 32 rows at a time.  4 members of 56-256x4-55
 // through fcs_mlp_forward: 65,536 rows 1,047 -> 600 us, 1,000 rows 437 -> 292 us
-// (555 and 251 us since the error code is read without a copy).
+// (560 and 237 us since the error code is read without a copy).
 
 constexpr int kMaxLayers = 9, kInferStages = 3, kWidth = 256;
 constexpr int kInferThreads = 320;
@@ -397,23 +397,20 @@ infer_kernel(const __grid_constant__ InferMaps maps, const InferArgs a) {
                     for (int c0 = 16 * part; c0 < a.nOut; c0 += 32) {
                         float v[16];
                         tc::tmem_ld16(lanes + c0, v);
+                        float* mine = reinterpret_cast<float*>(act + stage_offset(q, part));
 #pragma unroll
                         for (int u = 0; u < 16; u++) {
                             const int c = c0 + u;
                             if (c < a.nOut)
-                                *reinterpret_cast<float*>(act + stage_offset(q, part, lane, u)) =
+                                mine[stage_index(lane, u)] =
                                     fmaf(v[u] + __ldg(bias + c), __ldg(a.scale + c), __ldg(a.shift + c));
                         }
                         __syncwarp();
                         const int u = lane & 15, c = c0 + u;
                         if (c < a.nOut) {
-#pragma unroll 8
-                            for (int i = 0; i < 16; i++) {
-                                const int rr = 16 * (lane >> 4) + i;
-                                if (32 * q + rr < rows)
-                                    a.y[(m0 + 32 * q + rr) * a.nOut + c] =
-                                        *reinterpret_cast<const float*>(act + stage_offset(q, part, rr, u));
-                            }
+#pragma unroll 4
+                            for (int rr = 32 * q + (lane >> 4); rr < 32 * q + 32; rr += 2)
+                                if (rr < rows) a.y[(m0 + rr) * a.nOut + c] = mine[stage_index(rr, u)];
                         }
                         __syncwarp();
                     }

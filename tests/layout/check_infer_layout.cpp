@@ -26,7 +26,7 @@ int main() {
             for (int u = 0; u < 16; u++) {
                 unsigned banks = 0;
                 for (int r = 0; r < 32; r++) {
-                    const int at = stage_offset(q, part, r, u);
+                    const int at = stage_offset(q, part) + 4 * stage_index(32 * q + r, u);
                     banks |= 1u << (at / 4 % 32);
                     if (at % 4 || at < 0 || at + 4 > (int)owner.size()) return std::printf("offset %d\n", at), 1;
                     for (int b = 0; b < 4; b++) {
@@ -37,6 +37,12 @@ int main() {
                     }
                 }
                 if (banks != 0xffffffffu) return std::printf("bank conflict: %d %d %d\n", q, part, u), 1;
+            }
+            for (int r = 0; r < 32; r += 2) {  // the stores' reads: 16 columns of two rows
+                unsigned banks = 0;
+                for (int u = 0; u < 32; u++)
+                    banks |= 1u << ((stage_offset(q, part) / 4 + stage_index(r + (u >> 4), u & 15)) % 32);
+                if (banks != 0xffffffffu) return std::printf("bank conflict in the reads: %d %d %d\n", q, part, r), 1;
             }
         }
     std::printf("ok\n");

@@ -704,10 +704,13 @@ fcs_status fcs::plan_step(fcs_ctx* ctx, long long cells, bool binned, StepPlan& 
     if (!make_shape(ctx, plan.group, true, cells, plan.sh) ||
         (plan.byCost && !make_shape(ctx, FCS_MAPPING_LANE, true, cells, plan.lanes)))
         return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
-    // one workspace: only one of the two integrates cells
-    fcs_status s = ensure_gws(ctx, plan.sh);
-    if (s == FCS_OK && plan.byCost) s = ensure_gws(ctx, plan.lanes);
-    return s;
+    // one workspace: only one of the two integrates cells; without room for the
+    // lanes' the groups run
+    if (plan.byCost && ensure_gws(ctx, plan.lanes) != FCS_OK) {
+        cudaGetLastError();
+        plan.byCost = false;
+    }
+    return ensure_gws(ctx, plan.sh);
 }
 
 // Where costs decide, both kernels are launched on queues of their own, one of
@@ -862,9 +865,14 @@ static fcs_status integrate_impl(fcs_ctx* ctx, int64_t nc, double dt, const doub
         CK(cudaStreamSynchronize(st));
         const int nActive = len[0];
         const LaneUse use = lane_auto(ctx, nActive, sorted);
-        group = use == LaneUse::yes || (use == LaneUse::by_cost && len[1] > 0) ? (int)FCS_MAPPING_LANE
-                                                                                : auto_group(ctx, nActive);
         Shape sh;
+        bool lanes = use == LaneUse::yes;
+        if (use == LaneUse::by_cost && len[1] > 0) {
+            // without room for the lanes' workspace the groups run
+            lanes = make_shape(ctx, FCS_MAPPING_LANE, true, nActive, sh) && ensure_gws(ctx, sh) == FCS_OK;
+            if (!lanes) cudaGetLastError();
+        }
+        group = lanes ? (int)FCS_MAPPING_LANE : auto_group(ctx, nActive);
         if (!make_shape(ctx, group, true, nActive, sh))
             return set_err(ctx, FCS_ERR_UNSUPPORTED, "no launch shape for this mapping");
         fcs_status s = ensure_gws(ctx, sh);

@@ -7,7 +7,7 @@ import pytest
 from test_gpu_groups import small_case
 
 pytestmark = pytest.mark.gpu
-DT = 1e-8
+DT = 1e-10  # a few attempts a cell
 
 
 @pytest.mark.parametrize("ns", [34, 50])
@@ -72,3 +72,37 @@ def test_outside_the_choice(flags, n, mapping):
     T, Y, sub, RR, st = c.T.copy(), c.Y.copy(), c.subDt.copy(), np.zeros_like(c.Y), np.zeros(n, np.int32)
     code, stats, _ = ctx.integrate_raw(n, DT, c.p, c.rho0, T, Y, sub, RR, st, flags=2 if flags else 0)
     assert stats["mapping"] == mapping and stats["cells_integrated"] == n
+
+
+@pytest.mark.parametrize("how", ["plain", "graph"])
+def test_groups_where_the_lanes_workspace_has_no_room(how):
+    """Equal costs want the lanes; when their workspace cannot be allocated the groups
+    run, with the same result."""
+    import __graft_entry__
+    __graft_entry__.build()
+    import torch
+    from fcs import _lib
+    flat, few = small_case(34, n=16)
+    ctx = _lib.Context(0)
+    ctx.load_mechanism(flat)
+
+    def step(n, equal, flags, fails):
+        c = few.subset(np.arange(n) % 16)
+        c.subDt[:] = DT / 4.5 if equal else np.where(np.arange(n) % 64 == 0, DT / 70, DT)
+        d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (c.p, c.rho0, c.T, c.Y, c.subDt)]
+        torch.cuda.synchronize()
+        _lib.fail_allocations(fails)
+        try:
+            code, stats, _ = ctx.integrate_raw(n, DT, *d, device=True, flags=flags)
+        finally:
+            _lib.fail_allocations(0)
+        assert code == 0 and stats["cells_integrated"] == n
+        return stats["mapping"], [v.cpu().numpy() for v in d[2:]]
+
+    step(54400, False, 0, 0)  # groups: grows the other buffers, and another batch size keeps no costs
+    flags = _lib.CUDA_GRAPH if how == "graph" else 0
+    mapping, a = step(54000, True, flags, 1)
+    assert mapping > 1
+    _, b = step(54000, True, flags, 0)
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
